@@ -24,7 +24,7 @@
 
 #include "../../include/elmm_gpu.h"
 #include "elmm_kernels2.cuh"
-#include "elmm_poisson_reg.cuh"
+#include "elmm_poisson_any.cuh"
 #include "elmm_temperature.cuh"
 #include "elmm_solids.cuh"
 #include "elmm_slabs.cuh"
@@ -54,18 +54,37 @@ static const double kAlpha[3] = {4.0 / 15.0, 1.0 / 15.0, 1.0 / 6.0};
 static const double kBeta[3] = {8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0};
 static const double kRho[3] = {0.0, -17.0 / 60.0, -5.0 / 12.0};
 
+// The passes of a length n (false unless it factors into 2, 3 and 5): the
+// fewest radices up to 16, of those the smallest largest one, in descending
+// order (the first pass of a y tile loads its radix of rows at once).
 static bool factorize(int n, FFTFactors &f) {
+  static const int radix[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
   f.n = n;
   f.nfac = 0;
-  int r = n;
-  for (int p : {4, 2, 3, 5}) {
-    while (r % p == 0) {
-      if (f.nfac >= kMaxFac) return false;
-      f.fac[f.nfac++] = p;
-      r /= p;
+  int cur[kMaxFac], best = kMaxFac + 1;
+  std::function<void(int, int, size_t)> search = [&](int r, int depth, size_t from) {
+    if (r == 1 && depth > 0 && (depth < best || (depth == best && cur[0] < f.fac[0]))) {
+      best = depth;
+      std::copy(cur, cur + depth, f.fac);
     }
+    if (r == 1 || depth >= std::min(best, kMaxFac)) return;
+    for (size_t q = from; q < sizeof(radix) / sizeof(radix[0]); q++)
+      if (r % radix[q] == 0) {
+        cur[depth] = radix[q];
+        search(r / radix[q], depth + 1, q);
+      }
+  };
+  search(n, 0, 0);
+  if (best > kMaxFac) return false;
+  f.nfac = best;
+  int len = n;
+  for (int p = 0; p < best; p++) {
+    f.step[p] = n / len;
+    len /= f.fac[p];
+    f.M[p] = len;
+    f.magic[p] = len > 1 ? (unsigned)(((1ULL << 32) + len - 1) / len) : 0u;
   }
-  return r == 1;
+  return true;
 }
 
 static int round_up(int a, int b) { return (a + b - 1) / b * b; }
@@ -100,6 +119,28 @@ static int encode_box_map(CUtensorMap *m, T *base, long long pitch, int ny, int 
                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(ELMM_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
   return ELMM_OK;
+}
+
+// the axes the transforms take: 4 pairs of rows (x) or TyOf columns (y),
+// twice, within a block's shared memory
+template <typename T>
+static bool transforms_too_long(int nx, int ny, int optin) {
+  const size_t c = 2 * sizeof(typename Vec2<T>::type);
+  return c * (kRowsX / 2) * nx > (size_t)optin || c * TyOf<T>::v * ny > (size_t)optin;
+}
+// the shared-memory limit of the generic transforms: the opt-in maximum less
+// what they hold statically
+template <typename T>
+static cudaError_t fft_any_attributes(int optin) {
+  for (const void *f : {(const void *)k_fftx_fwd_any<T>, (const void *)k_fftx_inv_any<T>,
+                        (const void *)k_ffty_any<T, false>, (const void *)k_ffty_any<T, true>}) {
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, f);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // ------------------------------------------------------- host grid tables
@@ -283,7 +324,7 @@ struct LaunchSet {
 };
 
 enum { LK_CELLS = 0, LK_BOX, LK_ROWS, LK_YCOLS, LK_TRI, LK_MOM, LK_SHELL, LK_XREG, LK_YREG, LK_TRIT, LK_TCOL, LK_DCOL,
-       LK_AVG, LK_COMMIT, LK_TPAIR, LK_PROJ, LK_PROJ2, LK_DCOL2, LK_MOMT, LK_SGST, LK_WM, LK_N };
+       LK_AVG, LK_COMMIT, LK_TPAIR, LK_PROJ, LK_PROJ2, LK_DCOL2, LK_MOMT, LK_SGST, LK_WM, LK_WSUM, LK_N };
 
 // the z-chunk lengths (planes of a tile's column) the autotuner tries for
 // the momentum and SGS kernels
@@ -375,8 +416,9 @@ struct BatchT {
   // transform phase (a batch with several x or y lengths); joined back into
   // the stream before the next phase, captured as graph branches
   static constexpr int kBranches = 4;
-  cudaStream_t branch[kBranches] = {};
-  cudaEvent_t ev_fork = nullptr, ev_join[kBranches] = {};
+  // (and one more branch for the level sums of W2)
+  cudaStream_t branch[kBranches + 1] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[kBranches + 1] = {};
   float tune_ms[10] = {};  // rows 8, rows 4, cols 16, cols 32, momentum chunks 8/16/32, SGS chunks 8/16/32
   // immersed solid bodies per domain (elmm_set_solids): the gathers of the
   // velocity IB points followed by the nullified points, the gathers of the
@@ -517,7 +559,7 @@ struct BatchT {
       if (side) cudaStreamDestroy(side);
     }
     stream = side = nullptr;
-    for (int b = 0; b < kBranches; b++) {
+    for (int b = 0; b <= kBranches; b++) {
       if (branch[b]) cudaStreamDestroy(branch[b]);
       if (ev_join[b]) cudaEventDestroy(ev_join[b]);
       branch[b] = nullptr;
@@ -648,7 +690,7 @@ struct BatchT {
     const int n = nd;
     shell_per = n > 1 ? 4 : 1;
     CU(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    for (int b = 1; b < kBranches; b++) {
+    for (int b = 1; b <= kBranches; b++) {
       CU(cudaStreamCreateWithFlags(&branch[b], cudaStreamNonBlocking));
       CU(cudaEventCreateWithFlags(&ev_join[b], cudaEventDisableTiming));
     }
@@ -675,18 +717,19 @@ struct BatchT {
     }
     int maxnx = 0, maxny = 0, maxnz = 0, anyzper = 0;
     for (auto &h : hdom) { maxnx = std::max(maxnx, h.nx); maxny = std::max(maxny, h.ny); maxnz = std::max(maxnz, h.nz); anyzper |= h.zper; }
-    smem_x = sizeof(T2) * 2 * (kRowsX / 2) * maxnx;
-    smem_y = sizeof(T2) * 2 * TyOf<T>::v * maxny;
+    smem_x = smem_y = 0;
+    for (size_t d = 0; d < hdom.size(); d++) {
+      if (!fft_reg_supported(hdom[d].nx)) smem_x = std::max(smem_x, fft_any_smem_x<T>(hdom[d].nx, hplan[d].nsx));
+      if (!fft_reg_supported(hdom[d].ny)) smem_y = std::max(smem_y, fft_any_smem_y<T>(hdom[d].ny));
+    }
     smem_tri = sizeof(double) * kTriThreads * maxnz * (anyzper ? 2 : 1);
     // the opt-in maximum, so that handles of different sizes never lower the
     // limit under each other's launches
     int optin = 0;
     CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    if (smem_x > (size_t)optin || smem_y > (size_t)optin || smem_tri > (size_t)optin)
+    if (transforms_too_long<T>(maxnx, maxny, optin) || smem_tri > (size_t)optin)
       return fail(ELMM_ERR_INVALID_CONFIG, "grid too large for the shared-memory transforms");
-    CU(cudaFuncSetAttribute(k_fftx_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    CU(cudaFuncSetAttribute(k_fftx_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    CU(cudaFuncSetAttribute(k_ffty<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    CU((fft_any_attributes<T>(optin)));
     CU(cudaFuncSetAttribute(k_tri<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     CU(cudaFuncSetAttribute(k_momentum<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
     CU(cudaFuncSetAttribute(k_momentum<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
@@ -729,10 +772,10 @@ struct BatchT {
         cap_sgs[q] = cap(fs[q], SgsShape<T>::threads, smem_sgs);
       }
     }
-    grid_cap[2] = cap((const void *)k_fftx_fwd<T>, kFFTThreads, smem_x);
-    grid_cap[3] = cap((const void *)k_ffty<T>, kFFTThreads, smem_y);
+    grid_cap[2] = cap((const void *)k_fftx_fwd_any<T>, kFFTThreadsX, smem_x);
+    grid_cap[3] = cap((const void *)k_ffty_any<T, false>, kFFTThreads, smem_y);
     grid_cap[4] = cap((const void *)k_tri<T>, kTriThreads, smem_tri);
-    grid_cap[5] = cap((const void *)k_fftx_inv<T>, kFFTThreads, smem_x);
+    grid_cap[5] = cap((const void *)k_fftx_inv_any<T>, kFFTThreadsX, smem_x);
     grid_cap[6] = cap((const void *)k_project<T>, MX * MY, 0);
     grid_cap[10] = std::is_same<T, float>::value ? cap((const void *)k_project_pair, MX * MY / 2, 0) : 1;
     grid_cap[7] = cap((const void *)k_divres<T>, TX * TY, 0);
@@ -821,11 +864,16 @@ struct BatchT {
     switch (kind) {
       case LK_CELLS: return ntx * nty * h.nz;
       case LK_BOX: return ((h.nx + 2 + TX - 1) / TX) * ((h.ny + 2 + TY - 1) / TY) * (h.nz + 2);
-      case LK_ROWS: return fft_reg_supported(h.nx) ? 0 : (h.ny * h.nz + kRowsX - 1) / kRowsX;
+      case LK_ROWS: {
+        if (fft_reg_supported(h.nx)) return 0;
+        const int rows = 2 * fft_any_seqs<T>(h.nx);
+        return (h.ny * h.nz + rows - 1) / rows;
+      }
       case LK_YCOLS: return fft_reg_supported(h.ny) ? 0 : ((h.nxh + TyOf<T>::v - 1) / TyOf<T>::v) * h.nz;
       case LK_MOM: return ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY) * ((h.nz + MKC - 1) / MKC);
       case LK_MOMT: return ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY) * ((h.nz + tune_mom_kc - 1) / tune_mom_kc);
       case LK_SGST: return ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY) * ((h.nz + tune_sgs_kc - 1) / tune_sgs_kc);
+      case LK_WSUM: return h.nz + 1;
       case LK_WM: return (int)((wm_points_of(h) + kWmThreads - 1) / kWmThreads);
       case LK_PROJ: return fp32_pairs(h) && !slab_mode ? 0 : tiles(LK_MOM, h);
       case LK_PROJ2: return fp32_pairs(h) && !slab_mode ? tiles(LK_MOM, h) : 0;
@@ -942,6 +990,7 @@ struct BatchT {
     PoisPlan pl;
     factorize(h.nx, pl.fx);
     factorize(h.ny, pl.fy);
+    pl.nsx = fft_any_seqs<T>(h.nx);
     hplan[di] = pl;
     auto twiddles = [](int n) {
       std::vector<T2> w(n);
@@ -1134,6 +1183,9 @@ struct BatchT {
     // mixed path: the per-level offsets of U and V (zero until the first
     // upload; see Dom::voff)
     if (sizeof(T) == 4 && (r = dalloc((void **)&h.voff, sizeof(float) * 2 * (h.nz + 2)))) return r;
+    if ((r = dalloc((void **)&h.wsum, sizeof(double) * (h.nz + 2)))) return r;
+    if ((r = dalloc((void **)&h.zsol, sizeof(double) * (h.nz + 2)))) return r;
+    if ((r = dalloc((void **)&h.wticket, sizeof(int)))) return r;
     if ((r = dalloc((void **)&h.prm, sizeof(double)))) return r;
     h.nprpart = ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY);
     if ((r = dalloc((void **)&h.prpart, sizeof(double) * h.nprpart))) return r;
@@ -1341,7 +1393,7 @@ struct BatchT {
         r.k->fwd<<<std::max(1, std::min(r.ls.total, r.cap_fwd)), kRegThreads, r.smem, s>>>(ddom, r.ls.l(), coef_alpha2,
                                                                                            use_dt, rhs_from_phi, gate);
       } else {
-        k_fftx_fwd<T><<<gsz(2, ls[LK_ROWS].total), kFFTThreads, smem_x, s>>>(ddom, ls[LK_ROWS].l(), dplan, coef_alpha2,
+        k_fftx_fwd_any<T><<<gsz(2, ls[LK_ROWS].total), kFFTThreadsX, smem_x, s>>>(ddom, ls[LK_ROWS].l(), dplan, coef_alpha2,
                                                                              use_dt, rhs_from_phi, gate);
       }
     });
@@ -1355,8 +1407,8 @@ struct BatchT {
         (inverse ? r.k->yi : r.k->yf)<<<std::max(1, std::min(r.ls.total, inverse ? r.cap_inv : r.cap_fwd)),
                                          kRegThreads, r.smem, s>>>(ddom, r.ls.l(), gate);
       } else {
-        k_ffty<T><<<gsz(3, ls[LK_YCOLS].total), kFFTThreads, smem_y, s>>>(ddom, ls[LK_YCOLS].l(), dplan, inverse,
-                                                                         gate);
+        auto ky = inverse ? k_ffty_any<T, true> : k_ffty_any<T, false>;
+        ky<<<gsz(3, ls[LK_YCOLS].total), kFFTThreads, smem_y, s>>>(ddom, ls[LK_YCOLS].l(), dplan, gate);
       }
     });
   }
@@ -1387,19 +1439,19 @@ struct BatchT {
       }
     }
   }
-  void launch_tri(int gate) {
+  void launch_tri(int gate, int zsol) {
     if (ls[LK_TRIT].total > 0) {
       nlaunch++;
       if (tune_cols == 16)
         k_tri_tile<T, 16><<<gsz(13, ls[LK_TRIT].total), tri_tile_threads<16>(), smem_trit, stream>>>(
-            ddom, ls[LK_TRIT].l(), gate);
+            ddom, ls[LK_TRIT].l(), gate, zsol);
       else
         k_tri_tile<T, 32><<<gsz(15, ls[LK_TRIT].total), tri_tile_threads<32>(), smem_trit32, stream>>>(
-            ddom, ls[LK_TRIT].l(), gate);
+            ddom, ls[LK_TRIT].l(), gate, zsol);
     }
     if (ls[LK_TRI].total > 0) {
       nlaunch++;
-      k_tri<T><<<gsz(4, ls[LK_TRI].total), kTriThreads, smem_tri, stream>>>(ddom, ls[LK_TRI].l(), gate);
+      k_tri<T><<<gsz(4, ls[LK_TRI].total), kTriThreads, smem_tri, stream>>>(ddom, ls[LK_TRI].l(), gate, zsol);
     }
   }
   void launch_fftx_inv(int gate) {
@@ -1410,17 +1462,30 @@ struct BatchT {
         const RegSet &r = xreg[q];
         r.k->inv<<<std::max(1, std::min(r.ls.total, r.cap_inv)), kRegThreads, r.smem, s>>>(ddom, r.ls.l(), gate);
       } else {
-        k_fftx_inv<T><<<gsz(5, ls[LK_ROWS].total), kFFTThreads, smem_x, s>>>(ddom, ls[LK_ROWS].l(), dplan, gate);
+        k_fftx_inv_any<T><<<gsz(5, ls[LK_ROWS].total), kFFTThreadsX, smem_x, s>>>(ddom, ls[LK_ROWS].l(), dplan, gate);
       }
     });
   }
+  // the level sums of W2 and the (0,0) mode from them (k_wsum) on a branch,
+  // beside the forward transforms; joined before the z solve
+  void fork_wsum(double coef_alpha2, int use_dt) {
+    cudaEventRecord(ev_fork, stream);
+    cudaStreamWaitEvent(branch[kBranches], ev_fork, 0);
+    nlaunch++;
+    k_wsum<T><<<std::min(ls[LK_WSUM].total, 148 * 4), kWsumThreads, 0, branch[kBranches]>>>(ddom, ls[LK_WSUM].l(), coef_alpha2, use_dt);
+    cudaEventRecord(ev_join[kBranches], branch[kBranches]);
+  }
+  void join_wsum() { cudaStreamWaitEvent(stream, ev_join[kBranches], 0); }
   // the five transform kernels; rhs_from_phi: the right-hand side is in Phi.
   // Phi gets no ghost pass: its only reader, k_project, folds the i+1, j+1,
   // k+1 neighbours on the box faces itself.
   void launch_poisson(double coef_alpha2, int use_dt, int rhs_from_phi, int gate) {
+    const bool zsol = !rhs_from_phi;
+    if (zsol) fork_wsum(coef_alpha2, use_dt);
     launch_fftx_fwd(coef_alpha2, use_dt, rhs_from_phi, gate);
     launch_ffty(0, gate);
-    launch_tri(gate);
+    if (zsol) join_wsum();
+    launch_tri(gate, zsol);
     launch_ffty(1, gate);
     launch_fftx_inv(gate);
   }
@@ -1610,7 +1675,7 @@ struct BatchT {
       for (int v = 0; v < 2 && !r; v++) {
         tune_cols = v ? 32 : 16;
         if ((r = rebuild_ls(LK_TRIT))) break;
-        tune_ms[2 + v] = time10([&] { launch_tri(0); });
+        tune_ms[2 + v] = time10([&] { launch_tri(0, 0); });
       }
       tune_cols = tune_ms[3] < tune_ms[2] ? 32 : 16;
       if (!r) r = rebuild_ls(LK_TRIT);
@@ -2237,7 +2302,7 @@ struct BatchT {
       });
       timed(2, [&] { launch_fftx_fwd(a2, 1, 0, 0); });
       timed(3, [&] { launch_ffty(0, 0); });
-      timed(4, [&] { launch_tri(0); });
+      timed(4, [&] { launch_tri(0, 1); });
       timed(5, [&] { launch_ffty(1, 0); });
       timed(6, [&] { launch_fftx_inv(0); });
       timed(7, [&] { k_project_any(a2, 1, 0, 0); });
@@ -3318,9 +3383,7 @@ static int noalloc_setup(int device, NoAllocDev *out) {
   int optin = 0, nsm = 0;
   CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-  CU(cudaFuncSetAttribute(k_fftx_fwd<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  CU(cudaFuncSetAttribute(k_fftx_inv<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  CU(cudaFuncSetAttribute(k_ffty<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+  CU(fft_any_attributes<double>(optin));
   CU(cudaFuncSetAttribute(k_tri<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
   nd.base = ptr;
   nd.optin = optin;
@@ -3381,11 +3444,12 @@ extern "C" int elmm_poisson_solve_noalloc(const int32_t n[3], const double L[3],
   NoAllocDev nd;
   if ((r = noalloc_setup(device, &nd))) return r;
   unsigned char *base = nd.base;
-  const size_t smem_x = sizeof(double2) * 2 * (kRowsX / 2) * nx, smem_y = sizeof(double2) * 2 * TyOf<double>::v * ny;
+  const int nsx = fft_any_seqs<double>(nx);
+  const size_t smem_x = fft_any_smem_x<double>(nx, nsx), smem_y = fft_any_smem_y<double>(ny);
   const int zper = bcs[ELMM_BO] == ELMM_BC_PERIODIC;
   const size_t smem_tri = sizeof(double) * kTriThreads * nz * (zper ? 2 : 1);
   const size_t optin = (size_t)nd.optin;
-  if (smem_x > optin || smem_y > optin || smem_tri > optin)
+  if (transforms_too_long<double>(nx, ny, nd.optin) || smem_tri > optin)
     return fail(ELMM_ERR_INVALID_CONFIG, "grid too large for the shared-memory transforms");
 
   Dom<double> h;
@@ -3410,6 +3474,7 @@ extern "C" int elmm_poisson_solve_noalloc(const int32_t n[3], const double L[3],
   PoisPlan pl;
   factorize(nx, pl.fx);
   factorize(ny, pl.fy);
+  pl.nsx = nsx;
   const Dom<double> *ddom = reinterpret_cast<const Dom<double> *>(base + lay.dom);
   const PoisPlan *dplan = reinterpret_cast<const PoisPlan *>(base + lay.plan);
   const int *starts = reinterpret_cast<const int *>(base + lay.starts);
@@ -3420,7 +3485,7 @@ extern "C" int elmm_poisson_solve_noalloc(const int32_t n[3], const double L[3],
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, threads, smem) != cudaSuccess || b < 1) b = 1;
     return std::max(1, std::min(total, b * nsm));
   };
-  const Launch rows{starts, 1, (ny * nz + kRowsX - 1) / kRowsX};
+  const Launch rows{starts, 1, (ny * nz + 2 * nsx - 1) / (2 * nsx)};
   const Launch ycols{starts, 1, ((nxh + TyOf<double>::v - 1) / TyOf<double>::v) * nz};
   const Launch tri{starts, 1, (ny * spitch + kTriThreads - 1) / kTriThreads};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -3430,15 +3495,15 @@ extern "C" int elmm_poisson_solve_noalloc(const int32_t n[3], const double L[3],
   // point never reads it back (it would have to synchronise), so non-finite
   // input is not reported, as the header states
   k_unpack<double><<<256, 256, 0, st>>>(ddom, h.Phi, RHS, HostBox{0, nx + 2, ny + 2, nz + 2}, nx, ny, nz, bad);
-  k_fftx_fwd<double><<<blocks((const void *)k_fftx_fwd<double>, kFFTThreads, smem_x, rows.total), kFFTThreads, smem_x,
-                       st>>>(ddom, rows, dplan, 1.0, 0, 1, 0);
-  const int gy = blocks((const void *)k_ffty<double>, kFFTThreads, smem_y, ycols.total);
-  k_ffty<double><<<gy, kFFTThreads, smem_y, st>>>(ddom, ycols, dplan, 0, 0);
+  k_fftx_fwd_any<double><<<blocks((const void *)k_fftx_fwd_any<double>, kFFTThreadsX, smem_x, rows.total), kFFTThreadsX,
+                           smem_x, st>>>(ddom, rows, dplan, 1.0, 0, 1, 0);
+  const int gy = blocks((const void *)k_ffty_any<double, false>, kFFTThreads, smem_y, ycols.total);
+  k_ffty_any<double, false><<<gy, kFFTThreads, smem_y, st>>>(ddom, ycols, dplan, 0);
   k_tri<double><<<blocks((const void *)k_tri<double>, kTriThreads, smem_tri, tri.total), kTriThreads, smem_tri, st>>>(
-      ddom, tri, 0);
-  k_ffty<double><<<gy, kFFTThreads, smem_y, st>>>(ddom, ycols, dplan, 1, 0);
-  k_fftx_inv<double><<<blocks((const void *)k_fftx_inv<double>, kFFTThreads, smem_x, rows.total), kFFTThreads, smem_x,
-                       st>>>(ddom, rows, dplan, 0);
+      ddom, tri, 0, 0);
+  k_ffty_any<double, true><<<gy, kFFTThreads, smem_y, st>>>(ddom, ycols, dplan, 0);
+  k_fftx_inv_any<double><<<blocks((const void *)k_fftx_inv_any<double>, kFFTThreadsX, smem_x, rows.total), kFFTThreadsX,
+                           smem_x, st>>>(ddom, rows, dplan, 0);
   k_pack_scalar<double><<<256, 256, 0, st>>>(ddom, h.Phi, Phi, HostBox{-1, nx + 4, ny + 4, nz + 4}, 0, 0, nx, ny, nz);
   CU(cudaGetLastError());
   return ELMM_OK;

@@ -117,6 +117,11 @@ struct Dom {
   const double *lamx, *lamy, *Ab, *At, *dzc, *dzf;
   const double *tri_c0;  // [piece][ny * spitch]: carry of the pivot recurrence at each piece start (tiled z solve)
   int zper;
+  // sums of W2 over each level in FP64, index k (0: a slab's bottom ghost
+  // level), the solution of the (0,0) mode from them, index 1..nz, and the
+  // count of the levels done (k_wsum)
+  double *wsum, *zsol;
+  int *wticket;
   // grid tables (FP64), index k + 2 for k in [-2, nz + 3]
   const double *zPr, *dzPr, *zW, *dzW;
   const double *width;   // Smagorinsky filter width per k, index k (1..nz)

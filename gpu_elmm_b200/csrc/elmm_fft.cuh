@@ -1,11 +1,8 @@
-// elmm_fft.cuh -- in-shared-memory mixed-radix FFT (Stockham autosort).
+// elmm_fft.cuh -- the plan of a mixed-radix FFT and its small DFTs.
 //
 // Used by the Poisson solve that replaces the PoisFFT call of
 // src/poisson.f90:76-210: real-to-complex transforms along x, complex
-// transforms along y.  A block transforms `ntr` sequences of length N held
-// contiguously in shared memory; each pass applies radix-R butterflies with
-// twiddles from a per-length table tw[m] = exp(-2 pi i m / N) and writes the
-// result in natural order into the other buffer (no bit reversal).
+// transforms along y (elmm_fftreg.cuh, elmm_poisson_any.cuh).
 #pragma once
 
 #include "elmm_common.cuh"
@@ -14,10 +11,15 @@ namespace elmm {
 
 constexpr int kMaxFac = 12;
 
+// Passes of a length n: pass p takes blocks of fac[p] M[p] elements apart
+// with radix fac[p]; step[p] = n / (fac[p] M[p]) is the product of the
+// radices before it, magic[p] = ceil(2^32 / M[p]) divides by M[p] (exact for
+// dividends and M below 2^16).
 struct FFTFactors {
   int n;
   int nfac;
-  int fac[kMaxFac];
+  int fac[kMaxFac], M[kMaxFac], step[kMaxFac];
+  unsigned magic[kMaxFac];
 };
 
 template <typename T2>
@@ -87,51 +89,6 @@ __device__ __forceinline__ void dft_small(T2 *v, int R, bool inv) {
     v[2] = cadd(m2, n2);
     v[3] = csub(m2, n2);
   }
-}
-
-// Transforms ntr sequences of length f.n stored back to back in buf0;
-// returns the buffer (buf0 or buf1) that holds the result.  All threads of
-// the block must call it; it ends with __syncthreads().
-template <typename T, typename T2>
-__device__ T2 *fft_block(T2 *buf0, T2 *buf1, int ntr, const FFTFactors &f, const T2 *__restrict__ tw,
-                         bool inv) {
-  const int N = f.n;
-  T2 *src = buf0, *dst = buf1;
-  int Ns = 1;
-  for (int p = 0; p < f.nfac; p++) {
-    const int R = f.fac[p];
-    const int nb = N / R;
-    const int tstep = N / (Ns * R);
-    for (int w = threadIdx.x; w < nb * ntr; w += blockDim.x) {
-      int tr = w / nb;
-      int j = w - tr * nb;
-      const T2 *s = src + tr * N;
-      T2 *o = dst + tr * N;
-      int jm = j % Ns;
-      T2 v[5];
-#pragma unroll
-      for (int r = 0; r < 5; r++) {
-        if (r < R) {
-          T2 x = s[j + r * nb];
-          if (r > 0 && jm > 0) {
-            T2 t = __ldg(&tw[r * jm * tstep]);
-            if (inv) t.y = -t.y;
-            x = cmul(x, t);
-          }
-          v[r] = x;
-        }
-      }
-      dft_small<T, T2>(v, R, inv);
-      int od = (j - jm) * R + jm;
-#pragma unroll
-      for (int r = 0; r < 5; r++)
-        if (r < R) o[od + r * Ns] = v[r];
-    }
-    __syncthreads();
-    T2 *t = src; src = dst; dst = t;
-    Ns *= R;
-  }
-  return src;
 }
 
 }  // namespace elmm

@@ -1,0 +1,19 @@
+// elmm_fft_table.cuh -- the dispatch table of the register transforms.
+#pragma once
+
+#include "elmm_kernels.cuh"
+#include "elmm_poisson_reg.cuh"
+
+namespace elmm {
+
+template <typename T>
+const FFTRegKernels<T> *fft_reg_kernels(int n) {
+#define ELMM_REG_ENTRY(n_) {n_, k_fftx_fwd_reg<T, n_>, k_fftx_inv_reg<T, n_>, k_ffty_reg<T, n_, false>, k_ffty_reg<T, n_, true>},
+  static const FFTRegKernels<T> table[] = {ELMM_FFT_SIZES(ELMM_REG_ENTRY)};
+#undef ELMM_REG_ENTRY
+  for (const auto &e : table)
+    if (e.n == n) return &e;
+  return nullptr;
+}
+
+}  // namespace elmm

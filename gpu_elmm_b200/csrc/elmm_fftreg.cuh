@@ -141,8 +141,12 @@ struct FPlan {
   static_assert(P >= 2 && E >= P, "plan");
 };
 
-// Lengths with a register FFT; the generic transform handles the others.
-#define ELMM_FFT_SIZES(X) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384)
+// Lengths with a register FFT: the multiples of 16 from 32 to 512 that factor
+// into 2, 3 and 5 (rows of whole 16-byte vectors, at most 32 elements per
+// thread); the generic transform handles the others.
+#define ELMM_FFT_SIZES(X)                                                                                      \
+  X(32) X(48) X(64) X(80) X(96) X(128) X(144) X(160) X(192) X(240) X(256) X(288) X(320) X(384) X(400) X(432) \
+      X(480) X(512)
 
 __host__ __device__ constexpr bool fft_reg_supported(int n) {
 #define ELMM_FFT_CASE(n_) (n) == (n_) ||

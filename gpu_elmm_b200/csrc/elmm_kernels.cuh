@@ -392,130 +392,125 @@ __global__ void __launch_bounds__(kWmThreads) k_wm_points(const Dom<T> *__restri
 namespace elmm {
 
 // ------------------------------------------------------------- Poisson
-// FFT factorisations and plan of one domain, passed by value
-struct PoisPlan {
-  FFTFactors fx, fy;
-};
-
-constexpr int kRowsX = 8;  // real rows per block of the x transforms
-constexpr int kFFTThreads = 256;
-
-// divergence RHS of PrePoisson (pressure.f90:688-717, Q = 0) fused with the
-// forward real FFT along x of kRowsX rows (two real rows per complex FFT).
+// Sums of W2 over each level, FP64, one block a level in a fixed order, and
+// from them the (0,0) mode of the Poisson problem (src/poisson.f90:23-60):
+// the mean divergence of a level, whose x and y parts telescope to nothing,
+// is the difference of two of these sums, so the flux of the mode through a
+// level's top is the sum itself (less the bottom's) and its solution one
+// prefix sum, which the domain's last block takes, its mean pinned to zero.
+// Taken from the FP32 transform instead, the mode's rounding, independent
+// from level to level, is integrated twice: a large and, as one mode's, a
+// very uneven part of the error of the mixed pressure (64 x 64 x 32 after 40
+// steps: 3.2e-4 of the pressure, 1.4e-4 with the sums); and the serial sum
+// was the longest chain of the z solve on small grids.  One word per cell,
+// on a graph branch beside the forward transforms: wide blocks with kVec
+// vectors in flight per thread.  The mixed step of 256 x 256 x 128 takes 2.5%
+// longer with it (the z solve 10 us a stage less, the branch more), that of
+// 64 x 64 x 32 2% less.
+constexpr int kWsumThreads = 512;
 template <typename T>
-__global__ void __launch_bounds__(kFFTThreads) k_fftx_fwd(const Dom<T> *__restrict__ doms, Launch L,
-                                                  const PoisPlan *__restrict__ plans, double coef_alpha2,
-                                                  int use_dt, int rhs_from_phi, int gate) {
-  typedef typename Vec2<T>::type T2;
-  extern __shared__ unsigned char smem_raw[];
-  T2 *buf0 = reinterpret_cast<T2 *>(smem_raw);
+__global__ void __launch_bounds__(kWsumThreads, 2) k_wsum(const Dom<T> *__restrict__ doms, Launch L, double coef_alpha2,
+                                                       int use_dt) {
+  __shared__ double red[kWsumThreads / 32];
+  __shared__ int last;
+  constexpr int kVec = 8, VE = 16 / (int)sizeof(T);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
     const int di = find_dom(L.starts, L.nd, t);
     const Dom<T> &d = doms[di];
-    if (gate && !*d.refine_flag) continue;  // defect-correction sweep not needed
-    const PoisPlan &pl = plans[di];
-    const int N = d.nx;
-    const int ntr = kRowsX / 2;
-    T2 *buf1 = buf0 + ntr * N;
-    const int lt = t - __ldg(L.starts + di);
-    const int row0 = lt * kRowsX;
-    const int nrows = d.ny * d.nz;
-    const double coef = use_dt ? coef_alpha2 * d.dt : coef_alpha2;
-    const T rdt2 = (T)(1.0 / coef);
-    const T *U2 = d.U2, *V2 = d.V2, *W2 = d.W2;
-    const T rdx = (T)(1.0 / d.dx), rdy = (T)(1.0 / d.dy), rdz = (T)(1.0 / d.dz);
-#pragma unroll 4
-    for (int w = threadIdx.x; w < kRowsX * N; w += blockDim.x) {
-      const int r = w / N, i = w - r * N + 1;
-      const int row = row0 + r;
-      T rhs = 0;
-      if (row < nrows) {
-        const int j = row % d.ny + 1, k = row / d.ny + 1;
-        const long long c = bidx(d, i, j, k);
-        if (rhs_from_phi) {  // the RHS was put in Phi (PoisSolver interface, defect correction)
-          rhs = ld((const T *)d.Phi, c) * rdt2;
-        } else {
-          const T rdzk = d.vz ? (T)d.sgs_rdz[k] : rdz;
-          // on a box face the neighbours fold onto the interior (BoundUVW)
-          const bool face = i == 1 || i > d.ext[0][0] || j == 1 || j > d.ext[1][1] || k == 1 || k > d.ext[2][2] ||
-                            j > d.ext[0][1] || j > d.ext[2][1] || k > d.ext[0][2] || k > d.ext[1][2];
-          T uc, uw, vc, vs, wc, wb;
-          if (!face) {
-            uc = ld(U2, c); uw = ld(U2, c - 1);
-            vc = ld(V2, c); vs = ld(V2, c - d.pitch);
-            wc = ld(W2, c); wb = ld(W2, c - d.plane);
-          } else {
-            uc = vel_folded(d, U2, 0, i, j, k); uw = vel_folded(d, U2, 0, i - 1, j, k);
-            vc = vel_folded(d, V2, 1, i, j, k); vs = vel_folded(d, V2, 1, i, j - 1, k);
-            wc = vel_folded(d, W2, 2, i, j, k); wb = vel_folded(d, W2, 2, i, j, k - 1);
+    const int k = t - __ldg(L.starts + di);
+    const int nx = d.nx, ny = d.ny, nz = d.nz;
+    if (k <= d.ext[2][2] && (k > 0 || d.bt[SIDE_BO] == BC_HALO)) {
+      const long long pitch = d.pitch;
+      const T *W = d.W2 + bidx(d, 1, 1, k);
+      double s = 0;
+      if (nx % VE == 0) {
+        const int nv = nx / VE, n = nv * ny;  // 16-byte vectors of the level
+        for (int q0 = threadIdx.x; q0 < n; q0 += kWsumThreads * kVec) {
+          float4 v[kVec];
+#pragma unroll
+          for (int u = 0; u < kVec; u++) {
+            const int q = q0 + u * kWsumThreads, j = q / nv;
+            v[u] = q < n ? __ldg(reinterpret_cast<const float4 *>(W + j * pitch) + (q - j * nv)) : make_float4(0, 0, 0, 0);
           }
-          T div = (uc - uw) * rdx + (vc - vs) * rdy + (wc - wb) * rdzk;
-          rhs = div * rdt2;
+#pragma unroll
+          for (int u = 0; u < kVec; u++) {
+            const T *e = reinterpret_cast<const T *>(&v[u]);
+#pragma unroll
+            for (int c = 0; c < VE; c++) s += (double)e[c];
+          }
+        }
+      } else {
+        const int n = nx * ny;
+        for (int q0 = threadIdx.x; q0 < n; q0 += kWsumThreads * kVec) {
+          T v[kVec];
+#pragma unroll
+          for (int u = 0; u < kVec; u++) {
+            const int q = q0 + u * kWsumThreads, j = q / nx;
+            v[u] = q < n ? __ldg(W + j * pitch + (q - j * nx)) : (T)0;
+          }
+#pragma unroll
+          for (int u = 0; u < kVec; u++) s += (double)v[u];
         }
       }
-      T2 *z = buf0 + (r >> 1) * N + (i - 1);
-      if (r & 1) z->y = rhs; else z->x = rhs;
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) red[warp] = s;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double tot = 0;
+        for (int w = 0; w < kWsumThreads / 32; w++) tot += red[w];
+        d.wsum[k] = tot;
+      }
+    }
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(d.wticket, 1) == nz;  // nz + 1 tiles
+      if (last) *d.wticket = 0;
     }
     __syncthreads();
-    T2 *res = fft_block<T, T2>(buf0, buf1, ntr, pl.fx, d.twx, false);
-    // split Z = FFT(a + i b) into the half spectra of a and b
-    const int nxh = d.nxh;
-#pragma unroll 4
-    for (int w = threadIdx.x; w < ntr * nxh; w += blockDim.x) {
-      const int p = w / nxh, m = w - p * nxh;
-      const T2 *Z = res + p * N;
-      T2 zk = Z[m], zc = Z[m == 0 ? 0 : N - m];
-      T2 A, B;
-      A.x = (zk.x + zc.x) * (T)0.5;
-      A.y = (zk.y - zc.y) * (T)0.5;
-      B.x = (zk.y + zc.y) * (T)0.5;
-      B.y = (zc.x - zk.x) * (T)0.5;
-      const int ra = row0 + 2 * p, rb = ra + 1;
-      if (ra < nrows) d.S[((long long)(ra / d.ny) * d.ny + ra % d.ny) * d.spitch + m] = A;
-      if (rb < nrows) d.S[((long long)(rb / d.ny) * d.ny + rb % d.ny) * d.spitch + m] = B;
-    }
-    __syncthreads();
-  }
-}
-
-// complex FFT along y of a tile of kTy columns (kx) of one k plane
-template <typename T> struct TyOf;
-template <> struct TyOf<double> { static constexpr int v = 8; };
-template <> struct TyOf<float> { static constexpr int v = 16; };
-
-template <typename T>
-__global__ void __launch_bounds__(kFFTThreads) k_ffty(const Dom<T> *__restrict__ doms, Launch L,
-                                              const PoisPlan *__restrict__ plans, int inverse, int gate) {
-  typedef typename Vec2<T>::type T2;
-  constexpr int C = TyOf<T>::v;
-  extern __shared__ unsigned char smem_raw[];
-  T2 *buf0 = reinterpret_cast<T2 *>(smem_raw);
-  for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
-    const int di = find_dom(L.starts, L.nd, t);
-    const Dom<T> &d = doms[di];
-    if (gate && !*d.refine_flag) continue;  // defect-correction sweep not needed
-    const PoisPlan &pl = plans[di];
-    const int N = d.ny;
-    T2 *buf1 = buf0 + C * N;
-    const int lt = t - __ldg(L.starts + di);
-    const int ncx = (d.nxh + C - 1) / C;
-    const int cx = lt % ncx, k = lt / ncx;
-    const int kx0 = cx * C;
-    T2 *S = d.S + (long long)k * d.ny * d.spitch;
-#pragma unroll 4
-    for (int w = threadIdx.x; w < C * N; w += blockDim.x) {
-      const int j = w / C, c = w - j * C;
-      T2 v;
-      if (kx0 + c < d.nxh) v = S[(long long)j * d.spitch + kx0 + c];
-      else { v.x = 0; v.y = 0; }
-      buf0[c * N + j] = v;
-    }
-    __syncthreads();
-    T2 *res = fft_block<T, T2>(buf0, buf1, C, pl.fy, d.twy, inverse != 0);
-#pragma unroll 4
-    for (int w = threadIdx.x; w < C * N; w += blockDim.x) {
-      const int j = w / C, c = w - j * C;
-      if (kx0 + c < d.nxh) S[(long long)j * d.spitch + kx0 + c] = res[c * N + j];
+    if (last && d.bt[SIDE_BO] != BC_HALO && d.bt[SIDE_TO] != BC_HALO) {
+      __threadfence();
+      // x(k + 1) = x(k) + (F(k) + F0) dzf(k) with F(k) = (level(k) - level(0)) rdt norm
+      const double c = 1.0 / (use_dt ? coef_alpha2 * d.dt : coef_alpha2) * (1.0 / ((double)nx * (double)ny));
+      auto level = [&](int g) {
+        const Fold f = fold_vel(g, d.ext[2][2], d.bt[4], d.bt[5], true);
+        return f.zero ? 0.0 : f.sign * __ldcg(d.wsum + f.src);
+      };
+      const double l0 = level(0);
+      auto block_sum = [&](double v, double &before) -> double {  // the block's sum, and the sum of the threads before
+        double x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= o) x += y;
+        }
+        __syncthreads();
+        if (lane == 31) red[warp] = x;
+        __syncthreads();
+        double tot = 0, pre = 0;
+        for (int w = 0; w < kWsumThreads / 32; w++) {
+          if (w < warp) pre += red[w];
+          tot += red[w];
+        }
+        before = pre + (x - v);
+        return tot;
+      };
+      const int per = (nz + kWsumThreads - 1) / kWsumThreads, k0 = 1 + threadIdx.x * per, k1 = min(nz, k0 + per - 1);
+      double F0 = 0, before;
+      if (d.zper) {  // so that x is periodic: sum_k dzf(k) (F(k) + F0) = 0
+        double a = 0, b = 0;
+        for (int q = k0; q <= k1; q++) { a += (level(q) - l0) * c * d.dzf[q]; b += d.dzf[q]; }
+        const double sa = block_sum(a, before), sb = block_sum(b, before);
+        F0 = -sa / sb;
+      }
+      double g = 0;  // the increments of this thread's levels
+      for (int q = k0; q <= k1; q++) g += ((level(q) - l0) * c + F0) * d.dzf[q];
+      block_sum(g, before);
+      double x = before, sx = 0;
+      for (int q = k0; q <= k1; q++) { sx += x; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
+      double unused;
+      const double mean = block_sum(sx, unused) / nz;
+      x = before;
+      for (int q = k0; q <= k1; q++) { d.zsol[q] = x - mean; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
     }
     __syncthreads();
   }
@@ -523,12 +518,13 @@ __global__ void __launch_bounds__(kFFTThreads) k_ffty(const Dom<T> *__restrict__
 
 // Tridiagonal solve in z for each (kx, ky): the Thomas algorithm in FP64 on
 // the rows of Residue_variable_z (poisson.f90:23-60), Neumann rows at the
-// ends or a cyclic system for periodic z; the (0,0) mode is singular and is
-// solved by two prefix sums with its mean pinned to zero.
+// ends or a cyclic system for periodic z; the (0,0) mode is singular: k_wsum has
+// its solution (zsol), or, for a right-hand side that is not a divergence, it
+// is solved by two prefix sums with its mean pinned to zero.
 constexpr int kTriThreads = 64;
 
 template <typename T>
-__global__ void __launch_bounds__(kTriThreads) k_tri(const Dom<T> *__restrict__ doms, Launch L, int gate) {
+__global__ void __launch_bounds__(kTriThreads) k_tri(const Dom<T> *__restrict__ doms, Launch L, int gate, int zsol) {
   typedef typename Vec2<T>::type T2;
   extern __shared__ double cps[];  // [nz][kTriThreads]
   for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
@@ -546,28 +542,62 @@ __global__ void __launch_bounds__(kTriThreads) k_tri(const Dom<T> *__restrict__ 
     const double lam = d.lamx[kx] + d.lamy[ky];
     const double *Ab = d.Ab, *At = d.At;
     if (kx == 0 && ky == 0) {
-      // singular mode: F(k) = F(k-1) + dzc(k) r(k) is the flux (x(k+1)-x(k))/dzf(k)
+      if (zsol) {  // solved by k_wsum
+#pragma unroll 4
+        for (int k = 1; k <= nz; k++) {
+          T2 o; o.x = (T)d.zsol[k]; o.y = (T)0;
+          S[(long long)(k - 1) * ps] = o;
+        }
+        continue;
+      }
+      // singular mode: F(k) = F(k-1) + dzc(k) r(k) is the flux (x(k+1)-x(k))/dzf(k);
+      // the right-hand sides are fetched kPre at a time, so that their loads
+      // are in flight together
+      constexpr int kPre = 8;
+      auto rhs = [&](int kb2, int ke2, double (&rx)[kPre], double (&ry)[kPre]) {
+#pragma unroll
+        for (int q = 0; q < kPre; q++) {
+          rx[q] = ry[q] = 0;
+          if (kb2 + q <= ke2) {
+            const T2 r = S[(long long)(kb2 + q - 1) * ps];
+            rx[q] = ((double)r.x * norm) * d.dzc[kb2 + q];
+            ry[q] = ((double)r.y * norm) * d.dzc[kb2 + q];
+          }
+        }
+      };
       double F0x = 0, F0y = 0;
       if (d.zper) {  // choose F(0) so that x is periodic: sum_k dzf(k) F(k) = 0
         double Fx = 0, Fy = 0, swx = 0, swy = 0, sd = 0;
-        for (int k = 1; k <= nz; k++) {
-          T2 r = S[(long long)(k - 1) * ps];
-          Fx = Fx + ((double)r.x * norm) * d.dzc[k];
-          Fy = Fy + ((double)r.y * norm) * d.dzc[k];
-          swx += Fx * d.dzf[k]; swy += Fy * d.dzf[k]; sd += d.dzf[k];
+        for (int kb2 = 1; kb2 <= nz; kb2 += kPre) {
+          double rx[kPre], ry[kPre];
+          rhs(kb2, nz, rx, ry);
+#pragma unroll
+          for (int q = 0; q < kPre; q++) {
+            const int k = kb2 + q;
+            if (k > nz) break;
+            Fx = Fx + rx[q];
+            Fy = Fy + ry[q];
+            swx += Fx * d.dzf[k]; swy += Fy * d.dzf[k]; sd += d.dzf[k];
+          }
         }
         F0x = -swx / sd; F0y = -swy / sd;
       }
       double Fx = 0, Fy = 0, xx = 0, xy = 0, sx = 0, sy = 0;
-      for (int k = 1; k <= nz - 1; k++) {
-        T2 r = S[(long long)(k - 1) * ps];
-        Fx = Fx + ((double)r.x * norm) * d.dzc[k];
-        Fy = Fy + ((double)r.y * norm) * d.dzc[k];
-        T2 o; o.x = (T)xx; o.y = (T)xy;
-        S[(long long)(k - 1) * ps] = o;  // x(k)
-        sx += xx; sy += xy;
-        xx = xx + (Fx + F0x) * d.dzf[k];
-        xy = xy + (Fy + F0y) * d.dzf[k];
+      for (int kb2 = 1; kb2 <= nz - 1; kb2 += kPre) {
+        double rx[kPre], ry[kPre];
+        rhs(kb2, nz - 1, rx, ry);
+#pragma unroll
+        for (int q = 0; q < kPre; q++) {
+          const int k = kb2 + q;
+          if (k > nz - 1) break;
+          Fx = Fx + rx[q];
+          Fy = Fy + ry[q];
+          T2 o; o.x = (T)xx; o.y = (T)xy;
+          S[(long long)(k - 1) * ps] = o;  // x(k)
+          sx += xx; sy += xy;
+          xx = xx + (Fx + F0x) * d.dzf[k];
+          xy = xy + (Fy + F0y) * d.dzf[k];
+        }
       }
       sx += xx; sy += xy;
       sx = sx / nz; sy = sy / nz;

@@ -1,5 +1,5 @@
-// elmm_kernels2.cuh -- inverse transform, projection, reductions and the
-// host-layout pack / unpack kernels.
+// elmm_kernels2.cuh -- projection, reductions and the host-layout pack /
+// unpack kernels.
 #pragma once
 
 #include <cfloat>
@@ -7,59 +7,6 @@
 #include "elmm_kernels.cuh"
 
 namespace elmm {
-
-// inverse real FFT along x of kRowsX rows -> interior of Phi (its ghosts are
-// filled afterwards by k_ghosts)
-template <typename T>
-__global__ void __launch_bounds__(kFFTThreads) k_fftx_inv(const Dom<T> *__restrict__ doms, Launch L,
-                                                  const PoisPlan *__restrict__ plans, int gate) {
-  typedef typename Vec2<T>::type T2;
-  extern __shared__ unsigned char smem_raw[];
-  T2 *buf0 = reinterpret_cast<T2 *>(smem_raw);
-  for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
-    const int di = find_dom(L.starts, L.nd, t);
-    const Dom<T> &d = doms[di];
-    if (gate && !*d.refine_flag) continue;
-    const PoisPlan &pl = plans[di];
-    const int N = d.nx, nxh = d.nxh;
-    const int ntr = kRowsX / 2;
-    T2 *buf1 = buf0 + ntr * N;
-    const int lt = t - __ldg(L.starts + di);
-    const int row0 = lt * kRowsX;
-    const int nrows = d.ny * d.nz;
-    // Z_m = A_m + i B_m with the Hermitian completion A_{N-m} = conj(A_m);
-    // A_0 and A_{N/2} are real for a real row.
-#pragma unroll 4
-    for (int w = threadIdx.x; w < ntr * N; w += blockDim.x) {
-      const int p = w / N, m = w - p * N;
-      const int ra = row0 + 2 * p, rb = ra + 1;
-      const int mm = m < nxh ? m : N - m;
-      const bool cj = m >= nxh;
-      T2 A, B;
-      A.x = 0; A.y = 0; B.x = 0; B.y = 0;
-      if (ra < nrows) A = d.S[((long long)(ra / d.ny) * d.ny + ra % d.ny) * d.spitch + mm];
-      if (rb < nrows) B = d.S[((long long)(rb / d.ny) * d.ny + rb % d.ny) * d.spitch + mm];
-      if (mm == 0 || 2 * mm == N) { A.y = 0; B.y = 0; }
-      if (cj) { A.y = -A.y; B.y = -B.y; }
-      T2 z;
-      z.x = A.x - B.y;
-      z.y = A.y + B.x;
-      buf0[p * N + m] = z;
-    }
-    __syncthreads();
-    T2 *res = fft_block<T, T2>(buf0, buf1, ntr, pl.fx, d.twx, true);
-#pragma unroll 4
-    for (int w = threadIdx.x; w < kRowsX * N; w += blockDim.x) {
-      const int r = w / N, i = w - r * N + 1;
-      const int row = row0 + r;
-      if (row >= nrows) continue;
-      const int j = row % d.ny + 1, k = row / d.ny + 1;
-      const T2 z = res[(r >> 1) * N + i - 1];
-      d.Phi[bidx(d, i, j, k)] = (r & 1) ? z.y : z.x;
-    }
-    __syncthreads();
-  }
-}
 
 // PostPoisson (src/pressure.f90:728-870): velocity correction, Pr += Phi and
 // the partial sums of the top layer for FixPressureToReference.  A block

@@ -14,9 +14,9 @@ namespace elmm {
 constexpr int kRegThreads = 256;
 // resident blocks per SM the x-transform kernels are compiled for: for up to
 // 16 elements per thread three (FP32, 80 registers) or two (FP64, 128
-// registers) fit without spills; longer FP32 sequences (24 elements: lengths
-// 192, 384) two blocks of 128 registers, faster than one block of ~200 (the
-// y transform of those lengths spills at 128 and keeps the compiler's choice)
+// registers) fit without spills; longer FP32 sequences (up to 32 elements)
+// two blocks of 128 registers, faster than one block of ~200 (the y
+// transform of those lengths spills at 128 and keeps the compiler's choice)
 template <typename T, int N>
 constexpr int fft_reg_min_blocks() { return N / fplan_P(N) <= 16 ? (sizeof(T) == 4 ? 3 : 2) : (sizeof(T) == 4 ? 2 : 1); }
 // the forward x transform (with the fused divergence) of FP32 lengths up to
@@ -311,15 +311,11 @@ struct FFTRegKernels {
   void (*yi)(const Dom<T> *, Launch, int);
 };
 
+// (one translation unit per type: elmm_fft_f32.cu, elmm_fft_f64.cu)
 template <typename T>
-inline const FFTRegKernels<T> *fft_reg_kernels(int n) {
-#define ELMM_REG_ENTRY(n_) {n_, k_fftx_fwd_reg<T, n_>, k_fftx_inv_reg<T, n_>, k_ffty_reg<T, n_, false>, k_ffty_reg<T, n_, true>},
-  static const FFTRegKernels<T> table[] = {ELMM_FFT_SIZES(ELMM_REG_ENTRY)};
-#undef ELMM_REG_ENTRY
-  for (const auto &e : table)
-    if (e.n == n) return &e;
-  return nullptr;
-}
+const FFTRegKernels<T> *fft_reg_kernels(int n);
+extern template const FFTRegKernels<float> *fft_reg_kernels<float>(int n);
+extern template const FFTRegKernels<double> *fft_reg_kernels<double>(int n);
 
 // sequences (x) or columns (y) one block of the register kernels handles
 __host__ __device__ constexpr int fft_reg_batch(int n) { return kRegThreads / fplan_P(n); }
@@ -339,8 +335,8 @@ __host__ __device__ constexpr int fft_reg_batch(int n) { return kRegThreads / fp
 // segment of k, the segment maps are chained through shared memory, and each
 // thread then replays its segment from the exact entry value.  The tile of S
 // is copied into shared memory with cp.async (while the pivots are rebuilt)
-// and written back at the end.  The (0,0) mode is the zero-mean prefix-sum solution of
-// the generic kernel, k_tri.
+// and written back at the end.  The (0,0) mode is k_wsum's solution (zsol) or
+// the zero-mean prefix sums of the generic kernel, k_tri.
 #ifndef ELMM_TRI_COLS
 #define ELMM_TRI_COLS 16
 #endif
@@ -392,7 +388,7 @@ __host__ __device__ __forceinline__ int tri_piv_begin(int nz, int p) {
 // c0[p * ncol + col]: c(kb - 1) of mode col = ky * spitch + kx at the first
 // level kb of each pivot piece p (0 for the first); the tiled solve rebuilds
 // the reciprocal pivots of its pieces from it
-__global__ void k_tri_factors(double *c0, const double *__restrict__ lamx, const double *__restrict__ lamy,
+static __global__ void k_tri_factors(double *c0, const double *__restrict__ lamx, const double *__restrict__ lamy,
                               const double *__restrict__ Ab, const double *__restrict__ At, int nxh, int spitch, int ny,
                               int nz) {
   const int ncol = ny * spitch;
@@ -414,7 +410,7 @@ __global__ void k_tri_factors(double *c0, const double *__restrict__ lamx, const
 // the result does not depend on it)
 template <typename T, int COLS = kTriCols>
 __global__ void __launch_bounds__(tri_tile_threads<COLS>()) k_tri_tile(const Dom<T> *__restrict__ doms, Launch L,
-                                                                      int gate) {
+                                                                      int gate, int zsol) {
   constexpr int kTriCols = COLS, kTriTileThreads = tri_tile_threads<COLS>();  // this tile's shape
   typedef typename Vec2<T>::type T2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -443,6 +439,7 @@ __global__ void __launch_bounds__(tri_tile_threads<COLS>()) k_tri_tile(const Dom
     const bool active = col < ncol && kx < d.nxh;
     const bool zero_mode = kx == 0 && ky == 0;
     const bool solve = active && !zero_mode;
+    const double norm = 1.0 / ((double)d.nx * (double)d.ny);
     const int len = (nz + kTriSegs - 1) / kTriSegs;
     const int kb = tri_seg_begin(nz, seg), ke = min(nz, kb + len - 1);  // this thread's segment, kb > ke if empty
     // the reciprocal pivots of the column, rebuilt piece by piece from the
@@ -460,7 +457,6 @@ __global__ void __launch_bounds__(tri_tile_threads<COLS>()) k_tri_tile(const Dom
     __syncthreads();
     T *x = reinterpret_cast<T *>(tile) + sys;  // element k - 1 at x[(k - 1) * XS]
     const double *iv = ivs + c;                // element k - 1 at iv[(k - 1) * kTriCols]
-    const double norm = 1.0 / ((double)d.nx * (double)d.ny);
     // forward: y(k) = a(k) + b(k) y(k-1), a = r norm iv, b = -Ab iv (b(1) = 0)
     double A = 0, B = 1;
     if (solve)
@@ -505,7 +501,9 @@ __global__ void __launch_bounds__(tri_tile_threads<COLS>()) k_tri_tile(const Dom
         x[(k - 1) * XS] = (T)xv;
       }
     }
-    if (active && zero_mode && seg == 0) {
+    if (active && zero_mode && zsol) {  // solved by k_wsum
+      for (int k = kb; k <= ke; k++) x[(k - 1) * XS] = sys & 1 ? (T)0 : (T)d.zsol[k];
+    } else if (active && zero_mode && seg == 0) {
       // F(k) = F(k-1) + dzc(k) r(k) is the flux (x(k+1) - x(k)) / dzf(k)
       double F = 0, xx = 0, sx = 0;
       for (int k = 1; k <= nz - 1; k++) {

@@ -51,12 +51,25 @@ __global__ void k_slab_tri_pivots(double *iv, const double *__restrict__ lamx, c
   }
 }
 
+// the (0,0) mode's right-hand side at a slab's level k (before the norm): the
+// real part from the level sums, as the single domain takes it
+template <typename T>
+__device__ __forceinline__ double slab_zero_rhs(const Dom<T> &d, int k, int part, double coef_alpha2, int use_dt) {
+  if (part) return 0.0;  // the mean of a real field
+  auto level = [&](int g) {
+    const Fold f = fold_vel(g, d.ext[2][2], d.bt[4], d.bt[5], true);
+    return f.zero ? 0.0 : f.sign * d.wsum[f.src];
+  };
+  return (level(k) - level(k - 1)) * (d.vz ? d.sgs_rdz[k] : 1.0 / d.dz) / (use_dt ? coef_alpha2 * d.dt : coef_alpha2);
+}
+
 // The maps of a slab's forward sweep with entry y(k0) = 0:
 // fmap[part * ncol + col] = A (part 0 real, 1 imaginary), fmap[2 * ncol + col] = B.
 // The (0,0) mode's right-hand side goes to zcol[part * nzg + k0 + k - 1].
 template <typename T>
 __global__ void k_slab_tri_fmap(const Dom<T> *__restrict__ dom, const double *__restrict__ iv, double *fmap,
-                                double *zcol, int k0, int nzg) {
+                                double *zcol, int k0, int nzg, double coef_alpha2,
+                                int use_dt) {
   const Dom<T> &d = *dom;
   const int ncol = d.ny * d.spitch, nz = d.nz;
   const long long ks = 2LL * ncol;  // T elements per level of S
@@ -67,7 +80,7 @@ __global__ void k_slab_tri_fmap(const Dom<T> *__restrict__ dom, const double *__
     if (kx >= d.nxh) continue;
     const T *x = reinterpret_cast<const T *>(d.S) + 2LL * col + part;  // level k at x[(k - 1) * ks]
     if (kx == 0 && ky == 0) {
-      for (int k = 1; k <= nz; k++) zcol[(long long)part * nzg + k0 + k - 1] = (double)x[(k - 1) * ks];
+      for (int k = 1; k <= nz; k++) zcol[(long long)part * nzg + k0 + k - 1] = slab_zero_rhs(d, k, part, coef_alpha2, use_dt);
       continue;
     }
     double A = 0, B = 1;
@@ -106,18 +119,16 @@ __global__ void k_slab_tri_fwd(const Dom<T> *__restrict__ dom, const double *__r
     if (kx == 0 && ky == 0) {
       // F(k) = F(k-1) + dzc(k) r(k) is the flux (x(k+1) - x(k)) / dzf(k)
       const double *r = zcol + (long long)part * nzg;
-      double F = 0, xx = 0, sx = 0;
-      for (int k = 1; k <= nzg - 1; k++) {
-        F = F + (r[k - 1] * norm) * dzc[k];
-        if (k > k0 && k <= k0 + nz) x[(k - k0 - 1) * ks] = (T)xx;
-        sx += xx;
-        xx = xx + F * dzf[k];
-      }
-      sx += xx;
-      sx = sx / nzg;
-      for (int k = k0 + 1; k <= k0 + nz; k++) {
-        T &e = x[(k - k0 - 1) * ks];
-        e = k < nzg ? (T)((double)e - sx) : (T)(xx - sx);
+      double sx = 0;
+      for (int pass = 0; pass < 2; pass++) {  // the mean, then the levels less the mean
+        double F = 0, xx = 0;
+        for (int k = 1; k <= nzg; k++) {
+          if (pass == 0) sx += xx;
+          else if (k > k0 && k <= k0 + nz) x[(k - k0 - 1) * ks] = (T)(xx - sx);
+          F = F + (r[k - 1] * norm) * dzc[k];
+          xx = xx + F * dzf[k];
+        }
+        if (pass == 0) sx = sx / nzg;
       }
       continue;
     }
@@ -258,7 +269,7 @@ struct SlabTile {
 template <typename T, int COLS>
 __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
     k_slab_tri_fmap_tile(const Dom<T> *__restrict__ dom, const double *__restrict__ iv, double *fmap, double *zcol,
-                         int k0, int nzg) {
+                         int k0, int nzg, double coef_alpha2, int use_dt) {
   typedef SlabTile<T, COLS> Tl;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Dom<T> &d = *dom;
@@ -281,7 +292,8 @@ __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
       if (t.part == 0) fmap[2LL * ncol + t.col] = B;
     }
     if (t.seg == 0 && t.active && t.zero)
-      for (int k = 1; k <= t.nz; k++) zcol[(long long)t.part * nzg + k0 + k - 1] = (double)t.x(k);
+      for (int k = 1; k <= t.nz; k++)
+        zcol[(long long)t.part * nzg + k0 + k - 1] = slab_zero_rhs(d, k, t.part, coef_alpha2, use_dt);
     __syncthreads();  // the shared memory is free for the next tile
   }
 }
@@ -318,18 +330,16 @@ __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
     if (t.seg == 0 && t.active && t.zero) {
       // the zero-mean solution of the whole (0,0) column (k_slab_tri_fwd)
       const double *r = zcol + (long long)t.part * nzg;
-      double F = 0, xx = 0, sx = 0;
-      for (int k = 1; k <= nzg - 1; k++) {
-        F = F + (r[k - 1] * norm) * dzc[k];
-        if (k > k0 && k <= k0 + t.nz) t.x(k - k0) = (T)xx;
-        sx += xx;
-        xx = xx + F * dzf[k];
-      }
-      sx += xx;
-      sx = sx / nzg;
-      for (int k = k0 + 1; k <= k0 + t.nz; k++) {
-        T &e = t.x(k - k0);
-        e = k < nzg ? (T)((double)e - sx) : (T)(xx - sx);
+      double sx = 0;
+      for (int pass = 0; pass < 2; pass++) {  // the mean, then the levels less the mean
+        double F = 0, xx = 0;
+        for (int k = 1; k <= nzg; k++) {
+          if (pass == 0) sx += xx;
+          else if (k > k0 && k <= k0 + t.nz) t.x(k - k0) = (T)(xx - sx);
+          F = F + (r[k - 1] * norm) * dzc[k];
+          xx = xx + F * dzf[k];
+        }
+        if (pass == 0) sx = sx / nzg;
       }
     }
     __syncthreads();  // the forward maps are read, the segments replayed

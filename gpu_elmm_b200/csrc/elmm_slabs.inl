@@ -305,8 +305,10 @@ struct SlabsT {
   int projection(double coef_alpha2, int use_dt) {
     int r;
     each([&](int, BatchT<T> &B) {
+      B.fork_wsum(coef_alpha2, use_dt);
       B.launch_fftx_fwd(coef_alpha2, use_dt, 0, 0);
       B.launch_ffty(0, 0);
+      B.join_wsum();
     });
     std::vector<Copy> cps;
     each([&](int s, BatchT<T> &B) {
@@ -314,10 +316,10 @@ struct SlabsT {
       const int ntile = (ncol + kSlabCols - 1) / kSlabCols;
       if (tiled)
         k_slab_tri_fmap_tile<T, kSlabCols><<<ntile, Tile::THREADS, smem_tile, B.stream>>>(
-            B.ddom, tri[s].iv, tri[s].fmaps + 3LL * ncol * s, tri[s].zcol, k0[s], nzg);
+            B.ddom, tri[s].iv, tri[s].fmaps + 3LL * ncol * s, tri[s].zcol, k0[s], nzg, coef_alpha2, use_dt);
       else
         k_slab_tri_fmap<T><<<(2 * ncol + 127) / 128, 128, 0, B.stream>>>(B.ddom, tri[s].iv, tri[s].fmaps + 3LL * ncol * s,
-                                                                         tri[s].zcol, k0[s], nzg);
+                                                                         tri[s].zcol, k0[s], nzg, coef_alpha2, use_dt);
       B.nlaunch++;
       for (int t = 0; t < ns; t++) {
         if (t == s) continue;
