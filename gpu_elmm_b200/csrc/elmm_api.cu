@@ -320,15 +320,16 @@ struct LaunchSet {
   int *starts = nullptr;  // device
   int total = 0;
   int nd = 0;
-  Launch l() const { return Launch{starts, nd, total}; }
+  int kc = MKC;  // planes of a tile's column (the marching kernels)
+  Launch l() const { return Launch{starts, nd, total, kc}; }
 };
 
-enum { LK_CELLS = 0, LK_BOX, LK_ROWS, LK_YCOLS, LK_TRI, LK_MOM, LK_SHELL, LK_XREG, LK_YREG, LK_TRIT, LK_TCOL, LK_DCOL,
+enum { LK_CELLS = 0, LK_BOX, LK_ROWS, LK_YCOLS, LK_TRI, LK_SHELL, LK_XREG, LK_YREG, LK_TRIT, LK_TCOL, LK_DCOL,
        LK_AVG, LK_COMMIT, LK_TPAIR, LK_PROJ, LK_PROJ2, LK_DCOL2, LK_MOMT, LK_SGST, LK_WM, LK_WSUM, LK_N };
 
 // the z-chunk lengths (planes of a tile's column) the autotuner tries for
 // the momentum and SGS kernels
-constexpr int kChunks[3] = {8, 16, 32};
+constexpr int kChunks[3] = {8, MKC, kMaxChunk};
 
 // blocks of the host-layout pack / unpack kernels (8 per SM)
 constexpr int kPackBlocks = 148 * 8;
@@ -410,7 +411,6 @@ struct BatchT {
   // the FP32 scalar stage, spectral columns of a tile of the z solve
   int tune_rows = 8, tune_cols = 16;
   int tune_mom_kc = MKC, tune_sgs_kc = MKC;  // z chunks of k_momentum and k_sgs
-  int cap_mom[3] = {1, 1, 1}, cap_sgs[3] = {1, 1, 1};  // resident-block grids per chunk choice
   bool tuned = false;
   // parallel branches for the independent per-length launches of one
   // transform phase (a batch with several x or y lengths); joined back into
@@ -705,16 +705,6 @@ struct BatchT {
     CU(cudaMemcpy(dplan, hplan.data(), sizeof(PoisPlan) * n, cudaMemcpyHostToDevice));
     r = dalloc((void **)&dbad, sizeof(int));
     if (r) return r;
-    // launch maps
-    for (int k = 0; k < LK_N; k++) {
-      std::vector<int> st(n + 1, 0);
-      for (int d = 0; d < n; d++) st[d + 1] = st[d] + tiles(k, hdom[d]);
-      ls[k].nd = n;
-      ls[k].total = st[n];
-      r = dalloc((void **)&ls[k].starts, sizeof(int) * (n + 1));
-      if (r) return r;
-      CU(cudaMemcpy(ls[k].starts, st.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
-    }
     int maxnx = 0, maxny = 0, maxnz = 0, anyzper = 0;
     for (auto &h : hdom) { maxnx = std::max(maxnx, h.nx); maxny = std::max(maxny, h.ny); maxnz = std::max(maxnz, h.nz); anyzper |= h.zper; }
     smem_x = smem_y = 0;
@@ -731,12 +721,8 @@ struct BatchT {
       return fail(ELMM_ERR_INVALID_CONFIG, "grid too large for the shared-memory transforms");
     CU((fft_any_attributes<T>(optin)));
     CU(cudaFuncSetAttribute(k_tri<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    CU(cudaFuncSetAttribute(k_momentum<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-    CU(cudaFuncSetAttribute(k_momentum<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-    CU(cudaFuncSetAttribute(k_momentum<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-    CU(cudaFuncSetAttribute(k_sgs<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-    CU(cudaFuncSetAttribute(k_sgs<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
-    CU(cudaFuncSetAttribute(k_sgs<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+    CU(cudaFuncSetAttribute(k_momentum<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+    CU(cudaFuncSetAttribute(k_sgs<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
     for (auto &h : hdom) {
       reg_x |= fft_reg_supported(h.nx);
       reg_y |= fft_reg_supported(h.ny);
@@ -763,15 +749,6 @@ struct BatchT {
     };
     grid_cap[0] = cap((const void *)k_sgs<T>, SgsShape<T>::threads, smem_sgs);
     grid_cap[1] = cap((const void *)k_momentum<T>, MomShape<T>::threads, smem_mom);
-    {
-      const void *fm[3] = {(const void *)k_momentum<T, 8>, (const void *)k_momentum<T, 16>,
-                           (const void *)k_momentum<T, 32>};
-      const void *fs[3] = {(const void *)k_sgs<T, 8>, (const void *)k_sgs<T, 16>, (const void *)k_sgs<T, 32>};
-      for (int q = 0; q < 3; q++) {
-        cap_mom[q] = cap(fm[q], MomShape<T>::threads, smem_mom);
-        cap_sgs[q] = cap(fs[q], SgsShape<T>::threads, smem_sgs);
-      }
-    }
     grid_cap[2] = cap((const void *)k_fftx_fwd_any<T>, kFFTThreadsX, smem_x);
     grid_cap[3] = cap((const void *)k_ffty_any<T, false>, kFFTThreads, smem_y);
     grid_cap[4] = cap((const void *)k_tri<T>, kTriThreads, smem_tri);
@@ -787,6 +764,28 @@ struct BatchT {
     grid_cap[11] = cap((const void *)k_scalar<T>, TX * TY, 0);
     grid_cap[12] = std::is_same<T, float>::value ? cap((const void *)k_scalar_pair<8>, SPX * 8, 0) : 1;
     grid_cap[14] = std::is_same<T, float>::value ? cap((const void *)k_scalar_pair<4>, SPX * 4, 0) : 1;
+    // launch maps, the marching kernels' chunks by their resident blocks
+    auto chunk_cap = [&](int k) {
+      switch (k) {
+        case LK_PROJ: return grid_cap[6];
+        case LK_PROJ2: return grid_cap[10];
+        case LK_TCOL: return grid_cap[11];
+        case LK_TPAIR: return grid_cap[tune_rows == 8 ? 12 : 14];
+        case LK_DCOL:
+        case LK_DCOL2: return grid_cap[7];
+        default: return 0;
+      }
+    };
+    for (int k = 0; k < LK_N; k++) {
+      if (chunk_cap(k)) ls[k].kc = short_chunk(k, MKC, chunk_cap(k));
+      std::vector<int> st(n + 1, 0);
+      for (int d = 0; d < n; d++) st[d + 1] = st[d] + tiles(k, hdom[d]);
+      ls[k].nd = n;
+      ls[k].total = st[n];
+      r = dalloc((void **)&ls[k].starts, sizeof(int) * (n + 1));
+      if (r) return r;
+      CU(cudaMemcpy(ls[k].starts, st.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
+    }
     // one launch set per distinct x (y) length, holding only its domains
     auto reg_sets = [&](bool use, bool ydir, std::vector<RegSet> &out) -> int {
       if (!use) return ELMM_OK;
@@ -859,6 +858,10 @@ struct BatchT {
   // the same for the projection (the velocity is periodic in x for every domain)
   static bool fp32_pairs(const Dom<T> &h) { return sizeof(T) == 4 && h.nx % 2 == 0 && h.bt[SIDE_WE] == BC_PERIODIC; }
 
+  // tiles of a kernel that marches up bx x by columns in chunks of its ls[kind].kc planes
+  int column_tiles(int kind, const Dom<T> &h, int bx, int by) const {
+    return ((h.nx + bx - 1) / bx) * ((h.ny + by - 1) / by) * ((h.nz + ls[kind].kc - 1) / ls[kind].kc);
+  }
   int tiles(int kind, const Dom<T> &h) const {
     int ntx = (h.nx + TX - 1) / TX, nty = (h.ny + TY - 1) / TY;
     switch (kind) {
@@ -870,13 +873,12 @@ struct BatchT {
         return (h.ny * h.nz + rows - 1) / rows;
       }
       case LK_YCOLS: return fft_reg_supported(h.ny) ? 0 : ((h.nxh + TyOf<T>::v - 1) / TyOf<T>::v) * h.nz;
-      case LK_MOM: return ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY) * ((h.nz + MKC - 1) / MKC);
-      case LK_MOMT: return ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY) * ((h.nz + tune_mom_kc - 1) / tune_mom_kc);
-      case LK_SGST: return ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY) * ((h.nz + tune_sgs_kc - 1) / tune_sgs_kc);
+      case LK_MOMT:
+      case LK_SGST: return column_tiles(kind, h, MX, MY);
       case LK_WSUM: return h.nz + 1;
       case LK_WM: return (int)((wm_points_of(h) + kWmThreads - 1) / kWmThreads);
-      case LK_PROJ: return fp32_pairs(h) && !slab_mode ? 0 : tiles(LK_MOM, h);
-      case LK_PROJ2: return fp32_pairs(h) && !slab_mode ? tiles(LK_MOM, h) : 0;
+      case LK_PROJ: return fp32_pairs(h) && !slab_mode ? 0 : column_tiles(kind, h, MX, MY);
+      case LK_PROJ2: return fp32_pairs(h) && !slab_mode ? column_tiles(kind, h, MX, MY) : 0;
       case LK_SHELL: return (int)((shell_cells(h.nx, h.ny, h.nz) + kShellThreads * shell_per - 1) / (kShellThreads * shell_per));
       case LK_XREG: {
         if (!fft_reg_supported(h.nx)) return 0;
@@ -889,14 +891,10 @@ struct BatchT {
         return ((h.nxh + C - 1) / C) * h.nz;
       }
       case LK_TRIT: return tri_tiled(h) ? (h.ny * h.spitch + tune_cols - 1) / tune_cols : 0;
-      case LK_TCOL: return scalar_pairs(h) ? 0 : ntx * nty * ((h.nz + TMKC - 1) / TMKC) * h.nslot;
-      case LK_TPAIR:
-        return scalar_pairs(h) ? ((h.nx + 2 * SPX - 1) / (2 * SPX)) * ((h.ny + tune_rows - 1) / tune_rows) *
-                                     ((h.nz + TMKC - 1) / TMKC) * h.nslot
-                               : 0;
-      case LK_DCOL: return scalar_pairs(h) ? 0 : ntx * nty * ((h.nz + kDivChunk - 1) / kDivChunk);
-      case LK_DCOL2:
-        return scalar_pairs(h) ? ((h.nx + 2 * TX - 1) / (2 * TX)) * nty * ((h.nz + kDivChunk - 1) / kDivChunk) : 0;
+      case LK_TCOL: return scalar_pairs(h) ? 0 : column_tiles(kind, h, TX, TY) * h.nslot;
+      case LK_TPAIR: return scalar_pairs(h) ? column_tiles(kind, h, 2 * SPX, tune_rows) * h.nslot : 0;
+      case LK_DCOL: return scalar_pairs(h) ? 0 : column_tiles(kind, h, TX, TY);
+      case LK_DCOL2: return scalar_pairs(h) ? column_tiles(kind, h, 2 * TX, TY) : 0;
       case LK_AVG: return (h.nslot - (h.buoy ? 1 : 0)) * ((h.avg_k > 0 ? h.ny : 0) + (h.avg_j > 0 ? h.nz : 0));
       case LK_COMMIT: {
         const long long nvec = h.plane * h.nz * (long long)sizeof(T) / 16;
@@ -1229,14 +1227,10 @@ struct BatchT {
       k_ghosts<T><<<gsz(9, ls[LK_SHELL].total * nf), kShellThreads, 0, stream>>>(ddom, ls[LK_SHELL].l(), packed, nf,
                                                                                  gate, prref);
   }
-  static int chunk_index(int kc) { return kc == 8 ? 0 : kc == 16 ? 1 : 2; }
   // k_sgs with the tuned z chunk; init: 0 a stage, 1 the initial viscosity
   // and diffusivity, 2 the autotuner's timing mode (k_sgs)
   void sgs_kernel(int init) {
-    const int q = chunk_index(tune_sgs_kc), g = std::max(1, std::min(ls[LK_SGST].total, cap_sgs[q]));
-    if (tune_sgs_kc == 8) k_sgs<T, 8><<<g, SgsShape<T>::threads, smem_sgs, stream>>>(ddom, ls[LK_SGST].l(), init);
-    else if (tune_sgs_kc == 16) k_sgs<T, 16><<<g, SgsShape<T>::threads, smem_sgs, stream>>>(ddom, ls[LK_SGST].l(), init);
-    else k_sgs<T, 32><<<g, SgsShape<T>::threads, smem_sgs, stream>>>(ddom, ls[LK_SGST].l(), init);
+    k_sgs<T><<<gsz(0, ls[LK_SGST].total), SgsShape<T>::threads, smem_sgs, stream>>>(ddom, ls[LK_SGST].l(), init);
   }
   // the wall model of a stage (k_wm_points) from the state at its start, on
   // stream s; stage 1 outside a step (the initial fields).  Returns 1 if it
@@ -1247,10 +1241,7 @@ struct BatchT {
     return 1;
   }
   void momentum_kernel(const StageCoef &sc) {
-    const int q = chunk_index(tune_mom_kc), g = std::max(1, std::min(ls[LK_MOMT].total, cap_mom[q]));
-    if (tune_mom_kc == 8) k_momentum<T, 8><<<g, MomShape<T>::threads, smem_mom, stream>>>(ddom, ls[LK_MOMT].l(), sc);
-    else if (tune_mom_kc == 16) k_momentum<T, 16><<<g, MomShape<T>::threads, smem_mom, stream>>>(ddom, ls[LK_MOMT].l(), sc);
-    else k_momentum<T, 32><<<g, MomShape<T>::threads, smem_mom, stream>>>(ddom, ls[LK_MOMT].l(), sc);
+    k_momentum<T><<<gsz(1, ls[LK_MOMT].total), MomShape<T>::threads, smem_mom, stream>>>(ddom, ls[LK_MOMT].l(), sc);
   }
   int launch_sgs(int stage) {
     nlaunch++;
@@ -1630,8 +1621,32 @@ struct BatchT {
     return step_finish(nsteps, st);
   }
 
+  // The planes of a tile's column: kc, halved down to 2 while the halved
+  // tiles still run as one wave of the kernel's cap resident blocks.  A tile
+  // is a serial march over its planes, so on a small grid the time of a
+  // kernel is the length of its longest column, and the idle SMs take the
+  // extra tiles at no cost but the two halo planes each of them loads
+  // (64 x 64 x 32, FP32: k_project_pair 14 -> 6 us, a step 0.267 -> 0.240 ms;
+  // 256 x 256 x 128 keeps its 16 planes).
+  int short_chunk(int kind, int kc, int cap) {
+    for (;; kc /= 2) {
+      ls[kind].kc = kc / 2;
+      long long n = 0;
+      for (int d = 0; d < nd; d++) n += tiles(kind, hdom[d]);
+      ls[kind].kc = kc;
+      if (kc <= 2 || n > cap) return kc;
+    }
+  }
+  // the chunk of the momentum and SGS kernels for a tuned length: the
+  // shortest one is shortened further on small grids
+  void set_chunk(int kind, int tuned_kc) {
+    ls[kind].kc = tuned_kc == kChunks[0] ? short_chunk(kind, tuned_kc, grid_cap[kind == LK_SGST ? 0 : 1]) : tuned_kc;
+  }
   // the launch map of one kind after a change of tile shape
   int rebuild_ls(int kind) {
+    if (kind == LK_MOMT) set_chunk(kind, tune_mom_kc);
+    if (kind == LK_SGST) set_chunk(kind, tune_sgs_kc);
+    if (kind == LK_TPAIR) ls[kind].kc = short_chunk(kind, MKC, grid_cap[tune_rows == 8 ? 12 : 14]);
     std::vector<int> st(nd + 1, 0);
     for (int d = 0; d < nd; d++) st[d + 1] = st[d] + tiles(kind, hdom[d]);
     CU(cudaMemcpy(ls[kind].starts, st.data(), sizeof(int) * (nd + 1), cudaMemcpyHostToDevice));

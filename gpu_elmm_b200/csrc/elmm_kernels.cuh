@@ -35,6 +35,7 @@ struct Launch {
   const int *starts;  // per-domain first tile, nd + 1 entries (device)
   int nd;
   int total;          // total tiles
+  int kc;             // planes of a tile's column (kernels that march up a chunk of planes)
 };
 
 template <typename T>

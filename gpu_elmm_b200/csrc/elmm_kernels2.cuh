@@ -10,7 +10,7 @@ namespace elmm {
 
 // PostPoisson (src/pressure.f90:728-870): velocity correction, Pr += Phi and
 // the partial sums of the top layer for FixPressureToReference.  A block
-// marches up an MX x MY column of MKC planes; the inputs of plane k+1 are in
+// marches up an MX x MY column of L.kc planes; the inputs of plane k+1 are in
 // flight while plane k is written, and Phi(k+1) of plane k is Phi of k+1.
 // HZ: the domains are slabs whose top face is shared (BC_HALO); a
 // compile-time choice, since a run-time test of the face here cost the
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(MX *MY) k_project(const Dom<T> *__restrict__ d
     const int bx = lt % ntx; lt /= ntx;
     const int by = lt % nty;
     const int bk = lt / nty;
-    const int k0 = bk * MKC + 1, k1 = min(k0 + MKC - 1, d.nz);
+    const int k0 = bk * L.kc + 1, k1 = min(k0 + L.kc - 1, d.nz);
     const int i = bx * MX + (threadIdx.x % MX) + 1;
     const int j = by * MY + (threadIdx.x / MX) + 1;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(MX *MY) k_project(const Dom<T> *__restrict__ d
 
 // k_project for FP32 domains with an even Prnx (x is periodic for every
 // domain): two x-adjacent cells per thread, float2 loads and stores, the
-// same tiles (MX x MY x MKC) and partial sums per tile column.  Slabs of a
+// same tiles (MX x MY x L.kc) and partial sums per tile column.  Slabs of a
 // split domain take k_project<float, true> instead.
 __global__ void __launch_bounds__(MX *MY / 2) k_project_pair(const Dom<float> *__restrict__ doms, Launch L,
                                                           double coef_alpha2, int use_dt, int in_place, int gate) {
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(MX *MY / 2) k_project_pair(const Dom<float> *_
     const int bx = lt % ntx; lt /= ntx;
     const int by = lt % nty;
     const int bk = lt / nty;
-    const int k0 = bk * MKC + 1, k1 = min(k0 + MKC - 1, d.nz);
+    const int k0 = bk * L.kc + 1, k1 = min(k0 + L.kc - 1, d.nz);
     const int i = bx * MX + 2 * (threadIdx.x % (MX / 2)) + 1;  // odd: the pair is 8-byte aligned
     const int j = by * MY + (threadIdx.x / (MX / 2)) + 1;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -388,9 +388,6 @@ __global__ void __launch_bounds__(kShellThreads) k_ghosts(const Dom<T> *__restri
   }
 }
 
-// planes per column chunk of k_divmax
-constexpr int kDivChunk = 16;
-
 // Order-preserving bits of a non-negative double; NaN maps above every
 // finite value, so an integer maximum propagates it.
 __device__ __forceinline__ unsigned long long max_bits(double v) {
@@ -419,7 +416,7 @@ __device__ __forceinline__ void block_max_flush(unsigned long long *dst, unsigne
 // max |div u| in FP64 (the check of src/pressure.f90:884-989)
 template <typename T>
 __global__ void __launch_bounds__(TX *TY) k_divmax(const Dom<T> *__restrict__ doms, Launch L) {
-  // a TX x TY column of cells marches up a chunk of kDivChunk planes; W at
+  // a TX x TY column of cells marches up a chunk of L.kc planes; W at
   // k-1 rides along in a register.  One block reduction and one atomic per
   // domain the block visits.
   __shared__ unsigned long long red[TX * TY / 32];
@@ -438,7 +435,7 @@ __global__ void __launch_bounds__(TX *TY) k_divmax(const Dom<T> *__restrict__ do
     const int ntx = (nx + TX - 1) / TX, nty = (ny + TY - 1) / TY;
     const int tx = lt % ntx; lt /= ntx;
     const int ty = lt % nty;
-    const int k0 = (lt / nty) * kDivChunk + 1, k1 = min(k0 + kDivChunk - 1, nz);
+    const int k0 = (lt / nty) * L.kc + 1, k1 = min(k0 + L.kc - 1, nz);
     const int i = tx * TX + (threadIdx.x % TX) + 1;
     const int j = ty * TY + (threadIdx.x / TX) + 1;
     if (i > nx || j > ny) continue;
@@ -489,7 +486,7 @@ __global__ void __launch_bounds__(TX *TY) k_divmax_pair(const Dom<float> *__rest
     const int ntx = (nx + 2 * TX - 1) / (2 * TX), nty = (ny + TY - 1) / TY;
     const int tx = lt % ntx; lt /= ntx;
     const int ty = lt % nty;
-    const int k0 = (lt / nty) * kDivChunk + 1, k1 = min(k0 + kDivChunk - 1, nz);
+    const int k0 = (lt / nty) * L.kc + 1, k1 = min(k0 + L.kc - 1, nz);
     const int i = tx * 2 * TX + 2 * (threadIdx.x % TX) + 1;  // odd: the pair is 8-byte aligned
     const int j = ty * TY + (threadIdx.x / TX) + 1;
     if (i > nx || j > ny) continue;

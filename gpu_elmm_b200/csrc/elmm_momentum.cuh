@@ -27,10 +27,9 @@ struct StageCoef {
   int stage;
 };
 
-#ifndef ELMM_MOM_CHUNK
-#define ELMM_MOM_CHUNK 16
-#endif
-constexpr int MX = 32, MY = 8, MKC = ELMM_MOM_CHUNK;
+// MKC: the planes of a column the marching kernels start from (the host
+// halves it on small grids, the autotuner tries up to kMaxChunk)
+constexpr int MX = 32, MY = 8, MKC = 16, kMaxChunk = 32;
 // per-tile context in shared memory: everything the stencil code reads
 // besides the fields, so that no descriptor load sits on its critical path
 template <typename T>
@@ -480,9 +479,9 @@ struct MomShape<float> {
   static constexpr int cpt = 2, slots = 4, threads = MX * MY / 2, min_blocks = 4, nnf = 4;
 };
 
-// KC: planes of a tile's column (a tuning choice: every cell's arithmetic is
-// the same for any KC)
-template <typename T, int KC = MKC>
+// L.kc: planes of a tile's column (a tuning choice: every cell's arithmetic
+// is the same for any of them)
+template <typename T>
 __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
     k_momentum(const Dom<T> *__restrict__ doms, Launch L, StageCoef sc) {
   constexpr int NNF = MomShape<T>::nnf;
@@ -492,8 +491,8 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
   T *ring = reinterpret_cast<T *>(dyn_smem);
   __shared__ __align__(8) uint64_t bars[NSL];
   __shared__ MomCtx<T> ctx;
-  // mixed path: offsets of U and V on planes k0-1 .. k0+KC of the tile (see Dom::voff)
-  __shared__ float soff[2][KC + 2];
+  // mixed path: offsets of U and V on planes k0-1 .. k0+kc of the tile (see Dom::voff)
+  __shared__ float soff[2][kMaxChunk + 2];
   __shared__ int abort_flag;
   const int tx = threadIdx.x % TXN, ty = threadIdx.x / TXN;
   // tensor copies need 128-byte aligned destinations
@@ -516,8 +515,8 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
     const int bx = lt % ntx; lt /= ntx;
     const int by = lt % nty;
     const int bk = lt / nty;
-    const int i0 = bx * MX + 1, j0 = by * MY + 1, k0 = bk * KC + 1;
-    const int k1 = min(k0 + KC - 1, d.nz);
+    const int i0 = bx * MX + 1, j0 = by * MY + 1, k0 = bk * L.kc + 1;
+    const int k1 = min(k0 + L.kc - 1, d.nz);
     const int i = i0 + CPT * tx, j = j0 + ty;  // the thread's first cell
     const int nx = d.nx, ny = d.ny;
     const long long plane = d.plane;
@@ -530,8 +529,8 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
     __syncthreads();  // every slot and the context of the previous tile are free
     if (threadIdx.x == 0) fill_ctx(ctx, d);
     if constexpr (sizeof(T) == 4) {
-      if (threadIdx.x < 2 * (KC + 2)) {
-        const int c = threadIdx.x / (KC + 2), kk = k0 - 1 + threadIdx.x % (KC + 2);
+      if (threadIdx.x < 2 * (kMaxChunk + 2)) {
+        const int c = threadIdx.x / (kMaxChunk + 2), kk = k0 - 1 + threadIdx.x % (kMaxChunk + 2);
         soff[c][kk - k0 + 1] = kk <= d.nz + 1 ? __ldg(d.voff + c * (d.nz + 2) + kk) : 0.f;
       }
     }
@@ -892,7 +891,7 @@ struct SgsShape<float> {
 // diffusivity after the projection, 2 the autotuner's timing launches (a
 // stage's arithmetic; its outputs the real stage overwrites).  The
 // wall-model points are k_wm_points'.
-template <typename T, int KC = MKC>
+template <typename T>
 __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
     k_sgs(const Dom<T> *__restrict__ doms, Launch L, int init) {
   // planes of U, V, W (tile plus one-cell halo) arrive by tensor-map TMA in
@@ -904,7 +903,7 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
   __shared__ __align__(8) uint64_t bars[kRingSlots];
   __shared__ int abort_flag;
   // mixed path: the z-difference parts du, dv of the tile's planes (SgsK)
-  __shared__ float sdz[2][KC];
+  __shared__ float sdz[2][kMaxChunk];
   const int tx = threadIdx.x % TXN, ty = threadIdx.x / TXN;
   if (smem_addr(ring) & 127u) {  // tensor copies need 128-byte aligned destinations
     if (threadIdx.x == 0) doms[0].flags[1] = 1;
@@ -925,8 +924,8 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
     const int bx = lt % ntx; lt /= ntx;
     const int by = lt % nty;
     const int bk = lt / nty;
-    const int i0 = bx * MX + 1, j0 = by * MY + 1, k0 = bk * KC + 1;
-    const int k1 = min(k0 + KC - 1, d.nz);
+    const int i0 = bx * MX + 1, j0 = by * MY + 1, k0 = bk * L.kc + 1;
+    const int k1 = min(k0 + L.kc - 1, d.nz);
     const int i = i0 + CPT * tx, j = j0 + ty;  // the thread's first cell
     const int nx = d.nx, ny = d.ny, nz = d.nz;
     const int wide[3] = {F_U, F_V, F_W};
@@ -934,8 +933,8 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
     const CUtensorMap *maps = reinterpret_cast<const CUtensorMap *>(d.tmaps);
     __syncthreads();  // every slot and the z-difference parts of the previous tile are free
     if constexpr (sizeof(T) == 4) {
-      if (threadIdx.x < 2 * KC) {
-        const int c = threadIdx.x / KC, kk = k0 + threadIdx.x % KC;
+      if (threadIdx.x < 2 * kMaxChunk) {
+        const int c = threadIdx.x / kMaxChunk, kk = k0 + threadIdx.x % kMaxChunk;
         if (kk <= k1) {
           const float *o = d.voff + c * (d.nz + 2);
           sdz[c][kk - k0] = 2.f * (__ldg(o + kk + 1) - __ldg(o + kk - 1)) * (float)d.sgs_r2zz[kk];

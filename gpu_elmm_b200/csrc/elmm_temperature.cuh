@@ -100,14 +100,9 @@ __global__ void k_scalar_zghost(const Dom<T> *__restrict__ doms, int nd, int sta
 }
 
 // A block owns a TX x TY column of cells of one scalar slot and marches up a
-// chunk of TMKC planes; the scalar (k-2..k+2), the diffusivity (k-1..k+1)
+// chunk of L.kc planes; the scalar (k-2..k+2), the diffusivity (k-1..k+1)
 // and W(k-1) ride along in registers, x and y neighbours come from offsets
 // folded once per thread.  Tiles: (slot, column, chunk) per domain.
-#ifndef ELMM_SCALAR_CHUNK
-#define ELMM_SCALAR_CHUNK 16
-#endif
-constexpr int TMKC = ELMM_SCALAR_CHUNK;
-
 // BC: some slot has a stored z ghost plane, a surface flux or a surface
 // temperature (the launch picks the plain instantiation otherwise)
 template <typename T, bool BC = false>
@@ -119,13 +114,13 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 6 : 3)
     const Dom<T> &d = doms[di];
     int lt = t - __ldg(L.starts + di);
     const int nx = d.nx, ny = d.ny, nz = d.nz;
-    const int ntx = (nx + TX - 1) / TX, nty = (ny + TY - 1) / TY, nkc = (nz + TMKC - 1) / TMKC;
+    const int ntx = (nx + TX - 1) / TX, nty = (ny + TY - 1) / TY, nkc = (nz + L.kc - 1) / L.kc;
     const int tx = lt % ntx; lt /= ntx;
     const int ty = lt % nty; lt /= nty;
     const int kc = lt % nkc;
     const int s = lt / nkc;
     const ScalSlot<T> &sl = d.slot[s];
-    const int k0 = kc * TMKC + 1, k1 = min(k0 + TMKC - 1, nz);
+    const int k0 = kc * L.kc + 1, k1 = min(k0 + L.kc - 1, nz);
     const int i = tx * TX + (threadIdx.x % TX) + 1;
     const int j = ty * TY + (threadIdx.x / TX) + 1;
     if (i > nx || j > ny) continue;
@@ -322,13 +317,13 @@ __global__ void __launch_bounds__(SPX *SPY, ELMM_SCALAR_PAIR_MIN_BLOCKS * 8 / SP
     const Dom<T> &d = doms[di];
     int lt = t - __ldg(L.starts + di);
     const int nx = d.nx, ny = d.ny, nz = d.nz;
-    const int ntx = (nx + 2 * SPX - 1) / (2 * SPX), nty = (ny + SPY - 1) / SPY, nkc = (nz + TMKC - 1) / TMKC;
+    const int ntx = (nx + 2 * SPX - 1) / (2 * SPX), nty = (ny + SPY - 1) / SPY, nkc = (nz + L.kc - 1) / L.kc;
     const int tx = lt % ntx; lt /= ntx;
     const int ty = lt % nty; lt /= nty;
     const int kc = lt % nkc;
     const int s = lt / nkc;
     const ScalSlot<T> &sl = d.slot[s];
-    const int k0 = kc * TMKC + 1, k1 = min(k0 + TMKC - 1, nz);
+    const int k0 = kc * L.kc + 1, k1 = min(k0 + L.kc - 1, nz);
     const int i = tx * 2 * SPX + 2 * (threadIdx.x % SPX) + 1;  // odd: the pair is 8-byte aligned
     const int j = ty * SPY + (threadIdx.x / SPX) + 1;
     if (i > nx || j > ny) continue;
