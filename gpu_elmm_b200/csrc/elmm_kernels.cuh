@@ -211,13 +211,18 @@ __device__ void wm_pr_dirichlet(const Dom<T> &d, int f, int i, int j, int k, con
   d.wm_pr_tf[h][q] = tfl;
 }
 
-// ComputeUVWFluxesWM / fluxes for the point of component comp on side f at
-// cell (i,j,k) (src/wallmodels.f90:2159-2338); the wall-point distance is
-// the one of GetOutsideBoundariesWM_UVW (src/wallmodels.f90:690-909).
+// ComputeUVWFluxesWM / fluxes for the point of component comp next to side f
+// (bottom or top: x and y are periodic for every domain) at column (i, j),
+// point pidx of the face (src/wallmodels.f90:2159-2338); the wall-point
+// distance is the one of GetOutsideBoundariesWM_UVW (src/wallmodels.f90:690-909).
 template <typename T>
-__device__ void wm_point(const Dom<T> &d, int comp, int f, int i, int j, int k, long long pidx, const T *Tm) {
+__device__ void wm_point(const Dom<T> &d, int comp, int f, int i, int j, int pidx, const T *Tm) {
+  const bool hi = f & 1;
+  const int k = hi ? d.ext[comp][2] : 1;
   const T *U = d.U, *V = d.V, *W = d.W;
   const long long c = bidx(d, i, j, k), sx = 1, sy = d.pitch, sz = d.plane;
+  const int face = comp * 6 + f;
+  double ustar = d.wm_ustar[face][pidx];
   // full velocities: stored values plus the per-level offsets of U and V of
   // the mixed path (the FP64 path reads the stored values alone), in FP64
   const double ou0 = (double)vel_off(d, 0, k), ov0 = (double)vel_off(d, 1, k);
@@ -244,42 +249,19 @@ __device__ void wm_point(const Dom<T> &d, int comp, int f, int i, int j, int k, 
     vel[1] = (lv(sz, ov1) + lv(0, ov0) + lv(-sy + sz, ov1) + lv(-sy, ov0)) / 4.0;
     vel[2] = (double)ld(W, c);
   }
-  // distance to the wall: xU(0) - x(1) etc. with the staggered coordinate of the component
-  double dist[3] = {0, 0, 0};
-  const int axis = f >> 1;
-  const bool hi = f & 1;
-  if (axis == 0) {
-    // xU(i) = i dxmin + xmin, xPr(i) = (xU(i-1) + xU(i)) / 2 (initial.f90:4395-4450)
-    double xc = comp == 0 ? (double)i * d.dx + d.xmin
-                          : (((double)(i - 1) * d.dx + d.xmin) + ((double)i * d.dx + d.xmin)) / 2.0;
-    double xw = hi ? (double)(d.ext[0][0] + 1) * d.dx + d.xmin : 0.0 * d.dx + d.xmin;
-    dist[0] = xw - xc;
-  } else if (axis == 1) {
-    double yc = comp == 1 ? (double)j * d.dy + d.ymin
-                          : (((double)(j - 1) * d.dy + d.ymin) + ((double)j * d.dy + d.ymin)) / 2.0;
-    double yw = hi ? (double)(d.ext[1][1] + 1) * d.dy + d.ymin : 0.0 * d.dy + d.ymin;
-    dist[1] = yw - yc;
-  } else {
-    double zc = comp == 2 ? d.zW[k + 2] : d.zPr[k + 2];
-    double zw = hi ? d.zW[d.ext[2][2] + 1 + 2] : d.zW[0 + 2];
-    dist[2] = zw - zc;
-  }
-  double dd = norm2_3(dist);
-  double t[3] = {vel[0], vel[1], vel[2]};  // wall velocity 0
-  double dot = t[0] * dist[0] + t[1] * dist[1] + t[2] * dist[2];
-#pragma unroll
-  for (int m = 0; m < 3; m++) t[m] = t[m] - dot * dist[m] / (dd * dd);
-  double tv = norm2_3(t);
-  const int face = comp * 6 + f;
-  double ustar = d.wm_ustar[face][pidx];
+  // distance to the wall with the staggered coordinate of the component; the
+  // velocity along it (wall velocity 0) taken off
+  const double distz = d.zW[hi ? d.ext[2][2] + 1 + 2 : 0 + 2] - (comp == 2 ? d.zW[k + 2] : d.zPr[k + 2]);
+  const double dd = fabs(distz);
+  const double t[3] = {vel[0], vel[1], vel[2] - vel[2] * distz * distz / (dd * dd)};
+  const double tv = sqrt((t[0] * t[0] + t[1] * t[1]) + t[2] * t[2]);
   if (d.z0[f] > 0 && d.tdir[f]) {  // WM_MO_DirichletStress (src/wallmodels.f90:1922-1938, 2228-2253)
-    const double vel2 = sqrt((t[0] * t[0] + t[1] * t[1]) + t[2] * t[2]);  // sqrt(sum(tan_vect**2))
     // local_value of theta at the point (src/wallmodels.f90:2340-2353), x and y periodic
     const int i2 = comp == 0 ? (i + 1 > d.nx ? 1 : i + 1) : i, j2 = comp == 1 ? (j + 1 > d.ny ? 1 : j + 1) : j;
     const double temp = (((double)ld(Tm, bidx(d, i2, j2, comp == 2 ? k + 1 : k)) + d.toff) +
                          ((double)ld(Tm, bidx(d, i, j, k)) + d.toff)) / 2;
     double tfl = d.wm_tfl[face][pidx];
-    wm_mo_dirichlet(d, ustar, tfl, dd, d.z0[f], vel2, temp - d.tsurf[f]);
+    wm_mo_dirichlet(d, ustar, tfl, dd, d.z0[f], tv, temp - d.tsurf[f]);
     d.wm_tfl[face][pidx] = tfl;
   } else if (d.z0[f] > 0 && d.tflux[f] > 0)  // WM_MO_FluxStress (src/wallmodels.f90:1836-1854, 2255-2259)
     ustar = tv != 0 ? wm_mo_flux_ustar(ustar, tv, dd, d.z0[f], d.tflux[f], d.tref, d.grav, d.nu_mol) : 0.0;
@@ -287,22 +269,17 @@ __device__ void wm_point(const Dom<T> &d, int comp, int f, int i, int j, int k, 
     ustar = wm_ustar(ustar, tv, dd, d.z0[f], d.nu_mol);
   if (ustar < 0) ustar = 0;
   d.wm_ustar[face][pidx] = ustar;
-  double mag = norm2_3(t);
   double fp = 0, fm = 0;
-  if (mag > 1.4901161193847656e-08) {
-    if (d.vz && f == SIDE_BO) {
-      fp = (t[comp] / mag) * (ustar * ustar);
-      fm = fp;
-      if (comp < 2) { fp = fp / d.dzPr[k + 2]; fm = fm / d.dzPr[k - 1 + 2]; }
-      else { fp = fp / d.dzW[k + 2]; fm = fm / d.dzW[k - 1 + 2]; }
-    } else if (d.vz && f == SIDE_TO) {
-      fp = (t[comp] / mag) * (ustar * ustar);
-      fm = fp;
-      if (comp < 2) { fp = fp / d.dzPr[k + 1 + 2]; fm = fm / d.dzPr[k + 2]; }
-      else { fp = fp / d.dzW[k + 1 + 2]; fm = fm / d.dzW[k + 2]; }
+  if (tv > 1.4901161193847656e-08) {
+    fp = (t[comp] / tv) * (ustar * ustar);
+    if (d.vz) {
+      // U and V: the heights of the cells either side of the face, W: of the levels
+      const double *h = comp < 2 ? d.dzPr : d.dzW;
+      const int kp = f == SIDE_BO ? k : k + 1;
+      fm = fp / h[kp - 1 + 2];
+      fp = fp / h[kp + 2];
     } else {
-      double drec = axis == 0 ? 1 / d.dx : axis == 1 ? 1 / d.dy : 1 / d.dz;
-      fp = (t[comp] / mag) * (ustar * ustar) * drec;
+      fp = fp * (1 / d.dz);
       fm = fp;
     }
     if (!hi) { fp = -fp; fm = -fm; }  // MINUSX/Y/Z directions are odd
@@ -315,74 +292,43 @@ __device__ void wm_point(const Dom<T> &d, int comp, int f, int i, int j, int k, 
 // for the Pr points with a prescribed surface temperature, and
 // ComputeUVWFluxesWM for every velocity point on a wall-model face, from the
 // state at the start of the stage (tb: its temperature buffer).  One thread
-// a point; a domain's points in the order: the Pr points of the bottom and
-// top (i + nx j), then per component and side its face plane in index
-// order (x sides: j + ny k, y sides: i + nx k, z sides: i + nx j).  The
-// parts touch disjoint state.  Launched after k_sgs (whose viscosity they do
-// not read) and, with the initial fields, at the end of the initial
-// projection.
+// a point, in faces of nx ny points (i + nx j): the Pr points of the bottom
+// and top, then per component the bottom and the top.  The parts touch
+// disjoint state.  Launched beside k_sgs (whose viscosity they do not read)
+// and, with the initial fields, at the end of the initial projection.  On a
+// small grid k_momentum waits for it: a thread's time is its chain of
+// descriptor loads, integer divisions and FP64 divisions, roots and
+// logarithms, so the face comes from one 32-bit division and the norm of the
+// tangential velocity is formed once, without scaling (128 x 128 x 64 with a
+// scalar: a step of 0.482 -> 0.469 ms).
 constexpr int kWmThreads = 128;
 template <typename T>
-__host__ __device__ inline void wm_face_plane(const Dom<T> &d, int comp, int f, int &n0, int &n1) {
-  const int *e = d.ext[comp];
-  const int axis = f >> 1;
-  n0 = axis == 0 ? e[1] : e[0];
-  n1 = axis == 2 ? e[1] : e[2];
-}
-template <typename T>
 __host__ __device__ inline long long wm_points_of(const Dom<T> &d) {
-  long long n = 0;
-  for (int f = SIDE_BO; f <= SIDE_TO; f++)
-    if (d.tdir[f]) n += (long long)d.nx * d.ny;
-  for (int comp = 0; comp < 3; comp++)
-    for (int f = 0; f < 6; f++)
-      if (d.wall[f]) {
-        int n0, n1;
-        wm_face_plane(d, comp, f, n0, n1);
-        n += (long long)n0 * n1;
-      }
-  return n;
+  const int faces = (d.tdir[SIDE_BO] != 0) + (d.tdir[SIDE_TO] != 0) + 3 * ((d.wall[SIDE_BO] != 0) + (d.wall[SIDE_TO] != 0));
+  return (long long)faces * d.nx * d.ny;
 }
 template <typename T>
 __global__ void __launch_bounds__(kWmThreads) k_wm_points(const Dom<T> *__restrict__ doms, Launch L, int tb) {
   for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
     const int di = find_dom(L.starts, L.nd, t);
     const Dom<T> &d = doms[di];
-    long long p = (long long)(t - __ldg(L.starts + di)) * kWmThreads + threadIdx.x;
+    const int nx = d.nx, np = nx * d.ny;
+    const int pr_bo = d.tdir[SIDE_BO] != 0, pr_to = d.tdir[SIDE_TO] != 0;
+    const int bo = d.wall[SIDE_BO] != 0, to = d.wall[SIDE_TO] != 0;
+    const int p = (t - __ldg(L.starts + di)) * kWmThreads + threadIdx.x;
+    int face = p / np;
+    const int q = p - face * np, j = q / nx + 1, i = q - (j - 1) * nx + 1;
     const T *Tm = d.buoy ? d.slot[0].buf[tb] : nullptr;
-    bool done = false;
-#pragma unroll 1
-    for (int f = SIDE_BO; f <= SIDE_TO && !done; f++) {
-      if (!d.tdir[f]) continue;
-      const long long np = (long long)d.nx * d.ny;
-      if (p < np) {
-        wm_pr_dirichlet(d, f, (int)(p % d.nx) + 1, (int)(p / d.nx) + 1, f == SIDE_BO ? 1 : d.nz, Tm);
-        done = true;
-      } else {
-        p -= np;
-      }
+    if (face < pr_bo + pr_to) {
+      const int f = pr_bo && face == 0 ? SIDE_BO : SIDE_TO;
+      wm_pr_dirichlet(d, f, i, j, f == SIDE_BO ? 1 : d.nz, Tm);
+      continue;
     }
-#pragma unroll 1
-    for (int comp = 0; comp < 3 && !done; comp++)
-#pragma unroll 1
-      for (int f = 0; f < 6 && !done; f++) {
-        if (!d.wall[f]) continue;
-        int n0, n1;
-        wm_face_plane(d, comp, f, n0, n1);
-        const long long np = (long long)n0 * n1;
-        if (p >= np) {
-          p -= np;
-          continue;
-        }
-        const int *e = d.ext[comp];
-        const int axis = f >> 1, hi = f & 1;
-        const int a = (int)(p % n0) + 1, b = (int)(p / n0) + 1;
-        const int i = axis == 0 ? (hi ? e[0] : 1) : a;
-        const int j = axis == 0 ? a : axis == 1 ? (hi ? e[1] : 1) : b;
-        const int k = axis == 2 ? (hi ? e[2] : 1) : b;
-        wm_point(d, comp, f, i, j, k, p, Tm);
-        done = true;
-      }
+    face -= pr_bo + pr_to;
+    const int per = bo + to;
+    if (face >= 3 * per) continue;
+    const int comp = per == 2 ? face >> 1 : face;
+    wm_point(d, comp, bo && (per == 1 || !(face & 1)) ? SIDE_BO : SIDE_TO, i, j, q, Tm);
   }
 }
 
