@@ -104,7 +104,6 @@ struct Dom {
   // once per call (advection.f90: Ax = 0.25/dxmin etc.; momentum_diffusion.f90:
   // recdxmin2 = 1/dxmin**2)
   double cA[3];          // 0.25 / dxmin, dymin, dzmin
-  double cB[3][3];       // advective-form factors of component c: 0.5 along c, 0.125 across
   double rec2[3];        // 1 / dxmin**2, ...
   // fields (box layout)
   T *U, *V, *W, *U2, *V2, *W2, *Us, *Vs, *Ws, *P, *nu, *Phi;
@@ -139,9 +138,9 @@ struct Dom {
   double *wm_tfl[kFaces];
   double *wm_pr_us[2], *wm_pr_tf[2];
   double wm_af;
-  // stretched z, packed FP32 momentum path: per-level factors kz2[q * (nz + 2) + k]
+  // stretched z: per-level factors of the tendencies, kz2[q * (nz + 2) + k]
   // (q: kZ2 entries, see elmm_packed.cuh)
-  const float *kz2;
+  const T *kz2;
   // per component: 1 marks a bottom-plane point without a wall-model point
   // (next to or under a solid body), or null for none
   const unsigned char *bskip[3];

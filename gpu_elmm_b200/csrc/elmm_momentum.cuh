@@ -34,7 +34,7 @@ constexpr int MX = 32, MY = 8, MKC = 16, kMaxChunk = 32;
 // besides the fields, so that no descriptor load sits on its critical path
 template <typename T>
 struct MomCtx {
-  T cA[3], cB[3][3], rec2[3];
+  T cA[3], rec2[3];
   int wallmask;  // bit s: wall-model fluxes on side s
   int vz;
   int ext[3][3];
@@ -43,348 +43,90 @@ struct MomCtx {
   const unsigned char *bskip[3];
 };
 
+// called by every thread of the block, a value or two each (one thread alone
+// took longer over its chain of loads than a short column of planes)
 template <typename T>
 __device__ __forceinline__ void fill_ctx(MomCtx<T> &m, const Dom<T> &d) {
-  // called by one thread
-  for (int a = 0; a < 3; a++) {
-    m.cA[a] = (T)d.cA[a];
-    m.rec2[a] = (T)d.rec2[a];
-    for (int c = 0; c < 3; c++) { m.cB[c][a] = (T)d.cB[c][a]; m.ext[c][a] = d.ext[c][a]; }
+  const int t = threadIdx.x;
+  if (t < 9) {
+    m.ext[t / 3][t % 3] = d.ext[t / 3][t % 3];
+  } else if (t < 12) {
+    m.cA[t - 9] = (T)d.cA[t - 9];
+    m.rec2[t - 9] = (T)d.rec2[t - 9];
+    m.bskip[t - 9] = d.bskip[t - 9];
+  } else if (t == 12) {
+    int wm = 0;
+#pragma unroll
+    for (int f = 0; f < 6; f++) wm |= d.wall[f] ? (1 << f) : 0;
+    m.wallmask = wm;
+    m.vz = d.vz;
+  } else if (t == 13) {
+    m.dzPr = d.dzPr; m.dzW = d.dzW; m.zPr = d.zPr; m.zW = d.zW;
+  } else if (t >= 32 && t < 32 + kFaces) {
+    m.fluxp[t - 32] = d.wm_fluxp[t - 32];
+    m.fluxm[t - 32] = d.wm_fluxm[t - 32];
   }
-  int wm = 0;
-  for (int f = 0; f < 6; f++) wm |= d.wall[f] ? (1 << f) : 0;
-  m.wallmask = wm;
-  m.vz = d.vz;
-  m.dzPr = d.dzPr; m.dzW = d.dzW; m.zPr = d.zPr; m.zW = d.zW;
-  for (int f = 0; f < kFaces; f++) { m.fluxp[f] = d.wm_fluxp[f]; m.fluxm[f] = d.wm_fluxm[f]; }
-  for (int c = 0; c < 3; c++) m.bskip[c] = d.bskip[c];
 }
 
-// one velocity component's tendency at (i,j,k): advection + diffusion +
-// wall corrections, in the reference's order of operations
-// bt, bsub: the buoyancy of W, (a + bt) - bsub after the advection
-// (BuoyancyForce, src/dynamics.f90:679-688; zero without a temperature field)
-template <typename T, int C, typename RT>
-__device__ __forceinline__ T tendency(const MomCtx<T> &m, const RT &R, int i, int j, int k, int wallhere,
-                                      T bt = (T)0, T bsub = (T)0) {
-  // X(dx,dy,dz) with the component's own axis first: along = C, a1, a2 the others
-#define FU(dx, dy, dz) R.g(0, dx, dy, dz)
-#define FV(dx, dy, dz) R.g(1, dx, dy, dz)
-#define FW(dx, dy, dz) R.g(2, dx, dy, dz)
-#define FN(dx, dy, dz) R.g(3, dx, dy, dz)
-  T a;
-  const T rx = m.rec2[0], ry = m.rec2[1], rz = m.rec2[2];
-  if (C == 0) {
-    const T u = FU(0, 0, 0), ue = FU(1, 0, 0), uw = FU(-1, 0, 0), un = FU(0, 1, 0), us = FU(0, -1, 0);
-    const T ut = FU(0, 0, 1), ub = FU(0, 0, -1);
-    const T v = FV(0, 0, 0), ve = FV(1, 0, 0), vs = FV(0, -1, 0), vse = FV(1, -1, 0);
-    const T w = FW(0, 0, 0), we = FW(1, 0, 0), wb = FW(0, 0, -1), wbe = FW(1, 0, -1);
-    const T Ax = m.cA[0], Ay = m.cA[1];
-    const T Bx = m.cB[0][0], By = m.cB[0][1];
-    if (!m.vz) {
-      const T Az = m.cA[2], Bz = m.cB[0][2];
-      a = -((Ax * (ue + u) * (ue + u) - Ax * (u + uw) * (u + uw)) + (Ay * (un + u) * (ve + v) - Ay * (u + us) * (vse + vs)) +
-            (Az * (ut + u) * (we + w) - Az * (u + ub) * (wbe + wb)));
-      T Vadv = (v + ve + vs + vse);
-      T Wadv = (w + we + wb + wbe);
-      a = a - (Bx * (ue - uw) * u + By * (un - us) * Vadv + Bz * (ut - ub) * Wadv);
-    } else {
-      const T dzp = (T)m.dzPr[k + 2];
-      a = -((Ax * (ue + u) * (ue + u) - Ax * (u + uw) * (u + uw)) + (Ay * (un + u) * (ve + v) - Ay * (u + us) * (vse + vs)) +
-            ((ut + u) * (we + w) - (u + ub) * (wbe + wb)) / dzp / 4);
-      T Vadv = (v + ve + vs + vse);
-      T Wadv = (w + we + wb + wbe) / 4;
-      a = a - (Bx * (ue - uw) * u + By * (un - us) * Vadv + (ut - ub) / (T)(m.zPr[k + 1 + 2] - m.zPr[k - 1 + 2]) * Wadv);
-    }
-    a = a * (T)0.5;
-    const T n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nn = FN(0, 1, 0), nne = FN(1, 1, 0), ns = FN(0, -1, 0), nse = FN(1, -1, 0);
-    const T nt = FN(0, 0, 1), nte = FN(1, 0, 1), nb = FN(0, 0, -1), nbe = FN(1, 0, -1);
-    a = a + ne * (ue - u) * rx;
-    a = a - n0 * (u - uw) * rx;
-    a = a + (T)0.25 * (nne + ne + nn + n0) * (un - u) * ry;
-    a = a - (T)0.25 * (ne + nse + n0 + ns) * (u - us) * ry;
-    if (!m.vz) {
-      a = a + (T)0.25 * (nte + ne + nt + n0) * (ut - u) * rz;
-      a = a - (T)0.25 * (ne + nbe + n0 + nb) * (u - ub) * rz;
-    } else {
-      T tz = (T)0.25 * (nte + ne + nt + n0) * (ut - u) / (T)m.dzW[k + 2];
-      tz = tz - (T)0.25 * (ne + nbe + n0 + nb) * (u - ub) / (T)m.dzW[k - 1 + 2];
-      tz = tz / (T)m.dzPr[k + 2];
-      a = a + tz;
-    }
-    if (wallhere) {
-      const int *e = m.ext[0];
-      if ((m.wallmask & (1 << SIDE_WE)) && i == 1) {
-        long long p = (long long)(j - 1) + (long long)e[1] * (k - 1);
-        a = a + n0 * (u - uw) * rx;
-        a = a + m.fluxp[0 * 6 + SIDE_WE][p];
-      }
-      if ((m.wallmask & (1 << SIDE_EA)) && i == e[0]) {
-        long long p = (long long)(j - 1) + (long long)e[1] * (k - 1);
-        a = a - ne * (ue - u) * rx;
-        a = a - m.fluxm[0 * 6 + SIDE_EA][p];
-      }
-      if ((m.wallmask & (1 << SIDE_SO)) && j == 1) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (k - 1);
-        a = a + (ne + nse + n0 + ns) * (u - us) * ry / 4;
-        a = a + m.fluxp[0 * 6 + SIDE_SO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_NO)) && j == e[1]) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (k - 1);
-        a = a - (nne + ne + nn + n0) * (un - u) * ry / 4;
-        a = a - m.fluxm[0 * 6 + SIDE_NO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_BO)) && k == 1 &&
-          !(m.bskip[0] && m.bskip[0][(long long)(i - 1) + (long long)e[0] * (j - 1)])) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (j - 1);
-        T s = ne + nbe + n0 + nb;
-        if (m.vz) a = a + s * (u - ub) / (T)m.dzW[k - 1 + 2] / 4 / (T)m.dzPr[k + 2];
-        else a = a + s * (u - ub) * rz / 4;
-        a = a + m.fluxp[0 * 6 + SIDE_BO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_TO)) && k == e[2]) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (j - 1);
-        T s = nte + ne + nt + n0;
-        if (m.vz) a = a - s * (ut - u) / (T)m.dzW[k + 2] / 4 / (T)m.dzPr[k + 2];
-        else a = a - s * (ut - u) * rz / 4;
-        a = a - m.fluxm[0 * 6 + SIDE_TO][p];
-      }
-    }
-  } else if (C == 1) {
-    const T v = FV(0, 0, 0), ve = FV(1, 0, 0), vw = FV(-1, 0, 0), vn = FV(0, 1, 0), vs = FV(0, -1, 0);
-    const T vt = FV(0, 0, 1), vb = FV(0, 0, -1);
-    const T u = FU(0, 0, 0), un = FU(0, 1, 0), uw = FU(-1, 0, 0), unw = FU(-1, 1, 0);
-    const T w = FW(0, 0, 0), wn = FW(0, 1, 0), wb = FW(0, 0, -1), wbn = FW(0, 1, -1);
-    const T Ax = m.cA[0], Ay = m.cA[1];
-    const T Bx = m.cB[1][0], By = m.cB[1][1];
-    if (!m.vz) {
-      const T Az = m.cA[2], Bz = m.cB[1][2];
-      a = -((Ay * (vn + v) * (vn + v) - Ay * (v + vs) * (v + vs)) + (Ax * (ve + v) * (un + u) - Ax * (v + vw) * (unw + uw)) +
-            (Az * (vt + v) * (wn + w) - Az * (v + vb) * (wbn + wb)));
-      T Uadv = (u + un + uw + unw);
-      T Wadv = (w + wn + wb + wbn);
-      a = a - (Bx * (ve - vw) * Uadv + By * (vn - vs) * v + Bz * (vt - vb) * Wadv);
-    } else {
-      const T dzp = (T)m.dzPr[k + 2];
-      a = -((Ay * (vn + v) * (vn + v) - Ay * (v + vs) * (v + vs)) + (Ax * (ve + v) * (un + u) - Ax * (v + vw) * (unw + uw)) +
-            ((vt + v) * (wn + w) - (v + vb) * (wbn + wb)) / dzp / 4);
-      T Uadv = (u + un + uw + unw);
-      T Wadv = (w + wn + wb + wbn) / 4;
-      a = a - (Bx * (ve - vw) * Uadv + By * (vn - vs) * v + (vt - vb) / (T)(m.zPr[k + 1 + 2] - m.zPr[k - 1 + 2]) * Wadv);
-    }
-    a = a * (T)0.5;
-    const T n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nn = FN(0, 1, 0), nne = FN(1, 1, 0), nw = FN(-1, 0, 0), nnw = FN(-1, 1, 0);
-    const T nt = FN(0, 0, 1), nnt = FN(0, 1, 1), nb = FN(0, 0, -1), nnb = FN(0, 1, -1);
-    a = a + (T)0.25 * (nne + ne + nn + n0) * (ve - v) * rx;
-    a = a - (T)0.25 * (nn + n0 + nnw + nw) * (v - vw) * rx;
-    a = a + nn * (vn - v) * ry;
-    a = a - n0 * (v - vs) * ry;
-    if (!m.vz) {
-      a = a + (T)0.25 * (nnt + nn + nt + n0) * (vt - v) * rz;
-      a = a - (T)0.25 * (nn + nnb + n0 + nb) * (v - vb) * rz;
-    } else {
-      T tz = (T)0.25 * (nnt + nn + nt + n0) * (vt - v) / (T)m.dzW[k + 2];
-      tz = tz - (T)0.25 * (nn + nnb + n0 + nb) * (v - vb) / (T)m.dzW[k - 1 + 2];
-      tz = tz / (T)m.dzPr[k + 2];
-      a = a + tz;
-    }
-    if (wallhere) {
-      const int *e = m.ext[1];
-      if ((m.wallmask & (1 << SIDE_WE)) && i == 1) {
-        long long p = (long long)(j - 1) + (long long)e[1] * (k - 1);
-        a = a + (nn + n0 + nnw + nw) * (v - vw) * rx / 4;
-        a = a + m.fluxp[1 * 6 + SIDE_WE][p];
-      }
-      if ((m.wallmask & (1 << SIDE_EA)) && i == e[0]) {
-        long long p = (long long)(j - 1) + (long long)e[1] * (k - 1);
-        a = a - (nne + ne + nn + n0) * (ve - v) * rx / 4;
-        a = a - m.fluxm[1 * 6 + SIDE_EA][p];
-      }
-      if ((m.wallmask & (1 << SIDE_SO)) && j == 1) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (k - 1);
-        a = a + n0 * (v - vs) * ry;
-        a = a + m.fluxp[1 * 6 + SIDE_SO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_NO)) && j == e[1]) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (k - 1);
-        a = a - nn * (vn - v) * ry;
-        a = a - m.fluxm[1 * 6 + SIDE_NO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_BO)) && k == 1 &&
-          !(m.bskip[1] && m.bskip[1][(long long)(i - 1) + (long long)e[0] * (j - 1)])) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (j - 1);
-        T s = nn + nnb + n0 + nb;
-        if (m.vz) a = a + s * (v - vb) / (T)m.dzW[k - 1 + 2] / 4 / (T)m.dzPr[k + 2];
-        else a = a + s * (v - vb) * rz / 4;
-        a = a + m.fluxp[1 * 6 + SIDE_BO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_TO)) && k == e[2]) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (j - 1);
-        T s = nnt + nn + nt + n0;
-        if (m.vz) a = a - s * (vt - v) / (T)m.dzW[k + 2] / 4 / (T)m.dzPr[k + 2];
-        else a = a - s * (vt - v) * rz / 4;
-        a = a - m.fluxm[1 * 6 + SIDE_TO][p];
-      }
-    }
-  } else {
-    const T w = FW(0, 0, 0), we = FW(1, 0, 0), ww = FW(-1, 0, 0), wn = FW(0, 1, 0), ws = FW(0, -1, 0);
-    const T wt = FW(0, 0, 1), wb = FW(0, 0, -1);
-    const T u = FU(0, 0, 0), ut = FU(0, 0, 1), uw = FU(-1, 0, 0), utw = FU(-1, 0, 1);
-    const T v = FV(0, 0, 0), vt = FV(0, 0, 1), vs = FV(0, -1, 0), vts = FV(0, -1, 1);
-    const T Ax = m.cA[0], Ay = m.cA[1];
-    const T Bx = m.cB[2][0], By = m.cB[2][1];
-    if (!m.vz) {
-      const T Az = m.cA[2], Bz = m.cB[2][2];
-      a = -((Az * (wt + w) * (wt + w) - Az * (w + wb) * (w + wb)) + (Ay * (wn + w) * (vt + v) - Ay * (w + ws) * (vs + vts)) +
-            (Ax * (we + w) * (ut + u) - Ax * (w + ww) * (utw + uw)));
-      T Uadv = (u + ut + uw + utw);
-      T Vadv = (v + vt + vs + vts);
-      a = a - (Bx * (we - ww) * Uadv + By * (wn - ws) * Vadv + Bz * (wt - wb) * w);
-    } else {
-      const T dzw = (T)m.dzW[k + 2];
-      a = -(((wt + w) * (wt + w) - (w + wb) * (w + wb)) / dzw / 4 + (Ay * (wn + w) * (vt + v) - Ay * (w + ws) * (vts + vs)) +
-            (Ax * (we + w) * (ut + u) - Ax * (w + ww) * (utw + uw)));
-      T Uadv = (u + ut + uw + utw);
-      T Vadv = (v + vt + vs + vts);
-      a = a - (Bx * (we - ww) * Uadv + By * (wn - ws) * Vadv + (wt - wb) / (T)(m.zW[k + 1 + 2] - m.zW[k - 1 + 2]) * w);
-    }
-    a = a * (T)0.5;
-    a = (a + bt) - bsub;
-    const T n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nt = FN(0, 0, 1), nte = FN(1, 0, 1), nw = FN(-1, 0, 0), ntw = FN(-1, 0, 1);
-    const T nn = FN(0, 1, 0), ntn = FN(0, 1, 1), ns = FN(0, -1, 0), nts = FN(0, -1, 1);
-    a = a + (T)0.25 * (nte + ne + nt + n0) * (we - w) * rx;
-    a = a - (T)0.25 * (nt + n0 + ntw + nw) * (w - ww) * rx;
-    a = a + (T)0.25 * (ntn + nt + nn + n0) * (wn - w) * ry;
-    a = a - (T)0.25 * (nt + nts + n0 + ns) * (w - ws) * ry;
-    if (!m.vz) {
-      a = a + nt * (wt - w) * rz;
-      a = a - n0 * (w - wb) * rz;
-    } else {
-      T tz = nt * (wt - w) / (T)m.dzPr[k + 1 + 2];
-      tz = tz - n0 * (w - wb) / (T)m.dzPr[k + 2];
-      tz = tz / (T)m.dzW[k + 2];
-      a = a + tz;
-    }
-    if (wallhere) {
-      const int *e = m.ext[2];
-      if ((m.wallmask & (1 << SIDE_WE)) && i == 1) {
-        long long p = (long long)(j - 1) + (long long)e[1] * (k - 1);
-        a = a + (nt + n0 + ntw + nw) * (w - ww) * rx / 4;
-        a = a + m.fluxp[2 * 6 + SIDE_WE][p];
-      }
-      if ((m.wallmask & (1 << SIDE_EA)) && i == e[0]) {
-        long long p = (long long)(j - 1) + (long long)e[1] * (k - 1);
-        a = a - (nte + ne + nt + n0) * (we - w) * rx / 4;
-        a = a - m.fluxm[2 * 6 + SIDE_EA][p];
-      }
-      if ((m.wallmask & (1 << SIDE_SO)) && j == 1) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (k - 1);
-        a = a + (nt + nts + n0 + ns) * (w - ws) * ry / 4;
-        a = a + m.fluxp[2 * 6 + SIDE_SO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_NO)) && j == e[1]) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (k - 1);
-        a = a - (ntn + nt + nn + n0) * (wn - w) * ry / 4;
-        a = a - m.fluxm[2 * 6 + SIDE_NO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_BO)) && k == 1 &&
-          !(m.bskip[2] && m.bskip[2][(long long)(i - 1) + (long long)e[0] * (j - 1)])) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (j - 1);
-        if (m.vz) a = a + n0 * (w - wb) / (T)m.dzPr[k + 2] / (T)m.dzW[k + 2];
-        else a = a + n0 * (w - wb) * rz;
-        a = a + m.fluxp[2 * 6 + SIDE_BO][p];
-      }
-      if ((m.wallmask & (1 << SIDE_TO)) && k == e[2]) {
-        long long p = (long long)(i - 1) + (long long)e[0] * (j - 1);
-        if (m.vz) a = a - nt * (wt - w) / (T)m.dzPr[k + 1 + 2] / (T)m.dzW[k + 2];
-        else a = a - nt * (wt - w) * rz;
-        a = a - m.fluxm[2 * 6 + SIDE_TO][p];
-      }
-    }
-  }
-#undef FU
-#undef FV
-#undef FW
-#undef FN
-  return a;
+// one value, or the two of a pair, from a plane of values; 0 where the byte
+// mask (or null) is set
+__device__ __forceinline__ float wall_ld(const float *p, float) { return p[0]; }
+__device__ __forceinline__ double wall_ld(const double *p, double) { return p[0]; }
+__device__ __forceinline__ F2 wall_ld(const float *p, F2) { return F2{make_float2(p[0], p[1])}; }
+__device__ __forceinline__ float wall_keep(float a, const unsigned char *m) { return m && m[0] ? 0.f : a; }
+__device__ __forceinline__ double wall_keep(double a, const unsigned char *m) { return m && m[0] ? 0.0 : a; }
+__device__ __forceinline__ F2 wall_keep(F2 a, const unsigned char *m) {
+  return m ? F2{make_float2(m[0] ? 0.f : a.v.x, m[1] ? 0.f : a.v.y)} : a;
 }
+__device__ __forceinline__ float wall_scale(float v, float) { return v; }
+__device__ __forceinline__ double wall_scale(double v, double) { return v; }
+__device__ __forceinline__ F2 wall_scale(float v, F2) { return bc2(v); }
 
-// The wall-model corrections of one cell on the mixed path (the wall blocks
-// of tendency<T, C>: the diffusive flux through the face towards a wall-model
-// side taken back, the wall-model flux added; the wmfluxes-*-inc.f90
-// includes), on stored deviations: a difference across levels is the stored
-// difference plus the difference of the offsets (O, see tendency_dev).
-template <int C, typename RT>
-__device__ __forceinline__ float wall_dev(const MomCtx<float> &m, const RT &R, const VelOffN<float> &O, int i, int j,
-                                          int k) {
+// The wall-model corrections at the bottom and top: the diffusive flux
+// through the face towards the wall taken back, the wall-model flux added
+// (the wmfluxes-*-inc.f90 includes); with OFF on stored deviations, where a
+// difference across levels is the stored difference plus the difference of
+// the offsets (O, see tendency_dev).  For one cell or a pair (F2) whose first
+// cell is (i, j); x and y are periodic for every domain, so no other side has
+// a wall.  In the packed form: with one cell at a time the wall planes took a
+// tile two to four planes' time, which on a small grid was the kernel's.
+template <int C, bool OFF, typename T, typename N, typename RT>
+__device__ __forceinline__ N wall_dev(const MomCtx<T> &m, const RT &R, const VelOffN<N> &O, int i, int j, int k) {
 #define FN(dx, dy, dz) R.g(3, dx, dy, dz)
-  const float rx = m.rec2[0], ry = m.rec2[1], rz = m.rec2[2];
   const int *e = m.ext[C];
-  float a = 0.f;
-  const long long pyz = (long long)(j - 1) + (long long)e[1] * (k - 1), pxz = (long long)(i - 1) + (long long)e[0] * (k - 1);
   const long long pxy = (long long)(i - 1) + (long long)e[0] * (j - 1);
-  const bool bo = (m.wallmask & (1 << SIDE_BO)) && k == 1 && !(m.bskip[C] && m.bskip[C][pxy]);
-  const bool to = (m.wallmask & (1 << SIDE_TO)) && k == e[2];
-  if (C < 2) {
-    // U (C = 0) or V (C = 1): the component F and its offsets
-    const float f = R.g(C, 0, 0, 0), fe = R.g(C, 1, 0, 0), fw = R.g(C, -1, 0, 0), fn = R.g(C, 0, 1, 0);
-    const float fs = R.g(C, 0, -1, 0), ft = R.g(C, 0, 0, 1), fb = R.g(C, 0, 0, -1);
-    const float *o = C == 0 ? O.o : O.p;
-    const float n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nn = FN(0, 1, 0), nne = FN(1, 1, 0);
-    // the viscosities of the x- and y-faces of the point
-    const float nW = C == 0 ? n0 : 0.25f * (((nn + n0) + FN(-1, 1, 0)) + FN(-1, 0, 0));
-    const float nE = C == 0 ? ne : 0.25f * (((nne + ne) + nn) + n0);
-    const float nS = C == 0 ? 0.25f * (((ne + FN(1, -1, 0)) + n0) + FN(0, -1, 0)) : n0;
-    const float nN = C == 0 ? 0.25f * (((nne + ne) + nn) + n0) : nn;
-    if ((m.wallmask & (1 << SIDE_WE)) && i == 1) { a = a + nW * (f - fw) * rx; a = a + m.fluxp[C * 6 + SIDE_WE][pyz]; }
-    if ((m.wallmask & (1 << SIDE_EA)) && i == e[0]) { a = a - nE * (fe - f) * rx; a = a - m.fluxm[C * 6 + SIDE_EA][pyz]; }
-    if ((m.wallmask & (1 << SIDE_SO)) && j == 1) { a = a + nS * (f - fs) * ry; a = a + m.fluxp[C * 6 + SIDE_SO][pxz]; }
-    if ((m.wallmask & (1 << SIDE_NO)) && j == e[1]) { a = a - nN * (fn - f) * ry; a = a - m.fluxm[C * 6 + SIDE_NO][pxz]; }
-    if (bo) {
-      const float s = C == 0 ? ((ne + FN(1, 0, -1)) + n0) + FN(0, 0, -1) : ((nn + FN(0, 1, -1)) + n0) + FN(0, 0, -1);
-      const float db = (f - fb) + (o[1] - o[0]);
-      if (m.vz) a = a + s * db / (float)m.dzW[k - 1 + 2] / 4 / (float)m.dzPr[k + 2];
-      else a = a + s * db * rz / 4;
-      a = a + m.fluxp[C * 6 + SIDE_BO][pxy];
+  const N one = N{}, n0 = FN(0, 0, 0);
+  const T rz = m.rec2[2];
+  N a = cst(0.f, one);
+  const N f = R.g(C, 0, 0, 0);
+  // the viscosity sum of U's or V's face dz away (four times its mean)
+  auto sum = [&](int dz) {
+    return C == 0 ? ((FN(1, 0, 0) + FN(1, 0, dz)) + n0) + FN(0, 0, dz) : ((FN(0, 1, 0) + FN(0, 1, dz)) + n0) + FN(0, 0, dz);
+  };
+  const N *o = C == 0 ? O.o : O.p;
+  if ((m.wallmask & (1 << SIDE_BO)) && k == 1) {
+    N df = f - R.g(C, 0, 0, -1), c;
+    if (C < 2) {
+      if (OFF) df = df + (o[1] - o[0]);
+      const T r = m.vz ? (T)(1.0 / m.dzW[k - 1 + 2] / m.dzPr[k + 2]) : rz;
+      c = sum(-1) * df * wall_scale(r * (T)0.25, one);
+    } else {
+      const T r = m.vz ? (T)(1.0 / m.dzPr[k + 2] / m.dzW[k + 2]) : rz;
+      c = n0 * df * wall_scale(r, one);
     }
-    if (to) {
-      const float s = C == 0 ? ((FN(1, 0, 1) + ne) + FN(0, 0, 1)) + n0 : ((FN(0, 1, 1) + nn) + FN(0, 0, 1)) + n0;
-      const float dt = (ft - f) + (o[2] - o[1]);
-      if (m.vz) a = a - s * dt / (float)m.dzW[k + 2] / 4 / (float)m.dzPr[k + 2];
-      else a = a - s * dt * rz / 4;
-      a = a - m.fluxm[C * 6 + SIDE_TO][pxy];
+    a = a + wall_keep(c + wall_ld(m.fluxp[C * 6 + SIDE_BO] + pxy, one), m.bskip[C] ? m.bskip[C] + pxy : nullptr);
+  }
+  if ((m.wallmask & (1 << SIDE_TO)) && k == e[2]) {
+    N df = R.g(C, 0, 0, 1) - f, c;
+    if (C < 2) {
+      if (OFF) df = df + (o[2] - o[1]);
+      const T r = m.vz ? (T)(1.0 / m.dzW[k + 2] / m.dzPr[k + 2]) : rz;
+      c = sum(1) * df * wall_scale(r * (T)0.25, one);
+    } else {
+      const T r = m.vz ? (T)(1.0 / m.dzPr[k + 1 + 2] / m.dzW[k + 2]) : rz;
+      c = FN(0, 0, 1) * df * wall_scale(r, one);
     }
-  } else {
-    const float w = R.g(2, 0, 0, 0), we = R.g(2, 1, 0, 0), ww = R.g(2, -1, 0, 0), wn = R.g(2, 0, 1, 0);
-    const float ws = R.g(2, 0, -1, 0), wt = R.g(2, 0, 0, 1), wb = R.g(2, 0, 0, -1);
-    const float n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nt = FN(0, 0, 1), nte = FN(1, 0, 1), nw = FN(-1, 0, 0);
-    const float ntw = FN(-1, 0, 1), nn = FN(0, 1, 0), ntn = FN(0, 1, 1), ns = FN(0, -1, 0), nts = FN(0, -1, 1);
-    if ((m.wallmask & (1 << SIDE_WE)) && i == 1) {
-      a = a + (((nt + n0) + ntw) + nw) * (w - ww) * rx / 4;
-      a = a + m.fluxp[2 * 6 + SIDE_WE][pyz];
-    }
-    if ((m.wallmask & (1 << SIDE_EA)) && i == e[0]) {
-      a = a - (((nte + ne) + nt) + n0) * (we - w) * rx / 4;
-      a = a - m.fluxm[2 * 6 + SIDE_EA][pyz];
-    }
-    if ((m.wallmask & (1 << SIDE_SO)) && j == 1) {
-      a = a + (((nt + nts) + n0) + ns) * (w - ws) * ry / 4;
-      a = a + m.fluxp[2 * 6 + SIDE_SO][pxz];
-    }
-    if ((m.wallmask & (1 << SIDE_NO)) && j == e[1]) {
-      a = a - (((ntn + nt) + nn) + n0) * (wn - w) * ry / 4;
-      a = a - m.fluxm[2 * 6 + SIDE_NO][pxz];
-    }
-    if (bo) {
-      if (m.vz) a = a + n0 * (w - wb) / (float)m.dzPr[k + 2] / (float)m.dzW[k + 2];
-      else a = a + n0 * (w - wb) * rz;
-      a = a + m.fluxp[2 * 6 + SIDE_BO][pxy];
-    }
-    if (to) {
-      if (m.vz) a = a - nt * (wt - w) / (float)m.dzPr[k + 1 + 2] / (float)m.dzW[k + 2];
-      else a = a - nt * (wt - w) * rz;
-      a = a - m.fluxm[2 * 6 + SIDE_TO][pxy];
-    }
+    a = a - (c + wall_ld(m.fluxm[C * 6 + SIDE_TO] + pxy, one));
   }
 #undef FN
   return a;
@@ -526,32 +268,33 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
     const CUtensorMap *tmapT = (NNF == 4 && d.buoy && d.tmapT)
                                    ? reinterpret_cast<const CUtensorMap *>(d.tmapT) + (sc.stage - 1) % 3
                                    : nullptr;
+    // (asm memory clobbers in the loop below reload what is not in a register)
+    const int skip = d.skip_plane, wait_limit = d.wait_limit, aln = d.aln;
     __syncthreads();  // every slot and the context of the previous tile are free
-    if (threadIdx.x == 0) fill_ctx(ctx, d);
+    if (threadIdx.x == 0) {
+      fence_async_shared();
+      for (int kk = k0 - 1; kk <= min(k0 - 1 + NSL - 1, k1 + 1); kk++)
+        if (kk != skip)
+          issue_mom_plane<T, NNF>(ring + (kk % NSL) * Lay::SIZE, &bars[kk % NSL], maps, tmapT, !stage1, aln, i0, j0,
+                                  kk);
+    }
+    fill_ctx(ctx, d);
     if constexpr (sizeof(T) == 4) {
       if (threadIdx.x < 2 * (kMaxChunk + 2)) {
         const int c = threadIdx.x / (kMaxChunk + 2), kk = k0 - 1 + threadIdx.x % (kMaxChunk + 2);
         soff[c][kk - k0 + 1] = kk <= d.nz + 1 ? __ldg(d.voff + c * (d.nz + 2) + kk) : 0.f;
       }
     }
-    if (threadIdx.x == 0) {
-      fence_async_shared();
-      for (int kk = k0 - 1; kk <= min(k0 - 1 + NSL - 1, k1 + 1); kk++)
-        if (kk != d.skip_plane)
-          issue_mom_plane<T, NNF>(ring + (kk % NSL) * Lay::SIZE, &bars[kk % NSL], maps, tmapT, !stage1, d.aln, i0, j0,
-                                  kk);
-    }
     __syncthreads();  // the context is written
-    const T dt = (T)d.dt, rdt = (T)sc.rho, bdt = (T)sc.beta;
+    const T dt = (T)d.dt;
     const double coefd = sc.alpha2 * d.dt;
     const T coef = (T)coefd;
     const T gx = (T)(-coefd / d.dx), gy = (T)(-coefd / d.dy), gz = (T)(-coefd / d.dz);
-    const T m = (T)(*d.prm);
+    const T rdt = stage1 ? (T)0 : (T)sc.rho * dt, bdt = (T)sc.beta * dt;  // of the old and the new tendency
     const int kU = d.ext[0][2], kV = d.ext[1][2], kW = d.ext[2][2];
     const bool vz = d.vz != 0;
-    const bool prgx_on = d.prgx_on != 0, prgy_on = d.prgy_on != 0;
-    const T fx = prgx_on ? (-coef) * (T)d.prgx : (T)0, fy = prgy_on ? (-coef) * (T)d.prgy : (T)0;
-    const double *dzW = d.dzW;
+    // the mean pressure gradient's increments
+    const T fx = d.prgx_on ? (-coef) * (T)d.prgx : (T)0, fy = d.prgy_on ? (-coef) * (T)d.prgy : (T)0;
     T *__restrict__ U2o = d.U2;
     T *__restrict__ V2o = d.V2;
     T *__restrict__ W2o = d.W2;
@@ -561,14 +304,9 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
     const int o = (ty + 1) * Lay::SPW + (CPT * tx + Lay::XO);
     const bool inside0 = i <= nx && j <= ny;
     long long c = bidx(d, inside0 ? i : 1, inside0 ? j : 1, k0);
-    const int nz = d.nz;
-    // block-uniform: only tiles on a side of the box and the planes next to
-    // the bottom and top have wall-model corrections; a component's last
-    // index is n or n-1 (src/initial.f90:871-896)
-    const bool xlo = i0 == 1, xhi = i0 + MX - 1 >= nx - 1, ylo = j0 == 1, yhi = j0 + MY - 1 >= ny - 1;
-    int wmask = 0;
-    for (int f = 0; f < 6; f++) wmask |= d.wall[f] ? (1 << f) : 0;
-    const int wtile = wmask & ((xlo ? 1 : 0) | (xhi ? 2 : 0) | (ylo ? 4 : 0) | (yhi ? 8 : 0));
+    const int nz = d.nz, nzp = nz + 2;
+    // the walls (x and y are periodic): bottom and top
+    const int wmask = (d.wall[SIDE_BO] ? 1 << SIDE_BO : 0) | (d.wall[SIDE_TO] ? 1 << SIDE_TO : 0);
     // both cells of the thread's pair have all three components (the pairs of
     // a partial tile past the last cell take the per-cell path)
     const bool pair_full = i + CPT - 1 <= min(d.ext[0][0], min(d.ext[1][0], d.ext[2][0])) &&
@@ -579,35 +317,45 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
     const T bA2 = (T)(d.grav / d.tref / 2.0);
     const T bsub = buoy && d.toff == 0 ? (T)(d.grav / d.tref * d.tref) : (T)0;
     const T *__restrict__ Tm = buoy ? d.slot[0].buf[(sc.stage - 1) % 3] : nullptr;  // theta at the stage start
-    MomK2 K2;
+    MomKN<F2> K2;
     if constexpr (CPT == 2) {
-      K2.Ax = bc2((float)ctx.cA[0]); K2.Ay = bc2((float)ctx.cA[1]); K2.Az = bc2((float)ctx.cA[2]);
-      K2.rx = bc2((float)ctx.rec2[0]); K2.ry = bc2((float)ctx.rec2[1]); K2.rz = bc2((float)ctx.rec2[2]);
-      K2.q = bc2(0.25f);
-      for (int cc = 0; cc < 3; cc++)
-        for (int a2 = 0; a2 < 3; a2++) K2.B[cc][a2] = bc2((float)ctx.cB[cc][a2]);
-    }
-    for (int k = k0; k <= k1; k++) {
-      // planes k-1, k, k+1 must have landed
-      bool ok = true;
-      for (int kk = (k == k0 ? k0 - 1 : k + 1); kk <= k + 1; kk++) {
-        const int s2 = kk % NSL;
-        bool w = mbar_wait(&bars[s2], (phase >> s2) & 1u, d.wait_limit);
-        // a plane whose copies were issued always lands before the block
-        // moves on or gives up (so no copy into this block's shared memory
-        // outlives it): a lowered limit only cuts the wait on a skipped one
-        if (!w && kk != d.skip_plane) w = mbar_wait(&bars[s2], (phase >> s2) & 1u);
-        ok &= w;
-        phase ^= 1u << s2;
+      for (int a = 0; a < 3; a++) {
+        K2.A[a] = bc2((float)ctx.cA[a]);
+        K2.r[a] = bc2((float)ctx.rec2[a]);
+        K2.q[a] = bc2(0.25f * (float)ctx.rec2[a]);
       }
+    }
+    const T *__restrict__ kz2 = d.kz2;
+    // FP64: the temperature of levels k and k + 1 rides along, that of k + 2
+    // is on its way while level k is computed (its slots would not leave room
+    // for two blocks per SM; loaded at their use, the two values were the
+    // kernel's largest stall: 0.41 -> 0.385 ms at 256 x 256 x 128)
+    T th0 = (T)0, th1 = (T)0;
+    if (NNF == 3 && buoy && inside0) {
+      th0 = ld(Tm, c);
+      th1 = ld(Tm, c + plane);
+    }
+    // the wait for a plane's copies; a plane whose copies were issued always
+    // lands before the block moves on or gives up (so no copy into this
+    // block's shared memory outlives it): a lowered limit only cuts the wait
+    // on a skipped one
+    auto landed = [&](int kk, int s2) {
+      bool w = mbar_wait(&bars[s2], (phase >> s2) & 1u, wait_limit);
+      if (!w && kk != skip) w = mbar_wait(&bars[s2], (phase >> s2) & 1u);
+      phase ^= 1u << s2;
+      return w;
+    };
+    int sm = (k0 - 1) % NSL, s0 = k0 % NSL, sp = (k0 + 1) % NSL;  // slots of planes k-1, k, k+1
+    bool ok = landed(k0 - 1, sm);
+    ok &= landed(k0, s0);
+    for (int k = k0; k <= k1; k++) {
+      T th2 = (T)0;
+      if (NNF == 3 && buoy && inside0 && k < k1) th2 = ld(Tm, c + 2 * plane);
+      ok &= landed(k + 1, sp);
       if (!ok) { abort_flag = 1; d.flags[1] = 1; }
-      const int wallhere = wtile | (wmask & ((k == 1 ? 16 : 0) | (k >= nz - 1 ? 32 : 0)));
-      const T *p0s = ring + ((k - 1) % NSL) * Lay::SIZE, *p1s = ring + (k % NSL) * Lay::SIZE,
-              *p2s = ring + ((k + 1) % NSL) * Lay::SIZE;
-      bool packed = false;
-      if constexpr (CPT == 2)
-        packed = (!vz || d.kz2) && !wallhere && pair_full && k <= min(kU, min(kV, kW));
-      if (packed && ok) {
+      const bool wallhere = ((wmask >> SIDE_BO) & (k == 1)) | ((wmask >> SIDE_TO) & (k >= nz - 1));
+      const T *p0s = ring + sm * Lay::SIZE, *p1s = ring + s0 * Lay::SIZE, *p2s = ring + sp * Lay::SIZE;
+      if (CPT == 2 && ok && pair_full && k <= min(kU, kV)) {
         if constexpr (CPT == 2) {
           // two cells per thread, every operation on a pair
           Ring2<Lay::WB, Lay::SPW> R2;
@@ -620,8 +368,6 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
 #pragma unroll
           for (int q = 0; q < 3; q++) { O.o[q] = bc2(soff[0][k - k0 + q]); O.p[q] = bc2(soff[1][k - k0 + q]); }
           const float *nar = p1s + Lay::WIDE + ty * MX + CPT * tx;
-          const F2 mm = bc2(m);
-          const F2 p0 = R2.g(4, 0, 0, 0) - mm;
           F2 btp = bc2(0.f);
           if (buoy) {
             const int ot = Lay::WIDE + 3 * Lay::NB + ty * MX + CPT * tx;  // the temperature, narrow field 3
@@ -630,48 +376,54 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
           }
           F2 tu, tv, tw;
           F2 gz2 = bc2(gz);
+          const F2 zero = bc2(0.f);
           if (!vz) {
-            tu = tendency_dev<0, false>(K2, R2, O, bc2(0.f), (const KZ2 *)nullptr);
-            tv = tendency_dev<1, false>(K2, R2, O, bc2(0.f), (const KZ2 *)nullptr);
-            tw = tendency_dev<2, false>(K2, R2, O, btp, (const KZ2 *)nullptr);
+            tu = tendency_dev<0, false, true>(K2, R2, O, zero, (const KZN<F2> *)nullptr);
+            tv = tendency_dev<1, false, true>(K2, R2, O, zero, (const KZN<F2> *)nullptr);
+            tw = tendency_dev<2, false, true>(K2, R2, O, btp, (const KZN<F2> *)nullptr);
           } else {
-            const int nzp = nz + 2;
-            const float *kz = d.kz2 + k;
-            KZ2 Z;
+            const float *kz = kz2 + k;
+            KZN<F2> Z;
             Z.auv = bc2(__ldg(kz + KZ_AUV * nzp)); Z.buv = bc2(__ldg(kz + KZ_BUV * nzp));
             Z.d1uv = bc2(__ldg(kz + KZ_D1UV * nzp)); Z.d2uv = bc2(__ldg(kz + KZ_D2UV * nzp));
             Z.aw = bc2(__ldg(kz + KZ_AW * nzp)); Z.bw = bc2(__ldg(kz + KZ_BW * nzp));
             Z.d1w = bc2(__ldg(kz + KZ_D1W * nzp)); Z.d2w = bc2(__ldg(kz + KZ_D2W * nzp));
             gz2 = bc2((-coef) * __ldg(kz + KZ_RDZW * nzp));
-            tu = tendency_dev<0, true>(K2, R2, O, bc2(0.f), &Z);
-            tv = tendency_dev<1, true>(K2, R2, O, bc2(0.f), &Z);
-            tw = tendency_dev<2, true>(K2, R2, O, btp, &Z);
+            tu = tendency_dev<0, true, true>(K2, R2, O, zero, &Z);
+            tv = tendency_dev<1, true, true>(K2, R2, O, zero, &Z);
+            tw = tendency_dev<2, true, true>(K2, R2, O, btp, &Z);
           }
-          const F2 rd = bc2(rdt), dd = bc2(dt), bd = bc2(bdt);
-          const F2 zero = bc2(0.f);
-          F2 u2 = stage1 ? zero : F2{*reinterpret_cast<const float2 *>(nar)} * rd * dd;
-          F2 v2 = stage1 ? zero : F2{*reinterpret_cast<const float2 *>(nar + Lay::NB)} * rd * dd;
-          F2 w2 = stage1 ? zero : F2{*reinterpret_cast<const float2 *>(nar + 2 * Lay::NB)} * rd * dd;
-          u2 = u2 + tu * bd * dd;
-          if (prgx_on) u2 = u2 + bc2(fx);
-          u2 = u2 + bc2(gx) * ((R2.g(4, 1, 0, 0) - mm) - p0);
+          if (wallhere) {
+            tu = tu + wall_dev<0, true>(ctx, R2, O, i, j, k);
+            tv = tv + wall_dev<1, true>(ctx, R2, O, i, j, k);
+            tw = tw + wall_dev<2, true>(ctx, R2, O, i, j, k);
+          }
+          // the increments of the stage summed, then added; the pressure's
+          // reference offset cancels in its differences
+          const F2 p0 = R2.g(4, 0, 0, 0), rd = bc2(rdt), bd = bc2(bdt);
+          F2 u2 = fm(bd, tu, fm(bc2(gx), R2.g(4, 1, 0, 0) - p0, bc2(fx)));
+          F2 v2 = fm(bd, tv, fm(bc2(gy), R2.g(4, 0, 1, 0) - p0, bc2(fy)));
+          F2 w2 = fm(bd, tw, gz2 * (R2.g(4, 0, 0, 1) - p0));
+          if (!stage1) {
+            u2 = fm(rd, F2{*reinterpret_cast<const float2 *>(nar)}, u2);
+            v2 = fm(rd, F2{*reinterpret_cast<const float2 *>(nar + Lay::NB)}, v2);
+            w2 = fm(rd, F2{*reinterpret_cast<const float2 *>(nar + 2 * Lay::NB)}, w2);
+          }
           u2 = u2 + R2.g(0, 0, 0, 0);
-          v2 = v2 + tv * bd * dd;
-          if (prgy_on) v2 = v2 + bc2(fy);
-          v2 = v2 + bc2(gy) * ((R2.g(4, 0, 1, 0) - mm) - p0);
           v2 = v2 + R2.g(1, 0, 0, 0);
-          w2 = w2 + tw * bd * dd;
-          w2 = w2 + gz2 * ((R2.g(4, 0, 0, 1) - mm) - p0);
           w2 = w2 + R2.g(2, 0, 0, 0);
           *reinterpret_cast<float2 *>(Us + c) = tu.v;
           *reinterpret_cast<float2 *>(U2o + c) = u2.v;
           *reinterpret_cast<float2 *>(Vs + c) = tv.v;
           *reinterpret_cast<float2 *>(V2o + c) = v2.v;
-          *reinterpret_cast<float2 *>(Ws + c) = tw.v;
-          *reinterpret_cast<float2 *>(W2o + c) = w2.v;
+          if (k <= kW) {
+            *reinterpret_cast<float2 *>(Ws + c) = tw.v;
+            *reinterpret_cast<float2 *>(W2o + c) = w2.v;
+          }
         }
       } else if (ok) {
-#pragma unroll
+        constexpr bool OFF = sizeof(T) == 4;
+#pragma unroll 1
         for (int q = 0; q < CPT; q++) {
           const int iq = i + q;
           if (!(iq <= nx && j <= ny)) continue;
@@ -680,7 +432,6 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
           R.o = o + q;
           const T *nar = p1s + Lay::WIDE + ty * MX + CPT * tx + q;  // narrow blocks are NB apart
           const long long cq = c + q;
-          const T p0 = R.g(4, 0, 0, 0) - m;
           // all shared-memory reads first, then the stores: a global store in
           // between would make the compiler reload every shared value it may
           // alias
@@ -688,72 +439,68 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
           const bool doV = iq <= d.ext[1][0] && j <= d.ext[1][1] && k <= kV;
           const bool doW = iq <= d.ext[2][0] && j <= d.ext[2][1] && k <= kW;
           T bt = (T)0;
-          if (buoy && doW) {
+          if (buoy) {
             if constexpr (NNF == 4) {  // the temperature of planes k+1 and k from the ring
               const int ot = Lay::WIDE + 3 * Lay::NB + ty * MX + CPT * tx + q;
               bt = bA2 * (p2s[ot] + p1s[ot]);
             } else {
-              bt = bA2 * (ld(Tm, cq + plane) + ld(Tm, cq));
+              bt = bA2 * (th1 + th0) - bsub;
             }
           }
-          T tu, tv, tw;
-          if constexpr (sizeof(T) == 4) {
-            // mixed path: the deviation forms of tendency_dev plus the wall
-            // corrections of wall_dev (U and V are stored as deviations)
-            VelOffN<float> O;
+          VelOffN<T> O;
 #pragma unroll
-            for (int q3 = 0; q3 < 3; q3++) { O.o[q3] = soff[0][k - k0 + q3]; O.p[q3] = soff[1][k - k0 + q3]; }
-            MomKN<float> K1;
-            K1.Ax = ctx.cA[0]; K1.Ay = ctx.cA[1]; K1.Az = ctx.cA[2];
-            K1.rx = ctx.rec2[0]; K1.ry = ctx.rec2[1]; K1.rz = ctx.rec2[2];
-            K1.q = 0.25f;
-            for (int c3 = 0; c3 < 3; c3++)
-              for (int a3 = 0; a3 < 3; a3++) K1.B[c3][a3] = ctx.cB[c3][a3];
-            KZN<float> Z1;
-            if (vz) {
-              const int nzp = nz + 2;
-              const float *kz = d.kz2 + k;
-              Z1.auv = __ldg(kz + KZ_AUV * nzp); Z1.buv = __ldg(kz + KZ_BUV * nzp);
-              Z1.d1uv = __ldg(kz + KZ_D1UV * nzp); Z1.d2uv = __ldg(kz + KZ_D2UV * nzp);
-              Z1.aw = __ldg(kz + KZ_AW * nzp); Z1.bw = __ldg(kz + KZ_BW * nzp);
-              Z1.d1w = __ldg(kz + KZ_D1W * nzp); Z1.d2w = __ldg(kz + KZ_D2W * nzp);
-            }
-            auto td = [&](auto cc) -> float {
-              constexpr int CC = decltype(cc)::value;
-              const float b3 = CC == 2 ? bt : 0.f;
-              float a3 = vz ? tendency_dev<CC, true>(K1, R, O, b3, &Z1) : tendency_dev<CC, false>(K1, R, O, b3, &Z1);
-              if (wallhere) a3 = a3 + wall_dev<CC>(ctx, R, O, iq, j, k);
-              return a3;
-            };
-            tu = doU ? td(std::integral_constant<int, 0>{}) : 0.f;
-            tv = doV ? td(std::integral_constant<int, 1>{}) : 0.f;
-            tw = doW ? td(std::integral_constant<int, 2>{}) : 0.f;
-          } else {
-            tu = doU ? tendency<T, 0>(ctx, R, iq, j, k, wallhere) : (T)0;
-            tv = doV ? tendency<T, 1>(ctx, R, iq, j, k, wallhere) : (T)0;
-            tw = doW ? tendency<T, 2>(ctx, R, iq, j, k, wallhere, bt, bsub) : (T)0;
+          for (int q3 = 0; q3 < 3; q3++) {
+            O.o[q3] = OFF ? (T)soff[0][k - k0 + q3] : (T)0;
+            O.p[q3] = OFF ? (T)soff[1][k - k0 + q3] : (T)0;
           }
-          T u2 = stage1 ? (T)0 : nar[0] * rdt * dt;
-          T v2 = stage1 ? (T)0 : nar[Lay::NB] * rdt * dt;
-          T w2 = stage1 ? (T)0 : nar[2 * Lay::NB] * rdt * dt;
-          u2 = u2 + tu * bdt * dt;
-          if (prgx_on) u2 = u2 + fx;
-          u2 = u2 + gx * ((R.g(4, 1, 0, 0) - m) - p0);
+          MomKN<T> K1;
+#pragma unroll
+          for (int a3 = 0; a3 < 3; a3++) {
+            K1.A[a3] = ctx.cA[a3];
+            K1.r[a3] = ctx.rec2[a3];
+            K1.q[a3] = (T)0.25 * ctx.rec2[a3];
+          }
+          T tu, tv, tw, gzk = gz;
+          if (!vz) {
+            tu = tendency_dev<0, false, OFF>(K1, R, O, (T)0, (const KZN<T> *)nullptr);
+            tv = tendency_dev<1, false, OFF>(K1, R, O, (T)0, (const KZN<T> *)nullptr);
+            tw = tendency_dev<2, false, OFF>(K1, R, O, bt, (const KZN<T> *)nullptr);
+          } else {
+            const T *kz = kz2 + k;
+            KZN<T> Z1;
+            Z1.auv = __ldg(kz + KZ_AUV * nzp); Z1.buv = __ldg(kz + KZ_BUV * nzp);
+            Z1.d1uv = __ldg(kz + KZ_D1UV * nzp); Z1.d2uv = __ldg(kz + KZ_D2UV * nzp);
+            Z1.aw = __ldg(kz + KZ_AW * nzp); Z1.bw = __ldg(kz + KZ_BW * nzp);
+            Z1.d1w = __ldg(kz + KZ_D1W * nzp); Z1.d2w = __ldg(kz + KZ_D2W * nzp);
+            gzk = (-coef) * __ldg(kz + KZ_RDZW * nzp);
+            tu = tendency_dev<0, true, OFF>(K1, R, O, (T)0, &Z1);
+            tv = tendency_dev<1, true, OFF>(K1, R, O, (T)0, &Z1);
+            tw = tendency_dev<2, true, OFF>(K1, R, O, bt, &Z1);
+          }
+          if (wallhere) {
+            tu = tu + wall_dev<0, OFF>(ctx, R, O, iq, j, k);
+            tv = tv + wall_dev<1, OFF>(ctx, R, O, iq, j, k);
+            tw = tw + wall_dev<2, OFF>(ctx, R, O, iq, j, k);
+          }
+          const T p0 = R.g(4, 0, 0, 0);
+          T u2 = fm(bdt, tu, fm(gx, R.g(4, 1, 0, 0) - p0, fx));
+          T v2 = fm(bdt, tv, fm(gy, R.g(4, 0, 1, 0) - p0, fy));
+          T w2 = fm(bdt, tw, gzk * (R.g(4, 0, 0, 1) - p0));
+          if (!stage1) {
+            u2 = fm(rdt, nar[0], u2);
+            v2 = fm(rdt, nar[Lay::NB], v2);
+            w2 = fm(rdt, nar[2 * Lay::NB], w2);
+          }
           u2 = u2 + R.g(0, 0, 0, 0);
-          v2 = v2 + tv * bdt * dt;
-          if (prgy_on) v2 = v2 + fy;
-          v2 = v2 + gy * ((R.g(4, 0, 1, 0) - m) - p0);
           v2 = v2 + R.g(1, 0, 0, 0);
-          w2 = w2 + tw * bdt * dt;
-          const T dpz = (R.g(4, 0, 0, 1) - m) - p0;
-          if (vz) w2 = w2 - coef * dpz / (T)dzW[k + 2];
-          else w2 = w2 + gz * dpz;
           w2 = w2 + R.g(2, 0, 0, 0);
           if (doU) { Us[cq] = tu; U2o[cq] = u2; }
           if (doV) { Vs[cq] = tv; V2o[cq] = v2; }
           if (doW) { Ws[cq] = tw; W2o[cq] = w2; }
         }
       }
+      th0 = th1;
+      th1 = th2;
       __syncthreads();  // plane k-1 is no longer read
       if (abort_flag) {
         // a plane did not arrive: wait (bounded) for the copies still in
@@ -761,18 +508,20 @@ __global__ void __launch_bounds__(MomShape<T>::threads, MomShape<T>::min_blocks)
         if (threadIdx.x == 0)
           for (int kk = k + 2; kk <= min(k - 1 + NSL - 1, k1 + 1); kk++) {
             const int s2 = kk % NSL;
-            if (kk != d.skip_plane) mbar_wait(&bars[s2], (phase >> s2) & 1u);  // issued copies land: the full limit
+            if (kk != skip) mbar_wait(&bars[s2], (phase >> s2) & 1u);  // issued copies land: the full limit
             phase ^= 1u << s2;
           }
         return;
       }
       const int kn = k - 1 + NSL;
-      if (threadIdx.x == 0 && kn <= k1 + 1 && kn != d.skip_plane) {
+      if (threadIdx.x == 0 && kn <= k1 + 1 && kn != skip) {
         fence_async_shared();
-        issue_mom_plane<T, NNF>(ring + (kn % NSL) * Lay::SIZE, &bars[kn % NSL], maps, tmapT, !stage1, d.aln, i0, j0,
-                                kn);
+        issue_mom_plane<T, NNF>(ring + sm * Lay::SIZE, &bars[sm], maps, tmapT, !stage1, aln, i0, j0, kn);
       }
       c += plane;
+      sm = s0;
+      s0 = sp;
+      sp = sp + 1 == NSL ? 0 : sp + 1;
     }
   }
 }
@@ -795,79 +544,39 @@ struct SgsK {  // factors of NuSmag at one level k
   const float *du, *dv;
 };
 
-// The divisions by the (uniform) spacings of StrainIJ are multiplications by
-// reciprocals computed once, which changes the result by at most one
-// rounding; the sum of squares keeps the order of Strainu.
-template <typename T, typename RT>
-__device__ __forceinline__ T nusmag_ring(const SgsK<T> &q, const RT &R) {
+// One cell (float, double) or a pair (F2).  The divisions by the (uniform)
+// spacings of StrainIJ are multiplications by reciprocals computed once; the
+// symmetric pairs of the strain tensor are formed once, 2 S = 2 sum D_aa^2 +
+// sum (D_ab + D_ba)^2, with fused multiply-adds: 36 operations where the
+// nine terms of Strainu took 68 (256 x 256 x 128, k_sgs and k_wm_points one
+// after the other: FP32 93 -> 78 us, FP64 154 -> 132).  The square root is taken per cell.
+__device__ __forceinline__ float root(float a) { return sqrtf(a); }
+__device__ __forceinline__ double root(double a) { return sqrt(a); }
+__device__ __forceinline__ F2 root(F2 a) { return F2{make_float2(sqrtf(a.v.x), sqrtf(a.v.y))}; }
+template <bool OFF, typename T, typename N, typename RT>
+__device__ __forceinline__ N nusmag(const SgsK<T> &q, const RT &R, N) {
 #define GU(dx, dy, dz) R.g(0, dx, dy, dz)
 #define GV(dx, dy, dz) R.g(1, dx, dy, dz)
 #define GW(dx, dy, dz) R.g(2, dx, dy, dz)
-  T D00 = (GU(0, 0, 0) - GU(-1, 0, 0)) * q.rdx;
-  T D11 = (GV(0, 0, 0) - GV(0, -1, 0)) * q.rdy;
-  T D22 = (GW(0, 0, 0) - GW(0, 0, -1)) * q.rdz;
-  T D01 = (GU(0, 1, 0) + GU(-1, 1, 0) - GU(0, -1, 0) - GU(-1, -1, 0)) * q.r4dy;
-  T D02 = (GU(0, 0, 1) + GU(-1, 0, 1) - GU(0, 0, -1) - GU(-1, 0, -1)) * q.r2zz;
-  T D10 = (GV(1, 0, 0) + GV(1, -1, 0) - GV(-1, 0, 0) - GV(-1, -1, 0)) * q.r4dx;
-  T D12 = (GV(0, 0, 1) + GV(0, -1, 1) - GV(0, 0, -1) - GV(0, -1, -1)) * q.r2zz;
-  if constexpr (sizeof(T) == 4) {
-    D02 = D02 + *q.du;
-    D12 = D12 + *q.dv;
-  }
-  T D20 = (GW(1, 0, 0) + GW(1, 0, -1) - GW(-1, 0, 0) - GW(-1, 0, -1)) * q.r4dx;
-  T D21 = (GW(0, 1, 0) + GW(0, 1, -1) - GW(0, -1, 0) - GW(0, -1, -1)) * q.r4dy;
+  auto k = [](T v) { return wall_scale(v, N{}); };  // a factor, broadcast to a pair
+  const N r4dx = k(q.r4dx), r4dy = k(q.r4dy), r2zz = k(q.r2zz);
+  const N d0 = (GU(0, 0, 0) - GU(-1, 0, 0)) * k(q.rdx), d1 = (GV(0, 0, 0) - GV(0, -1, 0)) * k(q.rdy),
+          d2 = (GW(0, 0, 0) - GW(0, 0, -1)) * k(q.rdz);
+  const N S = fm(d2, d2, fm(d1, d1, d0 * d0));
+  const N uy = (GU(0, 1, 0) + GU(-1, 1, 0)) - (GU(0, -1, 0) + GU(-1, -1, 0));
+  const N vx = (GV(1, 0, 0) + GV(1, -1, 0)) - (GV(-1, 0, 0) + GV(-1, -1, 0));
+  const N t01 = fm(uy, r4dy, vx * r4dx);
+  const N uz = (GU(0, 0, 1) + GU(-1, 0, 1)) - (GU(0, 0, -1) + GU(-1, 0, -1));
+  const N wx = (GW(1, 0, 0) + GW(1, 0, -1)) - (GW(-1, 0, 0) + GW(-1, 0, -1));
+  const N t02 = fm(wx, r4dx, OFF ? fm(uz, r2zz, k((T)*q.du)) : uz * r2zz);
+  const N vz = (GV(0, 0, 1) + GV(0, -1, 1)) - (GV(0, 0, -1) + GV(0, -1, -1));
+  const N wy = (GW(0, 1, 0) + GW(0, 1, -1)) - (GW(0, -1, 0) + GW(0, -1, -1));
+  const N t12 = fm(wy, r4dy, OFF ? fm(vz, r2zz, k((T)*q.dv)) : vz * r2zz);
 #undef GU
 #undef GV
 #undef GW
-  T s, S = 0;
-  s = (D00 + D00) / 2; S = S + s * s;
-  s = (D10 + D01) / 2; S = S + s * s;
-  s = (D20 + D02) / 2; S = S + s * s;
-  s = (D01 + D10) / 2; S = S + s * s;
-  s = (D11 + D11) / 2; S = S + s * s;
-  s = (D21 + D12) / 2; S = S + s * s;
-  s = (D02 + D20) / 2; S = S + s * s;
-  s = (D12 + D21) / 2; S = S + s * s;
-  s = (D22 + D22) / 2; S = S + s * s;
-  T Sbar = sqrt((T)2 * S);
-  return Sbar * q.wc2;
+  return root(fm(t12, t12, fm(t02, t02, fm(t01, t01, S + S)))) * k(q.wc2);
 }
-
-// nusmag_ring for a pair of x-adjacent cells with packed FP32x2 arithmetic;
-// the square root is taken per cell
-template <typename RT>
-__device__ __forceinline__ F2 nusmag2(const SgsK<float> &q, const RT &R) {
-#define GU(dx, dy, dz) R.g(0, dx, dy, dz)
-#define GV(dx, dy, dz) R.g(1, dx, dy, dz)
-#define GW(dx, dy, dz) R.g(2, dx, dy, dz)
-  const F2 rdx = bc2(q.rdx), rdy = bc2(q.rdy), rdz = bc2(q.rdz), r4dx = bc2(q.r4dx), r4dy = bc2(q.r4dy),
-           r2zz = bc2(q.r2zz), half = bc2(0.5f);
-  const F2 D00 = (GU(0, 0, 0) - GU(-1, 0, 0)) * rdx;
-  const F2 D11 = (GV(0, 0, 0) - GV(0, -1, 0)) * rdy;
-  const F2 D22 = (GW(0, 0, 0) - GW(0, 0, -1)) * rdz;
-  const F2 D01 = (((GU(0, 1, 0) + GU(-1, 1, 0)) - GU(0, -1, 0)) - GU(-1, -1, 0)) * r4dy;
-  const F2 D02 = (((GU(0, 0, 1) + GU(-1, 0, 1)) - GU(0, 0, -1)) - GU(-1, 0, -1)) * r2zz + bc2(*q.du);
-  const F2 D10 = (((GV(1, 0, 0) + GV(1, -1, 0)) - GV(-1, 0, 0)) - GV(-1, -1, 0)) * r4dx;
-  const F2 D12 = (((GV(0, 0, 1) + GV(0, -1, 1)) - GV(0, 0, -1)) - GV(0, -1, -1)) * r2zz + bc2(*q.dv);
-  const F2 D20 = (((GW(1, 0, 0) + GW(1, 0, -1)) - GW(-1, 0, 0)) - GW(-1, 0, -1)) * r4dx;
-  const F2 D21 = (((GW(0, 1, 0) + GW(0, 1, -1)) - GW(0, -1, 0)) - GW(0, -1, -1)) * r4dy;
-#undef GU
-#undef GV
-#undef GW
-  F2 s, S = bc2(0.f);
-  s = (D00 + D00) * half; S = S + s * s;
-  s = (D10 + D01) * half; S = S + s * s;
-  s = (D20 + D02) * half; S = S + s * s;
-  s = (D01 + D10) * half; S = S + s * s;
-  s = (D11 + D11) * half; S = S + s * s;
-  s = (D21 + D12) * half; S = S + s * s;
-  s = (D02 + D20) * half; S = S + s * s;
-  s = (D12 + D21) * half; S = S + s * s;
-  s = (D22 + D22) * half; S = S + s * s;
-  const F2 Sbar{make_float2(sqrtf(2.f * S.v.x), sqrtf(2.f * S.v.y))};
-  return Sbar * bc2(q.wc2);
-}
-
 
 // ComputeTDiff (src/scalar_diffusion.f90:983-1009): the temperature
 // diffusivity from the viscosity, constant Pr_sgs = 0.6
@@ -902,6 +611,8 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
   T *ring = reinterpret_cast<T *>(dyn_smem);
   __shared__ __align__(8) uint64_t bars[kRingSlots];
   __shared__ int abort_flag;
+  // the factors 1/dzPr, 1/(2 (zPr(k+1) - zPr(k-1))), (width Cs)^2 of the tile's planes
+  __shared__ T sfac[3][kMaxChunk];
   // mixed path: the z-difference parts du, dv of the tile's planes (SgsK)
   __shared__ float sdz[2][kMaxChunk];
   const int tx = threadIdx.x % TXN, ty = threadIdx.x / TXN;
@@ -931,7 +642,15 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
     const int wide[3] = {F_U, F_V, F_W};
     const int none[1] = {0};
     const CUtensorMap *maps = reinterpret_cast<const CUtensorMap *>(d.tmaps);
-    __syncthreads();  // every slot and the z-difference parts of the previous tile are free
+    const int skip = d.skip_plane, wait_limit = d.wait_limit, aln = d.aln;
+    __syncthreads();  // every slot and the level factors of the previous tile are free
+    if (threadIdx.x == 0) {
+      fence_async_shared();
+      for (int kk = k0 - 1; kk <= min(k0 - 1 + kRingSlots - 1, k1 + 1); kk++)
+        if (kk != skip)
+          issue_plane<T, 3, 0>(ring + (kk % kRingSlots) * Lay::SIZE, &bars[kk % kRingSlots], maps, wide, none, false,
+                               aln, i0, j0, kk);
+    }
     if constexpr (sizeof(T) == 4) {
       if (threadIdx.x < 2 * kMaxChunk) {
         const int c = threadIdx.x / kMaxChunk, kk = k0 + threadIdx.x % kMaxChunk;
@@ -940,15 +659,13 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
           sdz[c][kk - k0] = 2.f * (__ldg(o + kk + 1) - __ldg(o + kk - 1)) * (float)d.sgs_r2zz[kk];
         }
       }
-      __syncthreads();
     }
-    if (threadIdx.x == 0) {
-      fence_async_shared();
-      for (int kk = k0 - 1; kk <= min(k0 - 1 + kRingSlots - 1, k1 + 1); kk++)
-        if (kk != d.skip_plane)
-          issue_plane<T, 3, 0>(ring + (kk % kRingSlots) * Lay::SIZE, &bars[kk % kRingSlots], maps, wide, none, false,
-                               d.aln, i0, j0, kk);
+    if (threadIdx.x < 3 * kMaxChunk) {
+      const int c = threadIdx.x / kMaxChunk, kk = k0 + threadIdx.x % kMaxChunk;
+      const double *tab = c == 0 ? d.sgs_rdz : c == 1 ? d.sgs_r2zz : d.sgs_wc2;
+      if (kk <= k1) sfac[c][kk - k0] = (T)tab[kk];
     }
+    __syncthreads();  // the factors are written
     const T num = (T)d.nu_mol;
     const bool sgs = d.sgs != 0, addmol = d.nu_mol > 0;
     // the scalar diffusivity too: every stage with buoyancy (ComputeTDiff,
@@ -960,38 +677,35 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
     SgsK<T> q;
     q.rdx = (T)(1.0 / d.dx); q.rdy = (T)(1.0 / d.dy);
     q.r4dx = (T)(1.0 / (4 * d.dx)); q.r4dy = (T)(1.0 / (4 * d.dy));
-    const double *tr = d.sgs_rdz, *t2 = d.sgs_r2zz, *tw = d.sgs_wc2;
     T *__restrict__ nu = d.nu;
+    T *__restrict__ td_out = d.TDiff;
     const int o = (ty + 1) * Lay::SPW + (CPT * tx + Lay::XO);
     const bool inside0 = i <= nx && j <= ny;
     const bool pair_inside = i + CPT - 1 <= nx && j <= ny;
     long long c = bidx(d, inside0 ? i : 1, inside0 ? j : 1, k0);
     const long long plane = d.plane;
+    auto landed = [&](int kk, int s2) {  // as in k_momentum
+      bool w = mbar_wait(&bars[s2], (phase >> s2) & 1u, wait_limit);
+      if (!w && kk != skip) w = mbar_wait(&bars[s2], (phase >> s2) & 1u);
+      phase ^= 1u << s2;
+      return w;
+    };
+    int sm = (k0 - 1) % kRingSlots, s0 = k0 % kRingSlots, sp = (k0 + 1) % kRingSlots;  // slots of planes k-1, k, k+1
+    bool ok = landed(k0 - 1, sm);
+    ok &= landed(k0, s0);
     for (int k = k0; k <= k1; k++) {
-      q.rdz = (T)tr[k]; q.r2zz = (T)t2[k]; q.wc2 = (T)tw[k];
+      q.rdz = sfac[0][k - k0]; q.r2zz = sfac[1][k - k0]; q.wc2 = sfac[2][k - k0];
       q.du = &sdz[0][k - k0];
       q.dv = &sdz[1][k - k0];
-      // planes k-1, k, k+1 must have landed
-      bool ok = true;
-      for (int kk = (k == k0 ? k0 - 1 : k + 1); kk <= k + 1; kk++) {
-        const int s2 = kk % kRingSlots;
-        bool w = mbar_wait(&bars[s2], (phase >> s2) & 1u, d.wait_limit);
-        // a plane whose copies were issued always lands before the block
-        // moves on or gives up (so no copy into this block's shared memory
-        // outlives it): a lowered limit only cuts the wait on a skipped one
-        if (!w && kk != d.skip_plane) w = mbar_wait(&bars[s2], (phase >> s2) & 1u);
-        ok &= w;
-        phase ^= 1u << s2;
-      }
+      ok &= landed(k + 1, sp);
       if (!ok) { abort_flag = 1; d.flags[1] = 1; }
-      const T *p0s = ring + ((k - 1) % kRingSlots) * Lay::SIZE, *p1s = ring + (k % kRingSlots) * Lay::SIZE,
-              *p2s = ring + ((k + 1) % kRingSlots) * Lay::SIZE;
+      const T *p0s = ring + sm * Lay::SIZE, *p1s = ring + s0 * Lay::SIZE, *p2s = ring + sp * Lay::SIZE;
       if (ok && CPT == 2 && sgs && pair_inside) {
         if constexpr (CPT == 2) {
           Ring2<Lay::WB, Lay::SPW> R2;
           R2.p[0] = p0s; R2.p[1] = p1s; R2.p[2] = p2s;
           R2.o = o;
-          F2 v = nusmag2(q, R2);
+          F2 v = nusmag<true>(q, R2, F2{});
           if (addmol) v = v + bc2(num);
           *reinterpret_cast<float2 *>(nu + c) = v.v;
           // the periodic x ghosts of the row's end cells (the ghost pass covers y and z)
@@ -1000,7 +714,7 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
           if (buoy) {
             const float2 td = init == 1 ? make_float2((v.v.x - num) / 0.6f + kap, (v.v.y - num) / 0.6f + kap)
                                    : make_float2(tdiff_of(v.v.x, num, kap), tdiff_of(v.v.y, num, kap));
-            *reinterpret_cast<float2 *>(d.TDiff + c) = td;
+            *reinterpret_cast<float2 *>(td_out + c) = td;
           }
         }
       } else if (ok) {
@@ -1012,13 +726,13 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
           R.o = o + qc;
           T v = num;
           if (sgs) {
-            v = nusmag_ring(q, R);
+            v = nusmag<sizeof(T) == 4>(q, R, T{});
             if (addmol) v = v + num;
           }
           nu[c + qc] = v;
           if (i + qc == 1) nu[c + qc + nx] = v;  // periodic x ghosts (the ghost pass covers y and z)
           if (i + qc == nx) nu[c + qc - nx] = v;
-          if (buoy) d.TDiff[c + qc] = init == 1 ? (v - num) / (T)0.6 + kap : tdiff_of(v, num, kap);
+          if (buoy) td_out[c + qc] = init == 1 ? (v - num) / (T)0.6 + kap : tdiff_of(v, num, kap);
         }
       }
       __syncthreads();  // plane k-1 is no longer read
@@ -1028,18 +742,21 @@ __global__ void __launch_bounds__(SgsShape<T>::threads, SgsShape<T>::min_blocks)
         if (threadIdx.x == 0)
           for (int kk = k + 2; kk <= min(k - 1 + kRingSlots - 1, k1 + 1); kk++) {
             const int s2 = kk % kRingSlots;
-            if (kk != d.skip_plane) mbar_wait(&bars[s2], (phase >> s2) & 1u);  // issued copies land: the full limit
+            if (kk != skip) mbar_wait(&bars[s2], (phase >> s2) & 1u);  // issued copies land: the full limit
             phase ^= 1u << s2;
           }
         return;
       }
       const int kn = k - 1 + kRingSlots;
-      if (threadIdx.x == 0 && kn <= k1 + 1 && kn != d.skip_plane) {
+      if (threadIdx.x == 0 && kn <= k1 + 1 && kn != skip) {
         fence_async_shared();
-        issue_plane<T, 3, 0>(ring + (kn % kRingSlots) * Lay::SIZE, &bars[kn % kRingSlots], maps, wide, none, false,
-                             d.aln, i0, j0, kn);
+        issue_plane<T, 3, 0>(ring + sm * Lay::SIZE, &bars[sm], maps, wide, none, false,
+                             aln, i0, j0, kn);
       }
       c += plane;
+      sm = s0;
+      s0 = sp;
+      sp = sp + 1 == kRingSlots ? 0 : sp + 1;
     }
   }
 }

@@ -1,11 +1,7 @@
-// elmm_packed.cuh -- packed FP32x2 arithmetic (sm_100 FFMA2 / FADD2 / FMUL2)
-// for the mixed-precision momentum kernel: one thread computes two
-// x-adjacent cells with one instruction per operation pair.
-//
-// tendency_dev<C> is the wall-free tendency of the mixed path, for one cell
-// (float) or a pair (F2); on a stretched z grid (VZ) the z terms use
-// per-level factors (below).  Tiles with wall-model corrections use the
-// per-cell code.
+// elmm_packed.cuh -- the wall-free tendency of a velocity component
+// (tendency_dev<C>) for one cell (float, double) or, on the mixed path, a pair
+// of x-adjacent cells in packed FP32x2 arithmetic (sm_100 FFMA2 / FADD2 /
+// FMUL2: one instruction per operation pair).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -41,24 +37,25 @@ struct Ring2 {
   }
 };
 
-// Arithmetic on one value (float) or on a pair (F2) in the same source.
+// Arithmetic on one value (float, double) or on a pair (F2) in the same source.
 __device__ __forceinline__ float cst(float a, float) { return a; }
+__device__ __forceinline__ double cst(float a, double) { return (double)a; }
 __device__ __forceinline__ F2 cst(float a, F2) { return bc2(a); }
+__device__ __forceinline__ float fm(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fm(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ F2 fm(F2 a, F2 b, F2 c) { return fma2(a, b, c); }
 
-// per-tile constants of the FP32 tendencies (float for one cell, F2 broadcast
-// to a pair)
+// per-tile constants of the tendencies (broadcast to a pair)
 template <typename N>
 struct MomKN {
-  N Ax, Ay, Az, rx, ry, rz, q;  // cA, rec2, 0.25
-  N B[3][3];                    // cB
+  N A[3], r[3], q[3];  // cA, rec2, rec2 / 4
 };
-typedef MomKN<F2> MomK2;
 
 // Stretched z (CDU/CDV/CDW_variable_z, src/advection_variable_z.f90:15-324,
 // and MomentumDiffusion_variable_z_nobranch_2ord, src/momentum_diffusion.f90:
 // 298-420): the divisions by dzPr(k), dzW(k) and the centred differences of
 // zPr, zW become multiplications by per-level factors computed once in FP64
-// and rounded to FP32 (one rounding where the reference's form has two).
+// (rounded to FP32 on the mixed path).
 // Table rows of Dom::kz2:
 enum {
   KZ_AUV = 0,   // 1 / (4 dzPr(k))                    U, V advection through z faces
@@ -76,7 +73,6 @@ template <typename N>
 struct KZN {
   N auv, buv, d1uv, d2uv, aw, bw, d1w, d2w;
 };
-typedef KZN<F2> KZ2;
 
 // The per-level offsets of U (o) and V (p) on planes k-1, k, k+1 (the mixed
 // path stores U and V as deviations from them; see Dom::voff).
@@ -85,114 +81,127 @@ struct VelOffN {
   N o[3], p[3];
 };
 
-// One velocity component's tendency on the mixed path without wall
-// corrections: the skew-symmetric CDS2 advection (advection.f90:15-327,
+// One velocity component's tendency without wall corrections: the
+// skew-symmetric CDS2 advection (advection.f90:15-327,
 // advection_variable_z.f90:15-324 with VZ) and the explicit diffusion
-// (momentum_diffusion.f90:169-420) of the FP32 state, whose U and V hold
-// deviations from per-level offsets.  R.g() returns stored values; the
-// offsets enter only where the full value is needed, through algebraic
-// identities that keep every difference of neighbouring values a difference
-// of stored deviations:
-//   (ue + u)^2 - (u + uw)^2 = (ue - uw)(ue + 2u + uw)                 (same level)
-//   (A + 2o)(B + 2p) - (C + 2o)(D + 2p) = (AB - CD) + 2p (A - C) + 2o (B - D)
-//   a value at level k+1 minus one at level k-1 = stored difference + (o1 - om)
-// The forms are equal to the reference's term by term in exact arithmetic;
-// in FP32 they avoid differences of rounded products of the full ~several m/s
-// velocity, whose rounding noise the projection would otherwise turn into
-// pressure.  bt: the buoyancy of W (theta stored as theta - T_ref).
-template <int C, bool VZ, typename N, typename RT>
+// (momentum_diffusion.f90:169-420).  OFF: the FP32 state, whose U and V hold
+// deviations from per-level offsets (O); the offsets enter only where the
+// full value is needed, so that every difference of neighbouring values is a
+// difference of stored ones and no rounded products of the full ~several m/s
+// velocity are subtracted, whose noise the projection would turn into
+// pressure.
+//
+// The two forms of the advection share their factors, so along each axis
+// they are summed before they are evaluated.  With values f, neighbours f+,
+// f- and the transporting velocity's sums B, D on the two faces (twice their
+// face values):
+//   along itself   A (f+ - f-) (f+ + f- + 4 f),                 A = 1 / (4 d)
+//   across         A ((f+ - f-) (B + D) + (B - D) (f+ + f-) / 2 + (B - D) f)
+// where (f+ + f) B - (f + f-) D = ((f+ - f-) (B + D) + (f+ + 2 f + f-) (B - D)) / 2
+// and the advective form adds A / 2 (f+ - f-) (B + D).  That and fused
+// multiply-adds take some 58 operations a component where the two forms term
+// by term took 105; the kernel is bound by their issue and latency (with
+// buoyancy, 256 x 256 x 128: FP32 152 -> 127 us, 3.96 TB/s of its 15 words a
+// cell; FP64, whose form before was the reference's with its divisions, 408
+// -> 234 us, 4.3 TB/s).  bt: the buoyancy of W.
+template <int C, bool VZ, bool OFF, typename N, typename RT>
 __device__ __forceinline__ N tendency_dev(const MomKN<N> &K, const RT &R, const VelOffN<N> &O, N bt,
                                           const KZN<N> *Z) {
+  const N half = cst(0.5f, N{}), two = cst(2.f, N{}), four = cst(4.f, N{});
+  N a;
+  if constexpr (C < 2) {
+    // the component f of axis C, the other horizontal component g; offsets
+    // along the component's own axis and across it
+#define F(al, cr, dz) (C == 0 ? R.g(0, al, cr, dz) : R.g(1, cr, al, dz))
+#define G(al, cr, dz) (C == 0 ? R.g(1, al, cr, dz) : R.g(0, cr, al, dz))
+#define H(al, dz) (C == 0 ? R.g(2, al, 0, dz) : R.g(2, 0, al, dz))
+#define M(al, cr, dz) (C == 0 ? R.g(3, al, cr, dz) : R.g(3, cr, al, dz))
+    const N Ka = K.A[C], Kc = K.A[1 - C], Kz = K.A[2];
+    const N *o = C == 0 ? O.o : O.p, *p = C == 0 ? O.p : O.o;
+    const N f = F(0, 0, 0), fe = F(1, 0, 0), fw = F(-1, 0, 0), fn = F(0, 1, 0), fs = F(0, -1, 0);
+    const N ft = F(0, 0, 1), fb = F(0, 0, -1);
+    N s = fm(four, f, fe + fw);
+    if (OFF) s = fm(cst(6.f, N{}), o[1], s);
+    N acc = (Ka * (fe - fw)) * s;
+    {
+      const N B = G(1, 0, 0) + G(0, 0, 0), D = G(1, -1, 0) + G(0, -1, 0), BpD = B + D, BmD = B - D, df = fn - fs;
+      N t = fm(half, fn + fs, f);
+      if (OFF) t = fm(two, o[1], t);
+      const N y = fm(BmD, t, df * (OFF ? fm(four, p[1], BpD) : BpD));
+      acc = fm(Kc, y, acc);
+    }
+    {
+      const N P = H(1, 0) + H(0, 0), Q = H(1, -1) + H(0, -1), PpQ = P + Q, PmQ = P - Q;
+      N df = ft - fb, t = fm(two, f, ft + fb);
+      if (OFF) {
+        df = df + (o[2] - o[0]);
+        t = t + fm(two, o[1], o[2] + o[0]);
+      }
+      if (VZ) {
+        const N c2 = half * Z->auv;
+        acc = fm(df * PpQ, c2 + Z->buv, acc);
+        acc = fm(t * PmQ, c2, acc);
+      } else {
+        acc = fm(Kz, fm(half, t * PmQ, df * PpQ), acc);
+      }
+    }
+    a = acc * cst(-0.5f, N{});
+    const N n0 = M(0, 0, 0), ne = M(1, 0, 0), s0 = ne + n0;
+    a = fm(K.r[C], fm(n0, fw - f, ne * (fe - f)), a);
+    const N sN = s0 + (M(1, 1, 0) + M(0, 1, 0)), sS = s0 + (M(1, -1, 0) + M(0, -1, 0));
+    a = fm(K.q[1 - C], fm(sS, fs - f, sN * (fn - f)), a);
+    const N sT = s0 + (M(1, 0, 1) + M(0, 0, 1)), sB = s0 + (M(1, 0, -1) + M(0, 0, -1));
+    N dT = ft - f, dB = fb - f;
+    if (OFF) {
+      dT = dT + (o[2] - o[1]);
+      dB = dB + (o[0] - o[1]);
+    }
+    if (VZ) {
+      const N q = cst(0.25f, N{});
+      a = fm(sT * dT, q * Z->d1uv, a);
+      a = fm(sB * dB, q * Z->d2uv, a);
+    } else {
+      a = fm(K.q[2], fm(sB, dB, sT * dT), a);
+    }
+#undef F
+#undef G
+#undef H
+#undef M
+  } else {
 #define FU(dx, dy, dz) R.g(0, dx, dy, dz)
 #define FV(dx, dy, dz) R.g(1, dx, dy, dz)
-#define FW(dx, dy, dz) R.g(2, dx, dy, dz)
 #define FN(dx, dy, dz) R.g(3, dx, dy, dz)
-  const N two = cst(2.f, N{}), four = cst(4.f, N{});
-  N a;
-  if (C == 0) {
-    const N u = FU(0, 0, 0), ue = FU(1, 0, 0), uw = FU(-1, 0, 0), un = FU(0, 1, 0), us = FU(0, -1, 0);
-    const N ut = FU(0, 0, 1), ub = FU(0, 0, -1);
-    const N v = FV(0, 0, 0), ve = FV(1, 0, 0), vs = FV(0, -1, 0), vse = FV(1, -1, 0);
-    const N w = FW(0, 0, 0), we = FW(1, 0, 0), wb = FW(0, 0, -1), wbe = FW(1, 0, -1);
-    const N om = O.o[0], o0 = O.o[1], o1 = O.o[2], p0 = O.p[1];
-    const N Bx = K.B[0][0], By = K.B[0][1], Bz = K.B[0][2];
-    const N X1 = K.Ax * (ue - uw) * (((ue + u) + (u + uw)) + four * o0);
-    const N A = un + u, B = ve + v, Cc = u + us, D = vse + vs;
-    const N Y1 = K.Ay * (((A * B - Cc * D) + two * p0 * (un - us)) + two * o0 * (B - D));
-    const N Z1v = ((ut + u) * (we + w) - (u + ub) * (wbe + wb)) + ((o1 + o0) * (we + w) - (o0 + om) * (wbe + wb));
-    const N Z1 = VZ ? Z1v * Z->auv : K.Az * Z1v;
-    a = cst(0.f, N{}) - ((X1 + Y1) + Z1);
-    const N Vadv = (((v + ve) + vs) + vse) + four * p0;
-    const N Wadv = ((w + we) + wb) + wbe;
-    const N dzu = (ut - ub) + (o1 - om);
-    a = a - ((Bx * (ue - uw) * (u + o0) + By * (un - us) * Vadv) + (VZ ? dzu * Z->buv * Wadv : Bz * dzu * Wadv));
-    a = a * cst(0.5f, N{});
-    const N n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nn = FN(0, 1, 0), nne = FN(1, 1, 0), ns = FN(0, -1, 0);
-    const N nse = FN(1, -1, 0), nt = FN(0, 0, 1), nte = FN(1, 0, 1), nb = FN(0, 0, -1), nbe = FN(1, 0, -1);
-    a = a + ne * (ue - u) * K.rx;
-    a = a - n0 * (u - uw) * K.rx;
-    a = a + K.q * (((nne + ne) + nn) + n0) * (un - u) * K.ry;
-    a = a - K.q * (((ne + nse) + n0) + ns) * (u - us) * K.ry;
-    const N dt = (ut - u) + (o1 - o0), db = (u - ub) + (o0 - om);
-    a = a + K.q * (((nte + ne) + nt) + n0) * dt * (VZ ? Z->d1uv : K.rz);
-    a = a - K.q * (((ne + nbe) + n0) + nb) * db * (VZ ? Z->d2uv : K.rz);
-  } else if (C == 1) {
-    const N v = FV(0, 0, 0), ve = FV(1, 0, 0), vw = FV(-1, 0, 0), vn = FV(0, 1, 0), vs = FV(0, -1, 0);
-    const N vt = FV(0, 0, 1), vb = FV(0, 0, -1);
-    const N u = FU(0, 0, 0), un = FU(0, 1, 0), uw = FU(-1, 0, 0), unw = FU(-1, 1, 0);
-    const N w = FW(0, 0, 0), wn = FW(0, 1, 0), wb = FW(0, 0, -1), wbn = FW(0, 1, -1);
-    const N o0 = O.o[1], pm = O.p[0], p0 = O.p[1], p1 = O.p[2];
-    const N Bx = K.B[1][0], By = K.B[1][1], Bz = K.B[1][2];
-    const N Y1 = K.Ay * (vn - vs) * (((vn + v) + (v + vs)) + four * p0);
-    const N A = ve + v, B = un + u, Cc = v + vw, D = unw + uw;
-    const N X1 = K.Ax * (((A * B - Cc * D) + two * o0 * (ve - vw)) + two * p0 * (B - D));
-    const N Z1v = ((vt + v) * (wn + w) - (v + vb) * (wbn + wb)) + ((p1 + p0) * (wn + w) - (p0 + pm) * (wbn + wb));
-    const N Z1 = VZ ? Z1v * Z->auv : K.Az * Z1v;
-    a = cst(0.f, N{}) - ((Y1 + X1) + Z1);
-    const N Uadv = (((u + un) + uw) + unw) + four * o0;
-    const N Wadv = ((w + wn) + wb) + wbn;
-    const N dzv = (vt - vb) + (p1 - pm);
-    a = a - ((Bx * (ve - vw) * Uadv + By * (vn - vs) * (v + p0)) + (VZ ? dzv * Z->buv * Wadv : Bz * dzv * Wadv));
-    a = a * cst(0.5f, N{});
-    const N n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nn = FN(0, 1, 0), nne = FN(1, 1, 0), nw = FN(-1, 0, 0);
-    const N nnw = FN(-1, 1, 0), nt = FN(0, 0, 1), nnt = FN(0, 1, 1), nb = FN(0, 0, -1), nnb = FN(0, 1, -1);
-    a = a + K.q * (((nne + ne) + nn) + n0) * (ve - v) * K.rx;
-    a = a - K.q * (((nn + n0) + nnw) + nw) * (v - vw) * K.rx;
-    a = a + nn * (vn - v) * K.ry;
-    a = a - n0 * (v - vs) * K.ry;
-    const N dt = (vt - v) + (p1 - p0), db = (v - vb) + (p0 - pm);
-    a = a + K.q * (((nnt + nn) + nt) + n0) * dt * (VZ ? Z->d1uv : K.rz);
-    a = a - K.q * (((nn + nnb) + n0) + nb) * db * (VZ ? Z->d2uv : K.rz);
-  } else {
-    const N w = FW(0, 0, 0), we = FW(1, 0, 0), ww = FW(-1, 0, 0), wn = FW(0, 1, 0), ws = FW(0, -1, 0);
-    const N wt = FW(0, 0, 1), wb = FW(0, 0, -1);
-    const N u = FU(0, 0, 0), ut = FU(0, 0, 1), uw = FU(-1, 0, 0), utw = FU(-1, 0, 1);
-    const N v = FV(0, 0, 0), vt = FV(0, 0, 1), vs = FV(0, -1, 0), vts = FV(0, -1, 1);
-    const N o01 = O.o[1] + O.o[2], p01 = O.p[1] + O.p[2];
-    const N Bx = K.B[2][0], By = K.B[2][1], Bz = K.B[2][2];
-    const N Z1v = (wt + w) * (wt + w) - (w + wb) * (w + wb);
-    const N Z1 = VZ ? Z1v * Z->aw : K.Az * Z1v;
-    const N Y1 = K.Ay * (((wn + w) * (vt + v) - (w + ws) * (vs + vts)) + p01 * (wn - ws));
-    const N X1 = K.Ax * (((we + w) * (ut + u) - (w + ww) * (utw + uw)) + o01 * (we - ww));
-    a = cst(0.f, N{}) - ((Z1 + Y1) + X1);
-    const N Uadv = (((u + ut) + uw) + utw) + two * o01;
-    const N Vadv = (((v + vt) + vs) + vts) + two * p01;
-    a = a - ((Bx * (we - ww) * Uadv + By * (wn - ws) * Vadv) + (VZ ? (wt - wb) * Z->bw * w : Bz * (wt - wb) * w));
-    a = a * cst(0.5f, N{});
-    a = a + bt;  // buoyancy (the mixed path stores theta - temperature_ref)
-    const N n0 = FN(0, 0, 0), ne = FN(1, 0, 0), nt = FN(0, 0, 1), nte = FN(1, 0, 1), nw = FN(-1, 0, 0);
-    const N ntw = FN(-1, 0, 1), nn = FN(0, 1, 0), ntn = FN(0, 1, 1), ns = FN(0, -1, 0), nts = FN(0, -1, 1);
-    a = a + K.q * (((nte + ne) + nt) + n0) * (we - w) * K.rx;
-    a = a - K.q * (((nt + n0) + ntw) + nw) * (w - ww) * K.rx;
-    a = a + K.q * (((ntn + nt) + nn) + n0) * (wn - w) * K.ry;
-    a = a - K.q * (((nt + nts) + n0) + ns) * (w - ws) * K.ry;
-    a = a + nt * (wt - w) * (VZ ? Z->d1w : K.rz);
-    a = a - n0 * (w - wb) * (VZ ? Z->d2w : K.rz);
-  }
+    const N w = R.g(2, 0, 0, 0), we = R.g(2, 1, 0, 0), ww = R.g(2, -1, 0, 0), wn = R.g(2, 0, 1, 0);
+    const N ws = R.g(2, 0, -1, 0), wt = R.g(2, 0, 0, 1), wb = R.g(2, 0, 0, -1);
+    N acc;
+    if (VZ) acc = (wt - wb) * fm(Z->aw, fm(two, w, wt + wb), Z->bw * w);
+    else acc = (K.A[2] * (wt - wb)) * fm(four, w, wt + wb);
+    {
+      const N B = FV(0, 0, 1) + FV(0, 0, 0), D = FV(0, -1, 1) + FV(0, -1, 0), BpD = B + D;
+      const N y = fm(B - D, fm(half, wn + ws, w), (wn - ws) * (OFF ? fm(two, O.p[1] + O.p[2], BpD) : BpD));
+      acc = fm(K.A[1], y, acc);
+    }
+    {
+      const N B = FU(0, 0, 1) + FU(0, 0, 0), D = FU(-1, 0, 1) + FU(-1, 0, 0), BpD = B + D;
+      const N x = fm(B - D, fm(half, we + ww, w), (we - ww) * (OFF ? fm(two, O.o[1] + O.o[2], BpD) : BpD));
+      acc = fm(K.A[0], x, acc);
+    }
+    a = fm(acc, cst(-0.5f, N{}), bt);
+    const N n0 = FN(0, 0, 0), nt = FN(0, 0, 1), s0 = nt + n0;
+    const N sE = s0 + (FN(1, 0, 1) + FN(1, 0, 0)), sW = s0 + (FN(-1, 0, 1) + FN(-1, 0, 0));
+    a = fm(K.q[0], fm(sW, ww - w, sE * (we - w)), a);
+    const N sN = s0 + (FN(0, 1, 1) + FN(0, 1, 0)), sS = s0 + (FN(0, -1, 1) + FN(0, -1, 0));
+    a = fm(K.q[1], fm(sS, ws - w, sN * (wn - w)), a);
+    if (VZ) {
+      a = fm(nt * (wt - w), Z->d1w, a);
+      a = fm(n0 * (wb - w), Z->d2w, a);
+    } else {
+      a = fm(K.r[2], fm(n0, wb - w, nt * (wt - w)), a);
+    }
 #undef FU
 #undef FV
-#undef FW
 #undef FN
+  }
   return a;
 }
 
