@@ -1,7 +1,8 @@
 """Short columns of the marching kernels: depths around the chunk lengths of
 2 to 16 planes that small grids take, with the wall model at the bottom, the
 top or both (the packed wall planes of the mixed path), uniform and stretched
-z, even and odd rows, against the oracle."""
+z, even and odd rows, against the oracle (its transforms take the factors 2, 3
+and 5)."""
 import pytest
 
 from conftest import rel
@@ -19,7 +20,7 @@ WALLS = {"bottom": (BC_NOSLIP, BC_FREESLIP), "top": (BC_FREESLIP, BC_NOSLIP), "b
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
 @pytest.mark.parametrize("stretched", [False, True])
 @pytest.mark.parametrize("walls", sorted(WALLS))
-@pytest.mark.parametrize("n", [(36, 10, 4), (15, 9, 5), (34, 8, 17)])
+@pytest.mark.parametrize("n", [(36, 10, 4), (15, 9, 5), (35, 8, 17)])
 def test_columns_and_wall_planes(n, walls, stretched, precision):
     btype = (P, P, P, P) + WALLS[walls]
     zW = stretched_zw(n[2], 0.5, 1.1) if stretched else None
