@@ -416,9 +416,13 @@ struct BatchT {
   // transform phase (a batch with several x or y lengths); joined back into
   // the stream before the next phase, captured as graph branches
   static constexpr int kBranches = 4;
-  // (and one more branch for the level sums of W2)
-  cudaStream_t branch[kBranches + 1] = {};
-  cudaEvent_t ev_fork = nullptr, ev_join[kBranches + 1] = {};
+  // (and two more branches: the level sums of W2, the scalar stage)
+  enum { BR_WSUM = kBranches, BR_SCALARS, BR_N };
+  cudaStream_t branch[BR_N] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[BR_N] = {};
+  // the stream the scalar stage launches on: the batch's own, or, inside a
+  // step, its branch (run_stage)
+  cudaStream_t sstream = nullptr;
   float tune_ms[10] = {};  // rows 8, rows 4, cols 16, cols 32, momentum chunks 8/16/32, SGS chunks 8/16/32
   // immersed solid bodies per domain (elmm_set_solids): the gathers of the
   // velocity IB points followed by the nullified points, the gathers of the
@@ -559,7 +563,7 @@ struct BatchT {
       if (side) cudaStreamDestroy(side);
     }
     stream = side = nullptr;
-    for (int b = 0; b <= kBranches; b++) {
+    for (int b = 0; b < BR_N; b++) {
       if (branch[b]) cudaStreamDestroy(branch[b]);
       if (ev_join[b]) cudaEventDestroy(ev_join[b]);
       branch[b] = nullptr;
@@ -645,7 +649,10 @@ struct BatchT {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= device) return fail(ELMM_ERR_CUDA, "no CUDA device");
     CU(cudaSetDevice(device));
-    CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    // a step's chain runs ahead of the scalar stage beside it (run_stage)
+    int least = 0, greatest = 0;
+    CU(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    CU(cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, greatest));
     CU(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     CU(cudaEventCreateWithFlags(&ev_ready, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&ev_packed, cudaEventDisableTiming));
@@ -690,8 +697,11 @@ struct BatchT {
     const int n = nd;
     shell_per = n > 1 ? 4 : 1;
     CU(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    for (int b = 1; b <= kBranches; b++) {
-      CU(cudaStreamCreateWithFlags(&branch[b], cudaStreamNonBlocking));
+    sstream = stream;
+    int least = 0, greatest = 0;
+    CU(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    for (int b = 1; b < BR_N; b++) {
+      CU(cudaStreamCreateWithPriority(&branch[b], cudaStreamNonBlocking, b == BR_SCALARS ? least : greatest));
       CU(cudaEventCreateWithFlags(&ev_join[b], cudaEventDisableTiming));
     }
     void *p;
@@ -1302,15 +1312,15 @@ struct BatchT {
       for (int s = 0; s < hdom[d].nslot; s++) zghost |= hdom[d].slot[s].zg[0] || hdom[d].slot[s].zg[1];
     if (zghost) {  // BoundTemperature / BoundScalar at the start of the stage, after the stage's TDiff
       nlaunch++;
-      k_scalar_zghost<T><<<2 * 148, 256, 0, stream>>>(ddom, nd, stage);
+      k_scalar_zghost<T><<<2 * 148, 256, 0, sstream>>>(ddom, nd, stage);
     }
     if (ls[LK_TCOL].total > 0) {
       nlaunch++;
       if (scalar_bcs())
-        k_scalar<T, true><<<gsz(11, ls[LK_TCOL].total), TX * TY, 0, stream>>>(ddom, ls[LK_TCOL].l(), kRho[stage - 1],
+        k_scalar<T, true><<<gsz(11, ls[LK_TCOL].total), TX * TY, 0, sstream>>>(ddom, ls[LK_TCOL].l(), kRho[stage - 1],
                                                                              kBeta[stage - 1], stage);
       else
-        k_scalar<T><<<gsz(11, ls[LK_TCOL].total), TX * TY, 0, stream>>>(ddom, ls[LK_TCOL].l(), kRho[stage - 1],
+        k_scalar<T><<<gsz(11, ls[LK_TCOL].total), TX * TY, 0, sstream>>>(ddom, ls[LK_TCOL].l(), kRho[stage - 1],
                                                                        kBeta[stage - 1], stage);
     }
     if constexpr (std::is_same<T, float>::value) {
@@ -1324,28 +1334,28 @@ struct BatchT {
     for (int d = 0; d < nd && d < (int)sol.size(); d++)
       if (sol[d].on && sol[d].nheat > 0) {
         nlaunch++;
-        k_heat_add<T><<<std::min((sol[d].nheat + 255) / 256, 148 * 4), 256, 0, stream>>>(ddom, d, sol[d].heat,
+        k_heat_add<T><<<std::min((sol[d].nheat + 255) / 256, 148 * 4), 256, 0, sstream>>>(ddom, d, sol[d].heat,
                                                                                         sol[d].nheat, stage,
                                                                                         kBeta[stage - 1]);
       }
     for (int d = 0; d < nd && d < (int)sol.size(); d++)
       if (sol[d].on && sol[d].nfill > 0) {
         nlaunch++;
-        k_theta_fill<T><<<std::min((sol[d].nfill + 255) / 256, 148 * 4), 256, 0, stream>>>(ddom, d, sol[d].fill,
+        k_theta_fill<T><<<std::min((sol[d].nfill + 255) / 256, 148 * 4), 256, 0, sstream>>>(ddom, d, sol[d].fill,
                                                                                           sol[d].nfill, stage % 3);
       }
     bool puffs = false;
     for (int d = 0; d < nd; d++) puffs |= hdom[d].npv > 0;
     if (puffs) {
       nlaunch++;
-      k_puff_add<T><<<1, kMaxPuffVols, 0, stream>>>(ddom, nd, stage, kBeta[stage - 1]);
+      k_puff_add<T><<<1, kMaxPuffVols, 0, sstream>>>(ddom, nd, stage, kBeta[stage - 1]);
     }
     if (standalone && stage % 3 != 0)
-      k_scalar_commit<T><<<std::min(ls[LK_COMMIT].total, 16 * 148), kCommitThreads, 0, stream>>>(
+      k_scalar_commit<T><<<std::min(ls[LK_COMMIT].total, 16 * 148), kCommitThreads, 0, sstream>>>(
           ddom, ls[LK_COMMIT].l(), stage % 3);
     if (accumulate && ls[LK_AVG].total > 0) {
       nlaunch++;
-      k_scalar_avg<T><<<std::min(ls[LK_AVG].total, 8 * 148), 128, 0, stream>>>(ddom, ls[LK_AVG].l());
+      k_scalar_avg<T><<<std::min(ls[LK_AVG].total, 8 * 148), 128, 0, sstream>>>(ddom, ls[LK_AVG].l());
     }
   }
   // PressureCorrection on U2 (in_place = 0) or on U itself (initial projection)
@@ -1421,11 +1431,11 @@ struct BatchT {
       const double rho = kRho[stage - 1], beta = kBeta[stage - 1];
       const bool bc = scalar_bcs();
       if (tune_rows == 8) {
-        if (bc) k_scalar_pair<8, true><<<gsz(12, ls[LK_TPAIR].total), SPX * 8, 0, stream>>>(ddom, l, rho, beta, stage);
-        else k_scalar_pair<8><<<gsz(12, ls[LK_TPAIR].total), SPX * 8, 0, stream>>>(ddom, l, rho, beta, stage);
+        if (bc) k_scalar_pair<8, true><<<gsz(12, ls[LK_TPAIR].total), SPX * 8, 0, sstream>>>(ddom, l, rho, beta, stage);
+        else k_scalar_pair<8><<<gsz(12, ls[LK_TPAIR].total), SPX * 8, 0, sstream>>>(ddom, l, rho, beta, stage);
       } else {
-        if (bc) k_scalar_pair<4, true><<<gsz(14, ls[LK_TPAIR].total), SPX * 4, 0, stream>>>(ddom, l, rho, beta, stage);
-        else k_scalar_pair<4><<<gsz(14, ls[LK_TPAIR].total), SPX * 4, 0, stream>>>(ddom, l, rho, beta, stage);
+        if (bc) k_scalar_pair<4, true><<<gsz(14, ls[LK_TPAIR].total), SPX * 4, 0, sstream>>>(ddom, l, rho, beta, stage);
+        else k_scalar_pair<4><<<gsz(14, ls[LK_TPAIR].total), SPX * 4, 0, sstream>>>(ddom, l, rho, beta, stage);
       }
     }
   }
@@ -1460,12 +1470,12 @@ struct BatchT {
   // beside the forward transforms; joined before the z solve
   void fork_wsum(double coef_alpha2, int use_dt) {
     cudaEventRecord(ev_fork, stream);
-    cudaStreamWaitEvent(branch[kBranches], ev_fork, 0);
+    cudaStreamWaitEvent(branch[BR_WSUM], ev_fork, 0);
     nlaunch++;
-    k_wsum<T><<<std::min(ls[LK_WSUM].total, 148 * 4), kWsumThreads, 0, branch[kBranches]>>>(ddom, ls[LK_WSUM].l(), coef_alpha2, use_dt);
-    cudaEventRecord(ev_join[kBranches], branch[kBranches]);
+    k_wsum<T><<<std::min(ls[LK_WSUM].total, 148 * 4), kWsumThreads, 0, branch[BR_WSUM]>>>(ddom, ls[LK_WSUM].l(), coef_alpha2, use_dt);
+    cudaEventRecord(ev_join[BR_WSUM], branch[BR_WSUM]);
   }
-  void join_wsum() { cudaStreamWaitEvent(stream, ev_join[kBranches], 0); }
+  void join_wsum() { cudaStreamWaitEvent(stream, ev_join[BR_WSUM], 0); }
   // the five transform kernels; rhs_from_phi: the right-hand side is in Phi.
   // Phi gets no ghost pass: its only reader, k_project, folds the i+1, j+1,
   // k+1 neighbours on the box faces itself.
@@ -1558,13 +1568,33 @@ struct BatchT {
     launch_sgs(stage);
     if (any_solids()) launch_ib(0, stage);  // after BoundViscosity (src/dynamics.f90:896-902)
     if (stop == 1) return ELMM_OK;
+    // ScalarRK3 between Convection and the projection (tsteps.f90:132-135):
+    // it reads the stage's start and the diffusivity and writes the scalar
+    // slots alone, so in a whole stage it runs on a branch of its own, joined
+    // before the projection writes the new velocity.  It is as long as the
+    // transforms and leaves memory idle where they wait for their tiles; the
+    // chain has the higher priority, since a scalar kernel ahead of it in the
+    // queue holds up five short kernels (256 x 256 x 128 with buoyancy, a step
+    // in FP32: 1.587 -> 1.565 ms, 135 x 135 x 75 0.757 -> 0.730)
+    const bool beside = stop == 3 && !standalone && (ls[LK_TCOL].total > 0 || ls[LK_TPAIR].total > 0);
     launch_momentum(stage);
-    launch_scalars(stage, accumulate, standalone);  // ScalarRK3 between Convection and the projection (tsteps.f90:132-135)
+    if (beside) {
+      CU(cudaEventRecord(ev_fork, stream));
+      CU(cudaStreamWaitEvent(branch[BR_SCALARS], ev_fork, 0));
+      sstream = branch[BR_SCALARS];
+      launch_scalars(stage, accumulate);
+      sstream = stream;
+      CU(cudaEventRecord(ev_join[BR_SCALARS], branch[BR_SCALARS]));
+    } else {
+      launch_scalars(stage, accumulate, standalone);
+    }
     if (any_solids()) launch_ib(1, stage);
     if (stop == 2) return ELMM_OK;
     // the projection writes the new velocity into U itself, which takes the
     // place of the U <-> U2 pointer exchange (exchange_alloc, tsteps.f90:211-213)
-    launch_projection(2 * kAlpha[stage - 1], 1, 0);
+    launch_poisson(2 * kAlpha[stage - 1], 1, 0, 0);
+    if (beside) CU(cudaStreamWaitEvent(stream, ev_join[BR_SCALARS], 0));
+    launch_project(2 * kAlpha[stage - 1], 1, 0, 0);
     launch_refine(2 * kAlpha[stage - 1], 1);
     if (any_solids()) {
       if (div) launch_divmax();

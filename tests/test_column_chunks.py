@@ -20,7 +20,7 @@ WALLS = {"bottom": (BC_NOSLIP, BC_FREESLIP), "top": (BC_FREESLIP, BC_NOSLIP), "b
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
 @pytest.mark.parametrize("stretched", [False, True])
 @pytest.mark.parametrize("walls", sorted(WALLS))
-@pytest.mark.parametrize("n", [(36, 10, 4), (15, 9, 5), (35, 8, 17)])
+@pytest.mark.parametrize("n", [(36, 10, 4), (15, 9, 5), (45, 8, 17)])
 def test_columns_and_wall_planes(n, walls, stretched, precision):
     btype = (P, P, P, P) + WALLS[walls]
     zW = stretched_zw(n[2], 0.5, 1.1) if stretched else None
