@@ -31,13 +31,18 @@ __device__ __forceinline__ int scal_fold(int g, int n, bool periodic) {
   return g < 1 ? 1 : n;
 }
 
-// FluxLimiter of KappaScalar (src/scalar_advection.f90:262-270).  The FP32
-// path of the mixed precision mode divides by 3 as a multiplication by 1/3
-// and forms the slope ratio with the fast division (both within a few ulp);
-// the FP64 path keeps the reference's divisions.
+// FluxLimiter of KappaScalar (src/scalar_advection.f90:262-270).  The
+// division by 3 is a product with 1/3 and one correction of its remainder
+// (Markstein), the quotient rounded as a division rounds it: it was one of the
+// two divisions of an FP64 flux, 374 -> 334 us for a stage of 256 x 256 x 128.
+// (An infinite product leaves a NaN, which fmin drops as it would the infinity.)
+// The FP32 path of the mixed precision mode takes the product alone and forms the
+// slope ratio with the fast division (both within a few ulp).
 template <typename T>
 __device__ __forceinline__ T kappa_limiter(T r) {
-  return fmax((T)0, fmin((T)2 * r, fmin((T)2, ((T)1 + (T)2 * r) / (T)3)));
+  const T x = (T)1 + (T)2 * r, q = x * (T)(1.0 / 3.0);
+  const T third = fma(fma((T)-3, q, x), (T)(1.0 / 3.0), q);
+  return fmax((T)0, fmin((T)2 * r, fmin((T)2, third)));
 }
 template <>
 __device__ __forceinline__ float kappa_limiter<float>(float r) {
@@ -102,11 +107,14 @@ __global__ void k_scalar_zghost(const Dom<T> *__restrict__ doms, int nd, int sta
 // A block owns a TX x TY column of cells of one scalar slot and marches up a
 // chunk of L.kc planes; the scalar (k-2..k+2), the diffusivity (k-1..k+1)
 // and W(k-1) ride along in registers, x and y neighbours come from offsets
-// folded once per thread.  Tiles: (slot, column, chunk) per domain.
+// folded once per thread.  Bound by the latency of the FP64 divisions: four
+// blocks an SM, whose few spills cost less than the idle issue slots of three
+// (256 x 256 x 128: 334 -> 299 us; five blocks 331).  Tiles: (slot, column,
+// chunk) per domain.
 // BC: some slot has a stored z ghost plane, a surface flux or a surface
 // temperature (the launch picks the plain instantiation otherwise)
 template <typename T, bool BC = false>
-__global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 6 : 3)
+__global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 6 : 4)
     k_scalar(const Dom<T> *__restrict__ doms, Launch L, double rho, double beta, int stage) {
   const int stage1 = stage == 1;
   for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
