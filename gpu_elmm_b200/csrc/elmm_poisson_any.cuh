@@ -272,16 +272,15 @@ __device__ __forceinline__ void fftx_stage(const Dom<T> &d, typename Vec2<T>::ty
         rdzk[h] = rdz;
         const int q = r0 + 2 * sq + h;
         if (q < nrows) {
-          const int k = q / ny + 1, j = q - (k - 1) * ny + 1;
-          const long long c0 = bidx(d, 1, j, k) + (long long)c * VE;
           const RhsRow<T> &r = rinfo[2 * sq + h];
+          const long long c0 = r.c0 + (long long)c * VE;
           row(d.U2 + c0, uc[h]);
           row(d.V2 + c0, vc[h]);
           row(d.V2 + c0 + r.o_vs, vs[h]);
           row(d.W2 + c0 + r.o_wc, wc[h]);
           row(d.W2 + c0 + r.o_wb, wb[h]);
           uw0[h] = c == 0 ? r.s_uw1 * ld((const T *)d.U2, c0 + r.o_uw1) : ld((const T *)d.U2, c0 - 1);
-          if (d.vz) rdzk[h] = (T)d.sgs_rdz[k];
+          rdzk[h] = r.rdz;
         }
       }
 #pragma unroll

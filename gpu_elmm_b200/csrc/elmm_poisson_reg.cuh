@@ -36,6 +36,8 @@ template <typename T>
 struct RhsRow {
   long long o_uw1, o_vs, o_wc, o_wb;  // offsets: U2 at i - 1 for i = 1, V2 at j - 1, W2 at k, W2 at k - 1
   T s_uw1, s_vs, s_wc, s_wb;
+  long long c0;  // box index of the row's first cell
+  T rdz;         // 1 / dzPr(k)
 };
 
 template <typename T>
@@ -53,6 +55,8 @@ __device__ __forceinline__ RhsRow<T> rhs_row(const Dom<T> &d, int j, int k) {
   fold(1, 1, j - 1, pitch, r.o_vs, r.s_vs);
   fold(2, 2, k, plane, r.o_wc, r.s_wc);
   fold(2, 2, k - 1, plane, r.o_wb, r.s_wb);
+  r.c0 = bidx(d, 1, j, k);
+  r.rdz = d.vz ? (T)d.sgs_rdz[k] : (T)(1.0 / d.dz);
   return r;
 }
 
@@ -120,44 +124,58 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
   __syncthreads();
   for (int task = threadIdx.x; task < NS * NCH; task += kRegThreads) {
     const int sq = task / NCH, c = task - sq * NCH;
-    T va[VE], vb[VE];
+    T rhs[2][VE];
+    if (rhs_from_phi) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      T *out = h ? vb : va;
-      const int q = r0 + 2 * sq + h;
+      for (int h = 0; h < 2; h++) {
+        const int q = r0 + 2 * sq + h, k = q / ny + 1, j = q - (k - 1) * ny + 1;
+        T ph[VE];
 #pragma unroll
-      for (int e = 0; e < VE; e++) out[e] = (T)0;
-      if (q >= nrows) continue;  // rows past the end are not read
-      const int k = q / ny + 1, j = q - (k - 1) * ny + 1;
-      const long long c0 = bidx(d, 1, j, k) + (long long)c * VE;
-      if (rhs_from_phi) {
-        T p[VE];
-        RV::ld(d.Phi + c0, p);
+        for (int e = 0; e < VE; e++) ph[e] = (T)0;
+        if (q < nrows) RV::ld(d.Phi + bidx(d, 1, j, k) + (long long)c * VE, ph);  // rows past the end are not read
 #pragma unroll
-        for (int e = 0; e < VE; e++) out[e] = p[e] * rdt2;
-        continue;
+        for (int e = 0; e < VE; e++) rhs[h][e] = ph[e] * rdt2;
       }
-      const RhsRow<T> &r = rinfo[2 * sq + h];
-      const T rdzk = d.vz ? (T)d.sgs_rdz[k] : rdz;
-      T uc[VE], vc[VE], vs[VE], wc[VE], wb[VE];
-      RV::ld(d.U2 + c0, uc);
-      RV::ld(d.V2 + c0, vc);
-      RV::ld(d.V2 + c0 + r.o_vs, vs);
-      RV::ld(d.W2 + c0 + r.o_wc, wc);
-      RV::ld(d.W2 + c0 + r.o_wb, wb);
-      const T uw0 = c == 0 ? r.s_uw1 * ld((const T *)d.U2, c0 + r.o_uw1) : ld((const T *)d.U2, c0 - 1);
+    } else {
+      // the loads of both rows before their arithmetic: the staging waits for
+      // memory (512 x 512 x 128 175 -> 142 us, FP64 256 x 256 x 128 100 -> 80, FP64
+      // 160 x 160 x 80 56 -> 41)
+      T uc[2][VE], vc[2][VE], vs[2][VE], wc[2][VE], wb[2][VE], uw0[2], rdzk[2];
 #pragma unroll
-      for (int e = 0; e < VE; e++) {
-        const T uw = e == 0 ? uw0 : uc[e - 1];
-        const T vse = r.s_vs * vs[e];
-        const T wce = r.s_wc * wc[e], wbe = r.s_wb * wb[e];
-        const T div = (uc[e] - uw) * rdx + (vc[e] - vse) * rdy + (wce - wbe) * rdzk;
-        out[e] = div * rdt2;
+      for (int h = 0; h < 2; h++) {
+#pragma unroll
+        for (int e = 0; e < VE; e++) uc[h][e] = vc[h][e] = vs[h][e] = wc[h][e] = wb[h][e] = (T)0;
+        uw0[h] = (T)0;
+        rdzk[h] = rdz;
+        const int q = r0 + 2 * sq + h;
+        if (q < nrows) {
+          const RhsRow<T> &r = rinfo[2 * sq + h];
+          const long long c0 = r.c0 + (long long)c * VE;
+          RV::ld(d.U2 + c0, uc[h]);
+          RV::ld(d.V2 + c0, vc[h]);
+          RV::ld(d.V2 + c0 + r.o_vs, vs[h]);
+          RV::ld(d.W2 + c0 + r.o_wc, wc[h]);
+          RV::ld(d.W2 + c0 + r.o_wb, wb[h]);
+          uw0[h] = c == 0 ? r.s_uw1 * ld((const T *)d.U2, c0 + r.o_uw1) : ld((const T *)d.U2, c0 - 1);
+          rdzk[h] = r.rdz;
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const RhsRow<T> &r = rinfo[2 * sq + h];
+#pragma unroll
+        for (int e = 0; e < VE; e++) {
+          const T uw = e == 0 ? uw0[h] : uc[h][e - 1];
+          const T vse = r.s_vs * vs[h][e];
+          const T wce = r.s_wc * wc[h][e], wbe = r.s_wb * wb[h][e];
+          const T div = (uc[h][e] - uw) * rdx + (vc[h][e] - vse) * rdy + (wce - wbe) * rdzk[h];
+          rhs[h][e] = div * rdt2;
+        }
       }
     }
     T2 *dst = smem + sq * Pl::SEQ + c * VE;
 #pragma unroll
-    for (int e = 0; e < VE; e++) dst[e] = T2{va[e], vb[e]};
+    for (int e = 0; e < VE; e++) dst[e] = T2{rhs[0][e], rhs[1][e]};
   }
   __syncthreads();
   T2 *sh = smem + s * Pl::SEQ;
