@@ -885,7 +885,7 @@ struct BatchT {
       case LK_YCOLS: return fft_reg_supported(h.ny) ? 0 : ((h.nxh + TyOf<T>::v - 1) / TyOf<T>::v) * h.nz;
       case LK_MOMT:
       case LK_SGST: return column_tiles(kind, h, MX, MY);
-      case LK_WSUM: return h.nz + 1;
+      case LK_WSUM: return h.wrows ? 0 : h.nz + 1;
       case LK_WM: return (int)((wm_points_of(h) + kWmThreads - 1) / kWmThreads);
       case LK_PROJ: return fp32_pairs(h) && !slab_mode ? 0 : column_tiles(kind, h, MX, MY);
       case LK_PROJ2: return fp32_pairs(h) && !slab_mode ? column_tiles(kind, h, MX, MY) : 0;
@@ -1193,6 +1193,19 @@ struct BatchT {
     if ((r = dalloc((void **)&h.wsum, sizeof(double) * (h.nz + 2)))) return r;
     if ((r = dalloc((void **)&h.zsol, sizeof(double) * (h.nz + 2)))) return r;
     if ((r = dalloc((void **)&h.wticket, sizeof(int)))) return r;
+    // The forward x transform sums W2 where its tiles reach at most two levels
+    // and the domain is large enough to keep the chip busy: there k_wsum beside
+    // it costs the bandwidth of one more read (a step of 192 x 192 x 96 mixed 0.769 ->
+    // 0.728 ms, 256 x 256 x 128 1.569 -> 1.514, 135 x 135 x 75 0.720 -> 0.704).  On a
+    // smaller one k_wsum runs in idle SMs, and sums that end with the transform
+    // are a longer chain (128 x 128 x 64 0.392 -> 0.42, 64 x 64 x 32 0.195 -> 0.201).
+    {
+      const int rows = 2 * (fft_reg_supported(h.nx) ? fft_reg_batch(h.nx) : fft_any_seqs<T>(h.nx));
+      if (!slab_mode && rows <= h.ny && (long long)h.nx * h.ny * h.nz > kTileSumCells) {
+        h.wrows = rows;
+        if ((r = dalloc((void **)&h.wpart, sizeof(double) * 2 * ((h.ny * (size_t)h.nz + rows - 1) / rows)))) return r;
+      }
+    }
     if ((r = dalloc((void **)&h.prm, sizeof(double)))) return r;
     h.nprpart = ((h.nx + MX - 1) / MX) * ((h.ny + MY - 1) / MY);
     if ((r = dalloc((void **)&h.prpart, sizeof(double) * h.nprpart))) return r;
@@ -1466,16 +1479,28 @@ struct BatchT {
       }
     });
   }
-  // the level sums of W2 and the (0,0) mode from them (k_wsum) on a branch,
-  // beside the forward transforms; joined before the z solve
+  // the (0,0) mode on a branch, joined before the z solve: k_wsum beside the
+  // forward transforms, k_zero_mode after the one in x, beside the one in y
   void fork_wsum(double coef_alpha2, int use_dt) {
     cudaEventRecord(ev_fork, stream);
     cudaStreamWaitEvent(branch[BR_WSUM], ev_fork, 0);
+    if (ls[LK_WSUM].total == 0) return;
     nlaunch++;
     k_wsum<T><<<std::min(ls[LK_WSUM].total, 148 * 4), kWsumThreads, 0, branch[BR_WSUM]>>>(ddom, ls[LK_WSUM].l(), coef_alpha2, use_dt);
-    cudaEventRecord(ev_join[BR_WSUM], branch[BR_WSUM]);
   }
-  void join_wsum() { cudaStreamWaitEvent(stream, ev_join[BR_WSUM], 0); }
+  void fork_zero_mode(double coef_alpha2, int use_dt) {
+    bool tiles_sum = false;
+    for (auto &h : hdom) tiles_sum |= h.wrows > 0;
+    if (!tiles_sum) return;
+    cudaEventRecord(ev_fork, stream);
+    cudaStreamWaitEvent(branch[BR_WSUM], ev_fork, 0);
+    nlaunch++;
+    k_zero_mode<T><<<std::min(nd, 148 * 4), kZeroThreads, 0, branch[BR_WSUM]>>>(ddom, nd, coef_alpha2, use_dt);
+  }
+  void join_wsum() {
+    cudaEventRecord(ev_join[BR_WSUM], branch[BR_WSUM]);
+    cudaStreamWaitEvent(stream, ev_join[BR_WSUM], 0);
+  }
   // the five transform kernels; rhs_from_phi: the right-hand side is in Phi.
   // Phi gets no ghost pass: its only reader, k_project, folds the i+1, j+1,
   // k+1 neighbours on the box faces itself.
@@ -1483,6 +1508,7 @@ struct BatchT {
     const bool zsol = !rhs_from_phi;
     if (zsol) fork_wsum(coef_alpha2, use_dt);
     launch_fftx_fwd(coef_alpha2, use_dt, rhs_from_phi, gate);
+    if (zsol) fork_zero_mode(coef_alpha2, use_dt);
     launch_ffty(0, gate);
     if (zsol) join_wsum();
     launch_tri(gate, zsol);

@@ -118,7 +118,11 @@ struct Dom {
   int zper;
   // sums of W2 over each level in FP64, index k (0: a slab's bottom ghost
   // level), the solution of the (0,0) mode from them, index 1..nz, and the
-  // count of the levels done (k_wsum)
+  // count of the levels done (k_wsum); with wrows > 0 the forward x transform
+  // leaves the sums of its tiles of wrows rows in wpart (tile, then the first
+  // and the second level it reaches) for k_zero_mode instead
+  double *wpart;
+  int wrows;
   double *wsum, *zsol;
   int *wticket;
   // grid tables (FP64), index k + 2 for k in [-2, nz + 3]

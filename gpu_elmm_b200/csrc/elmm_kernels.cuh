@@ -339,21 +339,95 @@ __global__ void __launch_bounds__(kWmThreads) k_wm_points(const Dom<T> *__restri
 namespace elmm {
 
 // ------------------------------------------------------------- Poisson
-// Sums of W2 over each level, FP64, one block a level in a fixed order, and
-// from them the (0,0) mode of the Poisson problem (src/poisson.f90:23-60):
-// the mean divergence of a level, whose x and y parts telescope to nothing,
-// is the difference of two of these sums, so the flux of the mode through a
-// level's top is the sum itself (less the bottom's) and its solution one
-// prefix sum, which the domain's last block takes, its mean pinned to zero.
-// Taken from the FP32 transform instead, the mode's rounding, independent
-// from level to level, is integrated twice: a large and, as one mode's, a
-// very uneven part of the error of the mixed pressure (64 x 64 x 32 after 40
-// steps: 3.2e-4 of the pressure, 1.4e-4 with the sums); and the serial sum
-// was the longest chain of the z solve on small grids.  One word per cell,
-// on a graph branch beside the forward transforms: wide blocks with kVec
-// vectors in flight per thread.  The mixed step of 256 x 256 x 128 takes 2.5%
-// longer with it (the z solve 10 us a stage less, the branch more), that of
-// 64 x 64 x 32 2% less.
+// The (0,0) mode of the Poisson problem (src/poisson.f90:23-60) from FP64 sums
+// of W2 over each level.  The mean divergence of a level, whose x and y parts
+// telescope to nothing, is the difference of two of these sums, so the flux
+// of the mode through a level's top is the sum itself (less the bottom's) and
+// its solution one prefix sum, its mean pinned to zero.  Taken from the FP32
+// transform instead, the mode's rounding, independent from level to level, is
+// integrated twice: a large and, as one mode's, a very uneven part of the
+// error of the mixed pressure (64 x 64 x 32 after 40 steps: 3.2e-4 of the
+// pressure, 1.4e-4 with the sums); and the serial sum was the longest chain
+// of the z solve on small grids.
+//
+// The sums come from the forward x transform, which has W2 in registers
+// (Dom::wrows: large domains), or from k_wsum beside it (small ones, slabs).
+
+// zsol from the level sums; every thread of the block calls it
+template <int NT, typename T>
+__device__ __forceinline__ void zero_mode_solve(const Dom<T> &d, double coef, double *red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nz = d.nz;
+  // x(k + 1) = x(k) + (F(k) + F0) dzf(k) with F(k) = (level(k) - level(0)) norm / coef
+  const double c = 1.0 / coef * (1.0 / ((double)d.nx * (double)d.ny));
+  auto level = [&](int g) {
+    const Fold f = fold_vel(g, d.ext[2][2], d.bt[4], d.bt[5], true);
+    return f.zero ? 0.0 : f.sign * __ldcg(d.wsum + f.src);
+  };
+  const double l0 = level(0);
+  auto block_sum = [&](double v, double &before) -> double {  // the block's sum, and the sum of the threads before
+    double x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) red[warp] = x;
+    __syncthreads();
+    double tot = 0, pre = 0;
+    for (int w = 0; w < NT / 32; w++) {
+      if (w < warp) pre += red[w];
+      tot += red[w];
+    }
+    before = pre + (x - v);
+    return tot;
+  };
+  const int per = (nz + NT - 1) / NT, k0 = 1 + threadIdx.x * per, k1 = min(nz, k0 + per - 1);
+  double F0 = 0, before;
+  if (d.zper) {  // so that x is periodic: sum_k dzf(k) (F(k) + F0) = 0
+    double a = 0, b = 0;
+    for (int q = k0; q <= k1; q++) { a += (level(q) - l0) * c * d.dzf[q]; b += d.dzf[q]; }
+    const double sa = block_sum(a, before), sb = block_sum(b, before);
+    F0 = -sa / sb;
+  }
+  double g = 0;  // the increments of this thread's levels
+  for (int q = k0; q <= k1; q++) g += ((level(q) - l0) * c + F0) * d.dzf[q];
+  block_sum(g, before);
+  double x = before, sx = 0;
+  for (int q = k0; q <= k1; q++) { sx += x; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
+  double unused;
+  const double mean = block_sum(sx, unused) / nz;
+  x = before;
+  for (int q = k0; q <= k1; q++) { d.zsol[q] = x - mean; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
+  __syncthreads();
+}
+
+// the domains whose level sums the forward x transform left per tile: a block
+// a domain, a thread a level
+constexpr int kZeroThreads = 256;
+constexpr long long kTileSumCells = 5 << 18;  // domains of more cells leave their sums per tile
+template <typename T>
+__global__ void __launch_bounds__(kZeroThreads) k_zero_mode(const Dom<T> *__restrict__ doms, int nd, double coef_alpha2,
+                                                            int use_dt) {
+  __shared__ double red[kZeroThreads / 32];
+  for (int di = blockIdx.x; di < nd; di += gridDim.x) {
+    const Dom<T> &d = doms[di];
+    if (!d.wrows) continue;
+    const int ny = d.ny, wr = d.wrows;
+    for (int k = 1 + threadIdx.x; k <= d.nz; k += kZeroThreads) {
+      // rows (k-1) ny .. k ny - 1; a tile's second level only if it is this one
+      const int t0 = (int)((long long)(k - 1) * ny / wr), t1 = (int)(((long long)k * ny - 1) / wr);
+      double s = 0;
+#pragma unroll 4
+      for (int t = t0; t <= t1; t++) s += __ldcg(d.wpart + 2 * t + (k - 1 - (int)((long long)t * wr / ny)));
+      d.wsum[k] = s;
+    }
+    __syncthreads();
+    zero_mode_solve<kZeroThreads>(d, use_dt ? coef_alpha2 * d.dt : coef_alpha2, red);
+  }
+}
+
+// Sums of W2 over each level, one block a level in a fixed order, wide blocks
+// with kVec vectors in flight per thread; the domain's last block solves.
 constexpr int kWsumThreads = 512;
 template <typename T>
 __global__ void __launch_bounds__(kWsumThreads, 2) k_wsum(const Dom<T> *__restrict__ doms, Launch L, double coef_alpha2,
@@ -417,47 +491,7 @@ __global__ void __launch_bounds__(kWsumThreads, 2) k_wsum(const Dom<T> *__restri
     __syncthreads();
     if (last && d.bt[SIDE_BO] != BC_HALO && d.bt[SIDE_TO] != BC_HALO) {
       __threadfence();
-      // x(k + 1) = x(k) + (F(k) + F0) dzf(k) with F(k) = (level(k) - level(0)) rdt norm
-      const double c = 1.0 / (use_dt ? coef_alpha2 * d.dt : coef_alpha2) * (1.0 / ((double)nx * (double)ny));
-      auto level = [&](int g) {
-        const Fold f = fold_vel(g, d.ext[2][2], d.bt[4], d.bt[5], true);
-        return f.zero ? 0.0 : f.sign * __ldcg(d.wsum + f.src);
-      };
-      const double l0 = level(0);
-      auto block_sum = [&](double v, double &before) -> double {  // the block's sum, and the sum of the threads before
-        double x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-          const double y = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += y;
-        }
-        __syncthreads();
-        if (lane == 31) red[warp] = x;
-        __syncthreads();
-        double tot = 0, pre = 0;
-        for (int w = 0; w < kWsumThreads / 32; w++) {
-          if (w < warp) pre += red[w];
-          tot += red[w];
-        }
-        before = pre + (x - v);
-        return tot;
-      };
-      const int per = (nz + kWsumThreads - 1) / kWsumThreads, k0 = 1 + threadIdx.x * per, k1 = min(nz, k0 + per - 1);
-      double F0 = 0, before;
-      if (d.zper) {  // so that x is periodic: sum_k dzf(k) (F(k) + F0) = 0
-        double a = 0, b = 0;
-        for (int q = k0; q <= k1; q++) { a += (level(q) - l0) * c * d.dzf[q]; b += d.dzf[q]; }
-        const double sa = block_sum(a, before), sb = block_sum(b, before);
-        F0 = -sa / sb;
-      }
-      double g = 0;  // the increments of this thread's levels
-      for (int q = k0; q <= k1; q++) g += ((level(q) - l0) * c + F0) * d.dzf[q];
-      block_sum(g, before);
-      double x = before, sx = 0;
-      for (int q = k0; q <= k1; q++) { sx += x; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
-      double unused;
-      const double mean = block_sum(sx, unused) / nz;
-      x = before;
-      for (int q = k0; q <= k1; q++) { d.zsol[q] = x - mean; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
+      zero_mode_solve<kWsumThreads>(d, use_dt ? coef_alpha2 * d.dt : coef_alpha2, red);
     }
     __syncthreads();
   }

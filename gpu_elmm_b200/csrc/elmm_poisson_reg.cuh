@@ -38,6 +38,7 @@ struct RhsRow {
   T s_uw1, s_vs, s_wc, s_wb;
   long long c0;  // box index of the row's first cell
   T rdz;         // 1 / dzPr(k)
+  int dk;        // the row's level less the level of its tile's first row
 };
 
 template <typename T>
@@ -60,22 +61,37 @@ __device__ __forceinline__ RhsRow<T> rhs_row(const Dom<T> &d, int j, int k) {
   return r;
 }
 
-// right-hand side at interior cell i of a row, box index c: the divergence
-// of (U2, V2, W2) / coef, or the value already stored in Phi (PoisSolver
-// interface, defect correction)
-template <typename T>
-__device__ __forceinline__ T poisson_rhs(const Dom<T> &d, const RhsRow<T> &r, long long c, int i, T rdx, T rdy,
-                                         T rdzk, T rdt2, int rhs_from_phi) {
-  if (rhs_from_phi) return ld((const T *)d.Phi, c) * rdt2;
-  const T *U2 = d.U2, *V2 = d.V2, *W2 = d.W2;
-  const long long ouw = i == 1 ? r.o_uw1 : -1;
-  const T suw = i == 1 ? r.s_uw1 : (T)1;
-  const T uc = ld(U2, c), uw = suw * ld(U2, c + ouw);
-  const T vc = ld(V2, c), vs = r.s_vs * ld(V2, c + r.o_vs);
-  const T wc = r.s_wc * ld(W2, c + r.o_wc), wb = r.s_wb * ld(W2, c + r.o_wb);
-  const T div = (uc - uw) * rdx + (vc - vs) * rdy + (wc - wb) * rdzk;
-  return div * rdt2;
-}
+// The level sums of W2 of an x tile (Dom::wpart): each thread adds the values
+// it stages, a row vector in T and the vectors in FP64, to the first or second
+// level of the tile's rows.
+struct LevelSums {
+  double a[2];
+  template <typename T, int VE>
+  __device__ __forceinline__ void add(const T (&w)[VE], const RhsRow<T> &r) {
+    T v = w[0];
+#pragma unroll
+    for (int e = 1; e < VE; e++) v += w[e];
+    const double x = (double)(v * r.s_wc);
+    a[0] += r.dk ? 0.0 : x;
+    a[1] += r.dk ? x : 0.0;
+  }
+  // a warp's sums into red[warp]; the block then calls put after a barrier
+  __device__ __forceinline__ void warp_sums(double (*red)[2]) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = a[q];
+    }
+  }
+  template <int NW>
+  static __device__ __forceinline__ void put(double (*red)[2], double *part) {
+    if (threadIdx.x < 2) {
+      double s = 0;
+      for (int w = 0; w < NW; w++) s += red[w][threadIdx.x];
+      part[threadIdx.x] = s;
+    }
+  }
+};
 
 // ------------------------------------------------------------ x forward
 // 16-byte vectors of a row: four floats or two doubles (rows start on a
@@ -111,6 +127,7 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
   constexpr int P = Pl::P, E = Pl::E, NS = kRegThreads / P;
   constexpr int VE = RV::n, NCH = N / VE;
   __shared__ RhsRow<T> rinfo[2 * NS];
+  __shared__ double wred[kRegThreads / 32][2];
   const int s = threadIdx.x / P, t = threadIdx.x - s * P;
   const int ny = d.ny, nrows = ny * d.nz;
   const int r0 = 2 * lt * NS;  // first row of the tile; sequence q holds rows r0 + 2q, r0 + 2q + 1
@@ -120,8 +137,11 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
     const int q = min(r0 + (int)threadIdx.x, nrows - 1);
     const int k = q / ny + 1;
     rinfo[threadIdx.x] = rhs_row(d, q - (k - 1) * ny + 1, k);
+    rinfo[threadIdx.x].dk = k - 1 - r0 / ny;
   }
   __syncthreads();
+  const bool sums = d.wrows > 0 && !rhs_from_phi;
+  LevelSums ls{{0, 0}};
   for (int task = threadIdx.x; task < NS * NCH; task += kRegThreads) {
     const int sq = task / NCH, c = task - sq * NCH;
     T rhs[2][VE];
@@ -171,13 +191,16 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
           const T div = (uc[h][e] - uw) * rdx + (vc[h][e] - vse) * rdy + (wce - wbe) * rdzk[h];
           rhs[h][e] = div * rdt2;
         }
+        if (sums) ls.add(wc[h], r);
       }
     }
     T2 *dst = smem + sq * Pl::SEQ + c * VE;
 #pragma unroll
     for (int e = 0; e < VE; e++) dst[e] = T2{rhs[0][e], rhs[1][e]};
   }
+  if (sums) ls.warp_sums(wred);
   __syncthreads();
+  if (sums) LevelSums::put<kRegThreads / 32>(wred, d.wpart + 2 * lt);
   T2 *sh = smem + s * Pl::SEQ;
   T2 v[E];
 #pragma unroll
