@@ -610,7 +610,11 @@ struct BatchT {
                                         std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
     allocs.push_back(*p);
-    return cudaMemset(*p, 0, bytes) == cudaSuccess ? ELMM_OK : fail(ELMM_ERR_CUDA, "cudaMemset");
+    // on the batch's stream, and done before the memory is handed out: a memset
+    // on the default stream is not ordered with the batch's copies and kernels,
+    // which on a busy GPU (a request admitted beside a running chunk) overtake it
+    return cudaMemsetAsync(*p, 0, bytes, stream) == cudaSuccess && cudaStreamSynchronize(stream) == cudaSuccess
+               ? ELMM_OK : fail(ELMM_ERR_CUDA, "cudaMemset");
   }
   // returns one allocation early (the host-layout staging of a serving
   // request after its upload)
