@@ -631,12 +631,21 @@ struct BatchT {
     }
   }
 
+  // Pageable host data into device memory, landed when the call returns.  On
+  // the batch's stream: a cudaMemcpy from pageable memory returns once the
+  // source is staged, and nothing orders its end on the default stream with
+  // the kernels of a non-blocking one, which could then start on an old launch
+  // map or descriptor.
+  int to_device(void *dst, const void *src, size_t bytes) {
+    CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
+    CU(cudaStreamSynchronize(stream));
+    return ELMM_OK;
+  }
   template <typename X>
   int upload_table(const X **dst, const std::vector<X> &v) {
     void *p;
     int r = dalloc(&p, v.size() * sizeof(X));
-    if (r) return r;
-    CU(cudaMemcpy(p, v.data(), v.size() * sizeof(X), cudaMemcpyHostToDevice));
+    if (r || (r = to_device(p, v.data(), v.size() * sizeof(X)))) return r;
     *dst = (const X *)p;
     return ELMM_OK;
   }
@@ -712,11 +721,11 @@ struct BatchT {
     int r = dalloc(&p, sizeof(Dom<T>) * n);
     if (r) return r;
     ddom = (Dom<T> *)p;
-    CU(cudaMemcpy(ddom, hdom.data(), sizeof(Dom<T>) * n, cudaMemcpyHostToDevice));
+    if ((r = to_device(ddom, hdom.data(), sizeof(Dom<T>) * n))) return r;
     r = dalloc(&p, sizeof(PoisPlan) * n);
     if (r) return r;
     dplan = (PoisPlan *)p;
-    CU(cudaMemcpy(dplan, hplan.data(), sizeof(PoisPlan) * n, cudaMemcpyHostToDevice));
+    if ((r = to_device(dplan, hplan.data(), sizeof(PoisPlan) * n))) return r;
     r = dalloc((void **)&dbad, sizeof(int));
     if (r) return r;
     int maxnx = 0, maxny = 0, maxnz = 0, anyzper = 0;
@@ -798,7 +807,7 @@ struct BatchT {
       ls[k].total = st[n];
       r = dalloc((void **)&ls[k].starts, sizeof(int) * (n + 1));
       if (r) return r;
-      CU(cudaMemcpy(ls[k].starts, st.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
+      if ((r = to_device(ls[k].starts, st.data(), sizeof(int) * (n + 1)))) return r;
     }
     // one launch set per distinct x (y) length, holding only its domains
     auto reg_sets = [&](bool use, bool ydir, std::vector<RegSet> &out) -> int {
@@ -818,8 +827,7 @@ struct BatchT {
         r.ls.nd = nd;
         r.ls.total = st[nd];
         int rr = dalloc((void **)&r.ls.starts, sizeof(int) * (nd + 1));
-        if (rr) return rr;
-        CU(cudaMemcpy(r.ls.starts, st.data(), sizeof(int) * (nd + 1), cudaMemcpyHostToDevice));
+        if (rr || (rr = to_device(r.ls.starts, st.data(), sizeof(int) * (nd + 1)))) return rr;
         const void *f1 = ydir ? (const void *)r.k->yf : (const void *)r.k->fwd;
         const void *f2 = ydir ? (const void *)r.k->yi : (const void *)r.k->inv;
         // the dynamic maximum leaves room for the kernel's static shared memory
@@ -990,7 +998,7 @@ struct BatchT {
       void *p;
       int r = dalloc(&p, maps.size() * sizeof(CUtensorMap));
       if (r) return r;
-      CU(cudaMemcpy(p, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+      if ((r = to_device(p, maps.data(), maps.size() * sizeof(CUtensorMap)))) return r;
       h.tmaps = p;
     }
     h.nxh = h.nx / 2 + 1;
@@ -1095,11 +1103,10 @@ struct BatchT {
         if ((r = dalloc((void **)&h.wm_fluxm[f], np * sizeof(T)))) return r;
         if ((r = dalloc((void **)&h.wm_ustar[f], np * sizeof(double)))) return r;
         std::vector<double> ones(np, 1.0);  // WMPointUVW%ustar = 1 initially (wallmodels.f90:80)
-        CU(cudaMemcpy(h.wm_ustar[f], ones.data(), np * sizeof(double), cudaMemcpyHostToDevice));
+        if ((r = to_device(h.wm_ustar[f], ones.data(), np * sizeof(double)))) return r;
         if (c.enable_buoyancy && (s == ELMM_BO || s == ELMM_TO) && c.TempBtype[s] == ELMM_BC_DIRICHLET) {
-          // a prescribed surface temperature: the points' temperature_flux, 0 initially
+          // a prescribed surface temperature: the points' temperature_flux, 0 initially (dalloc)
           if ((r = dalloc((void **)&h.wm_tfl[f], np * sizeof(double)))) return r;
-          CU(cudaMemset(h.wm_tfl[f], 0, np * sizeof(double)));
         }
       }
     if (c.enable_buoyancy) {
@@ -1120,7 +1127,7 @@ struct BatchT {
           if ((r = encode_box_map(&tm[b2], sl.buf[b2], h.pitch, h.ny, h.nz, MX, MY))) return r;
         void *p;
         if ((r = dalloc(&p, tm.size() * sizeof(CUtensorMap)))) return r;
-        CU(cudaMemcpy(p, tm.data(), tm.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
+        if ((r = to_device(p, tm.data(), tm.size() * sizeof(CUtensorMap)))) return r;
         h.tmapT = p;
       }
       for (int s2 = 0; s2 < 6; s2++) sl.bt[s2] = c.TempBtype[s2];
@@ -1145,8 +1152,7 @@ struct BatchT {
           if ((r = dalloc((void **)&h.wm_pr_us[hh], np * sizeof(double)))) return r;
           if ((r = dalloc((void **)&h.wm_pr_tf[hh], np * sizeof(double)))) return r;
           std::vector<double> ones(np, 1.0);
-          CU(cudaMemcpy(h.wm_pr_us[hh], ones.data(), np * sizeof(double), cudaMemcpyHostToDevice));
-          CU(cudaMemset(h.wm_pr_tf[hh], 0, np * sizeof(double)));
+          if ((r = to_device(h.wm_pr_us[hh], ones.data(), np * sizeof(double)))) return r;
         }
       h.wm_af = area_factor;
       set_zghosts(sl, c.TempBtype, c.sideTemp, h.wall);
@@ -1188,7 +1194,7 @@ struct BatchT {
       // TDiff starts at the molecular diffusivity (src/initial.f90:4262-4268)
       if (c.molecular_viscosity > 0) {
         std::vector<T> kv(alloc_elems, (T)c.molecular_diffusivity);
-        CU(cudaMemcpy(h.TDiff, kv.data(), alloc_elems * sizeof(T), cudaMemcpyHostToDevice));
+        if ((r = to_device(h.TDiff, kv.data(), alloc_elems * sizeof(T)))) return r;
       }
     }
     // mixed path: the per-level offsets of U and V (zero until the first
@@ -1218,7 +1224,7 @@ struct BatchT {
     {
       const double ts[2] = {0.0, c.dt};  // time 0, no step yet
       if ((r = dalloc((void **)&h.tstate, sizeof(ts)))) return r;
-      CU(cudaMemcpy(h.tstate, ts, sizeof(ts), cudaMemcpyHostToDevice));
+      if ((r = to_device(h.tstate, ts, sizeof(ts)))) return r;
     }
     if ((r = dalloc((void **)&h.flags, 4 * sizeof(int)))) return r;
     h.wait_limit = kWaitLimit;
@@ -1231,7 +1237,7 @@ struct BatchT {
     if ((r = dalloc((void **)&pr_image[di], pe * sizeof(double)))) return r;
     // viscosity starts at the molecular value (src/initial.f90:4275)
     std::vector<T> nuv(box, (T)c.molecular_viscosity);
-    CU(cudaMemcpy(h.nu, nuv.data(), box * sizeof(T), cudaMemcpyHostToDevice));
+    if ((r = to_device(h.nu, nuv.data(), box * sizeof(T)))) return r;
     hdom[di] = h;
     return ELMM_OK;
   }
@@ -1708,9 +1714,8 @@ struct BatchT {
     if (kind == LK_TPAIR) ls[kind].kc = short_chunk(kind, MKC, grid_cap[tune_rows == 8 ? 12 : 14]);
     std::vector<int> st(nd + 1, 0);
     for (int d = 0; d < nd; d++) st[d + 1] = st[d] + tiles(kind, hdom[d]);
-    CU(cudaMemcpy(ls[kind].starts, st.data(), sizeof(int) * (nd + 1), cudaMemcpyHostToDevice));
     ls[kind].total = st[nd];
-    return ELMM_OK;
+    return to_device(ls[kind].starts, st.data(), sizeof(int) * (nd + 1));
   }
 
   // The autotuner: before the first step of a batch (or view), times each
@@ -1884,8 +1889,8 @@ struct BatchT {
         h.puff_clear_any = 1;
       }
     }
-    CU(cudaMemcpy(h.puff_state, st.data(), st.size() * sizeof(double), cudaMemcpyHostToDevice));
-    return push_dom(d);
+    int r = to_device(h.puff_state, st.data(), st.size() * sizeof(double));
+    return r ? r : push_dom(d);
   }
 
   // ------------------------------------------------------------ solids
@@ -1979,8 +1984,7 @@ struct BatchT {
         }
     if (fc.empty()) return ELMM_OK;
     int rr = dalloc((void **)&x.fill, fc.size() * sizeof(FillCell));
-    if (rr) return rr;
-    CU(cudaMemcpy(x.fill, fc.data(), fc.size() * sizeof(FillCell), cudaMemcpyHostToDevice));
+    if (rr || (rr = to_device(x.fill, fc.data(), fc.size() * sizeof(FillCell)))) return rr;
     x.nfill = (int)fc.size();
     return ELMM_OK;
   }
@@ -2100,8 +2104,7 @@ struct BatchT {
       if (bytes == 0) return (int)ELMM_OK;
       int rr = dalloc(dst, bytes);
       if (rr) return rr;
-      return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess ? (int)ELMM_OK
-                                                                                 : fail(ELMM_ERR_CUDA, "cudaMemcpy");
+      return to_device(*dst, src, bytes);
     };
     if ((r = up((void **)&x.vel, vel.data(), vel.size() * sizeof(IBGather)))) return r;
     if ((r = up((void **)&x.null, nulls.data(), nulls.size() * sizeof(long long)))) return r;
@@ -2203,8 +2206,7 @@ struct BatchT {
     return ELMM_OK;
   }
   int push_dom(int d) {
-    CU(cudaMemcpy(ddom + d, &hdom[d], sizeof(Dom<T>), cudaMemcpyHostToDevice));
-    return ELMM_OK;
+    return to_device(ddom + d, &hdom[d], sizeof(Dom<T>));
   }
 
   // enqueues nsteps replays of the step graph (captured on first use) without
@@ -2272,11 +2274,11 @@ struct BatchT {
       CU(cudaMemcpy(fl, hdom[d].flags, sizeof(fl), cudaMemcpyDeviceToHost));
       if (fl[1]) {  // a bounded device-side wait gave up: report it once
         gave_up = 1;
-        CU(cudaMemset(hdom[d].flags + 1, 0, sizeof(int)));
+        CU(cudaMemsetAsync(hdom[d].flags + 1, 0, sizeof(int), stream));
       }
       if (fl[2]) {  // a variable step started at end_time
         past_end = 1;
-        CU(cudaMemset(hdom[d].flags + 2, 0, sizeof(int)));
+        CU(cudaMemsetAsync(hdom[d].flags + 2, 0, sizeof(int), stream));
       }
       unsigned long long b1 = 0, b2 = 0;
       CU(cudaMemcpy(&b1, hdom[d].maxdiv_bits, sizeof(b1), cudaMemcpyDeviceToHost));

@@ -519,7 +519,7 @@ struct SlabsT {
       CU(cudaMemcpy(fl, h.flags, sizeof(fl), cudaMemcpyDeviceToHost));
       if (fl[1]) {
         gave_up = 1;
-        CU(cudaMemset(h.flags + 1, 0, sizeof(int)));
+        CU(cudaMemsetAsync(h.flags + 1, 0, sizeof(int), sl[s]->stream));
       }
       unsigned long long b1 = 0, b2 = 0;
       CU(cudaMemcpy(&b1, h.maxdiv_bits, sizeof(b1), cudaMemcpyDeviceToHost));
