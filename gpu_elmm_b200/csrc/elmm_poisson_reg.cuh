@@ -62,16 +62,15 @@ __device__ __forceinline__ RhsRow<T> rhs_row(const Dom<T> &d, int j, int k) {
 }
 
 // The level sums of W2 of an x tile (Dom::wpart): each thread adds the values
-// it stages, a row vector in T and the vectors in FP64, to the first or second
-// level of the tile's rows.
+// it stages, in FP64, to the first or second level of the tile's rows.
 struct LevelSums {
   double a[2];
   template <typename T, int VE>
   __device__ __forceinline__ void add(const T (&w)[VE], const RhsRow<T> &r) {
-    T v = w[0];
+    double x = 0;
 #pragma unroll
-    for (int e = 1; e < VE; e++) v += w[e];
-    const double x = (double)(v * r.s_wc);
+    for (int e = 0; e < VE; e++) x += (double)w[e];
+    x *= (double)r.s_wc;
     a[0] += r.dk ? 0.0 : x;
     a[1] += r.dk ? x : 0.0;
   }

@@ -52,3 +52,28 @@ def test_step_follows_the_oracle(n, z, precision):
         else:
             # two roundings of W meet in a level's flux: its own and the level's below
             assert float(np.abs(a - b).max()) < 2 * P_MIXED_ABS * max(1.0, n[2] / 64)
+
+
+# Both kinds of x transform that leave the sums of their tiles (domains of more
+# than 1.3 M cells).  A row of W repeats (1, e, -1, e) with 1 + e = 1 in FP32:
+# the mean e / 2 of a level survives only if every value is widened before it
+# is added.  Away from the walls, where the rest of the divergence is, the
+# pressure rises by its solution's e / 2 a level; the bound is the FP32
+# rounding of a level's value, at most nz / 2 such rises from the mean.
+@pytest.mark.parametrize("n", [(256, 256, 40), (300, 128, 40)])
+def test_tile_sums_keep_every_bit(n):
+    nx, ny, nz = n
+    e = 2.0 ** -26
+    rise = []
+    for precision in (PREC_FP64, PREC_MIXED):
+        cfg = make_config(*n, precision=precision, btype=(P, P, P, P) + BOTTOM)
+        g = grid_of(cfg)
+        st = [np.zeros(s) for s in (g.shape_u(), g.shape_v(), g.shape_w(), g.shape_p())]
+        st[2][3:-3, 3:-3, 3:-3] = np.tile([1.0, e, -1.0, e], nx // 4)
+        d = L.Domain(cfg)
+        d.upload(*st)
+        d.project(1.0)
+        rise.append(np.diff(d.download()[3][2:-2, 2:-2, 2:-2].mean((1, 2)))[nz // 2 - 5:nz // 2 + 4])
+        d.close()
+    assert rel(rise[0], np.full(9, e / 2)) < 1e-9
+    assert rel(rise[1], rise[0]) < 2 * nz / 2 * 2.0 ** -24
