@@ -897,7 +897,7 @@ struct BatchT {
       case LK_YCOLS: return fft_reg_supported(h.ny) ? 0 : ((h.nxh + TyOf<T>::v - 1) / TyOf<T>::v) * h.nz;
       case LK_MOMT:
       case LK_SGST: return column_tiles(kind, h, MX, MY);
-      case LK_WSUM: return h.wrows ? 0 : h.nz + 1;
+      case LK_WSUM: return h.wrows ? 0 : h.nz;
       case LK_WM: return (int)((wm_points_of(h) + kWmThreads - 1) / kWmThreads);
       case LK_PROJ: return fp32_pairs(h) && !slab_mode ? 0 : column_tiles(kind, h, MX, MY);
       case LK_PROJ2: return fp32_pairs(h) && !slab_mode ? column_tiles(kind, h, MX, MY) : 0;
@@ -1200,20 +1200,20 @@ struct BatchT {
     // mixed path: the per-level offsets of U and V (zero until the first
     // upload; see Dom::voff)
     if (sizeof(T) == 4 && (r = dalloc((void **)&h.voff, sizeof(float) * 2 * (h.nz + 2)))) return r;
-    if ((r = dalloc((void **)&h.wsum, sizeof(double) * (h.nz + 2)))) return r;
-    if ((r = dalloc((void **)&h.zsol, sizeof(double) * (h.nz + 2)))) return r;
+    // (a slab's level sums, or their parts, lie in the whole domain's: SlabsT)
+    if (!slab_mode && (r = dalloc((void **)&h.wsum, sizeof(double) * (h.nz + 2)))) return r;
+    if (!slab_mode && (r = dalloc((void **)&h.zsol, sizeof(double) * (h.nz + 2)))) return r;
     if ((r = dalloc((void **)&h.wticket, sizeof(int)))) return r;
-    // The forward x transform sums W2 where its tiles reach at most two levels
+    // The forward x transform sums W2 where its tiles lie each in one level
     // and the domain is large enough to keep the chip busy: there k_wsum beside
     // it costs the bandwidth of one more read (a step of 192 x 192 x 96 mixed 0.769 ->
-    // 0.728 ms, 256 x 256 x 128 1.569 -> 1.514, 135 x 135 x 75 0.720 -> 0.704).  On a
-    // smaller one k_wsum runs in idle SMs, and sums that end with the transform
+    // 0.728 ms, 256 x 256 x 128 1.569 -> 1.514).  On a smaller one k_wsum runs in idle SMs, and sums that end with the transform
     // are a longer chain (128 x 128 x 64 0.392 -> 0.42, 64 x 64 x 32 0.195 -> 0.201).
     {
       const int rows = 2 * (fft_reg_supported(h.nx) ? fft_reg_batch(h.nx) : fft_any_seqs<T>(h.nx));
-      if (!slab_mode && rows <= h.ny && (long long)h.nx * h.ny * h.nz > kTileSumCells) {
+      if (h.ny % rows == 0 && (long long)h.nx * h.ny * (zparent ? zparent->nz : h.nz) > kTileSumCells) {
         h.wrows = rows;
-        if ((r = dalloc((void **)&h.wpart, sizeof(double) * 2 * ((h.ny * (size_t)h.nz + rows - 1) / rows)))) return r;
+        if (!slab_mode && (r = dalloc((void **)&h.wpart, sizeof(double) * (h.ny / rows) * (size_t)h.nz))) return r;
       }
     }
     if ((r = dalloc((void **)&h.prm, sizeof(double)))) return r;

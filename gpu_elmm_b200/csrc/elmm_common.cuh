@@ -116,11 +116,11 @@ struct Dom {
   const double *lamx, *lamy, *Ab, *At, *dzc, *dzf;
   const double *tri_c0;  // [piece][ny * spitch]: carry of the pivot recurrence at each piece start (tiled z solve)
   int zper;
-  // sums of W2 over each level in FP64, index k (0: a slab's bottom ghost
-  // level), the solution of the (0,0) mode from them, index 1..nz, and the
-  // count of the levels done (k_wsum); with wrows > 0 the forward x transform
-  // leaves the sums of its tiles of wrows rows in wpart (tile, then the first
-  // and the second level it reaches) for k_zero_mode instead
+  // sums of W2 over each level in FP64, index k, the solution of the (0,0)
+  // mode from them, index 1..nz (null in a slab: k_slab_zero), and the count
+  // of the levels done (k_wsum); with wrows > 0 the forward x transform leaves
+  // the sums of its tiles of wrows rows (ny / wrows tiles a level) in wpart
+  // for k_zero_mode instead
   double *wpart;
   int wrows;
   double *wsum, *zsol;

@@ -351,18 +351,21 @@ namespace elmm {
 // of the z solve on small grids.
 //
 // The sums come from the forward x transform, which has W2 in registers
-// (Dom::wrows: large domains), or from k_wsum beside it (small ones, slabs).
+// (Dom::wrows: large domains), or from k_wsum beside it.  Both add them in an
+// order that depends on nx and ny alone, so that a level has one sum wherever
+// a domain is cut into slabs.
 
-// zsol from the level sums; every thread of the block calls it
-template <int NT, typename T>
-__device__ __forceinline__ void zero_mode_solve(const Dom<T> &d, double coef, double *red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nz = d.nz;
+// zsol[1..nz] from the level sums (level(k), k = 0..nz, with the boundary
+// conditions applied); c: norm / coef; every thread of the block calls it.
+// One block size for every caller, so that a domain, alone or in slabs, has
+// one result.
+constexpr int kZeroThreads = 512;
+template <typename F>
+__device__ __forceinline__ void zero_mode_solve(int nz, int zper, const double *__restrict__ dzf, double c, F &&level,
+                                                double *zsol, double *red) {
+  constexpr int NT = kZeroThreads;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // x(k + 1) = x(k) + (F(k) + F0) dzf(k) with F(k) = (level(k) - level(0)) norm / coef
-  const double c = 1.0 / coef * (1.0 / ((double)d.nx * (double)d.ny));
-  auto level = [&](int g) {
-    const Fold f = fold_vel(g, d.ext[2][2], d.bt[4], d.bt[5], true);
-    return f.zero ? 0.0 : f.sign * __ldcg(d.wsum + f.src);
-  };
   const double l0 = level(0);
   auto block_sum = [&](double v, double &before) -> double {  // the block's sum, and the sum of the threads before
     double x = v;
@@ -383,27 +386,45 @@ __device__ __forceinline__ void zero_mode_solve(const Dom<T> &d, double coef, do
   };
   const int per = (nz + NT - 1) / NT, k0 = 1 + threadIdx.x * per, k1 = min(nz, k0 + per - 1);
   double F0 = 0, before;
-  if (d.zper) {  // so that x is periodic: sum_k dzf(k) (F(k) + F0) = 0
+  if (zper) {  // so that x is periodic: sum_k dzf(k) (F(k) + F0) = 0
     double a = 0, b = 0;
-    for (int q = k0; q <= k1; q++) { a += (level(q) - l0) * c * d.dzf[q]; b += d.dzf[q]; }
+    for (int q = k0; q <= k1; q++) { a += (level(q) - l0) * c * dzf[q]; b += dzf[q]; }
     const double sa = block_sum(a, before), sb = block_sum(b, before);
     F0 = -sa / sb;
   }
   double g = 0;  // the increments of this thread's levels
-  for (int q = k0; q <= k1; q++) g += ((level(q) - l0) * c + F0) * d.dzf[q];
+  for (int q = k0; q <= k1; q++) g += ((level(q) - l0) * c + F0) * dzf[q];
   block_sum(g, before);
   double x = before, sx = 0;
-  for (int q = k0; q <= k1; q++) { sx += x; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
+  for (int q = k0; q <= k1; q++) { sx += x; x += ((level(q) - l0) * c + F0) * dzf[q]; }
   double unused;
   const double mean = block_sum(sx, unused) / nz;
   x = before;
-  for (int q = k0; q <= k1; q++) { d.zsol[q] = x - mean; x += ((level(q) - l0) * c + F0) * d.dzf[q]; }
+  for (int q = k0; q <= k1; q++) { zsol[q] = x - mean; x += ((level(q) - l0) * c + F0) * dzf[q]; }
   __syncthreads();
 }
 
+// the level sums from the forward x transform's np tiles a level, a thread a level
+__device__ __forceinline__ void sum_tiles(const double *part, int np, int nz, double *wsum) {
+  for (int k = 1 + threadIdx.x; k <= nz; k += kZeroThreads) {
+    double s = 0;
+#pragma unroll 4
+    for (int q = 0; q < np; q++) s += __ldcg(part + (long long)(k - 1) * np + q);
+    wsum[k] = s;
+  }
+  __syncthreads();
+}
+template <typename T>
+__device__ __forceinline__ void zero_mode(const Dom<T> &d, double coef, double *red) {
+  auto level = [&](int g) {
+    const Fold f = fold_vel(g, d.ext[2][2], d.bt[4], d.bt[5], true);
+    return f.zero ? 0.0 : f.sign * __ldcg(d.wsum + f.src);
+  };
+  zero_mode_solve(d.nz, d.zper, d.dzf, 1.0 / coef * (1.0 / ((double)d.nx * (double)d.ny)), level, d.zsol, red);
+}
+
 // the domains whose level sums the forward x transform left per tile: a block
-// a domain, a thread a level
-constexpr int kZeroThreads = 256;
+// a domain
 constexpr long long kTileSumCells = 5 << 18;  // domains of more cells leave their sums per tile
 template <typename T>
 __global__ void __launch_bounds__(kZeroThreads) k_zero_mode(const Dom<T> *__restrict__ doms, int nd, double coef_alpha2,
@@ -412,23 +433,15 @@ __global__ void __launch_bounds__(kZeroThreads) k_zero_mode(const Dom<T> *__rest
   for (int di = blockIdx.x; di < nd; di += gridDim.x) {
     const Dom<T> &d = doms[di];
     if (!d.wrows) continue;
-    const int ny = d.ny, wr = d.wrows;
-    for (int k = 1 + threadIdx.x; k <= d.nz; k += kZeroThreads) {
-      // rows (k-1) ny .. k ny - 1; a tile's second level only if it is this one
-      const int t0 = (int)((long long)(k - 1) * ny / wr), t1 = (int)(((long long)k * ny - 1) / wr);
-      double s = 0;
-#pragma unroll 4
-      for (int t = t0; t <= t1; t++) s += __ldcg(d.wpart + 2 * t + (k - 1 - (int)((long long)t * wr / ny)));
-      d.wsum[k] = s;
-    }
-    __syncthreads();
-    zero_mode_solve<kZeroThreads>(d, use_dt ? coef_alpha2 * d.dt : coef_alpha2, red);
+    sum_tiles(d.wpart, d.ny / d.wrows, d.nz, d.wsum);
+    zero_mode(d, use_dt ? coef_alpha2 * d.dt : coef_alpha2, red);
   }
 }
 
 // Sums of W2 over each level, one block a level in a fixed order, wide blocks
-// with kVec vectors in flight per thread; the domain's last block solves.
-constexpr int kWsumThreads = 512;
+// with kVec vectors in flight per thread; the last block of a domain (of no
+// slab) solves.
+constexpr int kWsumThreads = kZeroThreads;
 template <typename T>
 __global__ void __launch_bounds__(kWsumThreads, 2) k_wsum(const Dom<T> *__restrict__ doms, Launch L, double coef_alpha2,
                                                        int use_dt) {
@@ -439,39 +452,27 @@ __global__ void __launch_bounds__(kWsumThreads, 2) k_wsum(const Dom<T> *__restri
   for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
     const int di = find_dom(L.starts, L.nd, t);
     const Dom<T> &d = doms[di];
-    const int k = t - __ldg(L.starts + di);
+    const int k = t - __ldg(L.starts + di) + 1;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
-    if (k <= d.ext[2][2] && (k > 0 || d.bt[SIDE_BO] == BC_HALO)) {
+    if (k <= d.ext[2][2]) {
       const long long pitch = d.pitch;
       const T *W = d.W2 + bidx(d, 1, 1, k);
       double s = 0;
-      if (nx % VE == 0) {
-        const int nv = nx / VE, n = nv * ny;  // 16-byte vectors of the level
-        for (int q0 = threadIdx.x; q0 < n; q0 += kWsumThreads * kVec) {
-          float4 v[kVec];
+      const int nv = (nx + VE - 1) / VE, n = nv * ny;  // 16-byte vectors of the level, a row's last one into its padding
+      for (int q0 = threadIdx.x; q0 < n; q0 += kWsumThreads * kVec) {
+        float4 v[kVec];
+        int left[kVec];  // values of the row from the vector's first on
 #pragma unroll
-          for (int u = 0; u < kVec; u++) {
-            const int q = q0 + u * kWsumThreads, j = q / nv;
-            v[u] = q < n ? __ldg(reinterpret_cast<const float4 *>(W + j * pitch) + (q - j * nv)) : make_float4(0, 0, 0, 0);
-          }
-#pragma unroll
-          for (int u = 0; u < kVec; u++) {
-            const T *e = reinterpret_cast<const T *>(&v[u]);
-#pragma unroll
-            for (int c = 0; c < VE; c++) s += (double)e[c];
-          }
+        for (int u = 0; u < kVec; u++) {
+          const int q = q0 + u * kWsumThreads, j = q / nv, c = q - j * nv;
+          left[u] = q < n ? nx - c * VE : 0;
+          v[u] = q < n ? __ldg(reinterpret_cast<const float4 *>(W + j * pitch) + c) : make_float4(0, 0, 0, 0);
         }
-      } else {
-        const int n = nx * ny;
-        for (int q0 = threadIdx.x; q0 < n; q0 += kWsumThreads * kVec) {
-          T v[kVec];
 #pragma unroll
-          for (int u = 0; u < kVec; u++) {
-            const int q = q0 + u * kWsumThreads, j = q / nx;
-            v[u] = q < n ? __ldg(W + j * pitch + (q - j * nx)) : (T)0;
-          }
+        for (int u = 0; u < kVec; u++) {
+          const T *e = reinterpret_cast<const T *>(&v[u]);
 #pragma unroll
-          for (int u = 0; u < kVec; u++) s += (double)v[u];
+          for (int c = 0; c < VE; c++) s += c < left[u] ? (double)e[c] : 0.0;
         }
       }
       for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
@@ -485,13 +486,13 @@ __global__ void __launch_bounds__(kWsumThreads, 2) k_wsum(const Dom<T> *__restri
     }
     if (threadIdx.x == 0) {
       __threadfence();
-      last = atomicAdd(d.wticket, 1) == nz;  // nz + 1 tiles
+      last = atomicAdd(d.wticket, 1) == nz - 1;  // nz tiles
       if (last) *d.wticket = 0;
     }
     __syncthreads();
-    if (last && d.bt[SIDE_BO] != BC_HALO && d.bt[SIDE_TO] != BC_HALO) {
+    if (last && d.zsol) {
       __threadfence();
-      zero_mode_solve<kWsumThreads>(d, use_dt ? coef_alpha2 * d.dt : coef_alpha2, red);
+      zero_mode(d, use_dt ? coef_alpha2 * d.dt : coef_alpha2, red);
     }
     __syncthreads();
   }

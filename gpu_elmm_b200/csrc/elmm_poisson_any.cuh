@@ -235,10 +235,10 @@ __device__ __forceinline__ void fftx_passes(const FFTFactors &f, int ns, typenam
 
 // the right-hand sides of an x tile's rows into buf, VE cells a task: the
 // divergence of PrePoisson (pressure.f90:688-717) from vectors of VE cells of
-// a row; and their level sums of W2
+// a row; and the tile's sum of W2
 template <typename T, int VE>
 __device__ __forceinline__ void fftx_stage(const Dom<T> &d, typename Vec2<T>::type *buf, const RhsRow<T> *rinfo, int r0,
-                                           int ns, double coef, int rhs_from_phi, LevelSums &ls) {
+                                           int ns, double coef, int rhs_from_phi, TileSum &ls) {
   typedef typename Vec2<T>::type T2;
   const int pitch = fft_any_pitch(ns), nch = d.nx / VE, ny = d.ny, nrows = ny * d.nz;
   const T rdt2 = (T)(1.0 / coef);
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kFFTThreadsX, sizeof(T) == 4 ? 6 : 4)
   typedef typename Vec2<T>::type T2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ RhsRow<T> rinfo[2 * kMaxSeqX];
-  __shared__ double wred[kFFTThreadsX / 32][2];
+  __shared__ double wred[kFFTThreadsX / 32];
   T2 *buf = reinterpret_cast<T2 *>(smem_raw);
   for (int t = blockIdx.x; t < L.total; t += gridDim.x) {
     const int di = find_dom(L.starts, L.nd, t);
@@ -327,16 +327,15 @@ __global__ void __launch_bounds__(kFFTThreadsX, sizeof(T) == 4 ? 6 : 4)
       const int q = min(r0 + (int)threadIdx.x, nrows - 1);
       const int k = q / ny + 1;
       rinfo[threadIdx.x] = rhs_row(d, q - (k - 1) * ny + 1, k);
-      rinfo[threadIdx.x].dk = k - 1 - r0 / ny;
     }
     __syncthreads();
     const bool sums = d.wrows > 0 && !rhs_from_phi;
-    LevelSums ls{{0, 0}};
+    TileSum ls{0};
     if (N % Row16<T>::n == 0) fftx_stage<T, Row16<T>::n>(d, buf, rinfo, r0, ns, coef, rhs_from_phi, ls);
     else fftx_stage<T, 1>(d, buf, rinfo, r0, ns, coef, rhs_from_phi, ls);
-    if (sums) ls.warp_sums(wred);
+    if (sums) ls.warp_sum(wred);
     __syncthreads();
-    if (sums) LevelSums::put<kFFTThreadsX / 32>(wred, d.wpart + 2 * (t - __ldg(L.starts + di)));
+    if (sums) TileSum::put<kFFTThreadsX / 32>(wred, d.wpart + (t - __ldg(L.starts + di)));
     fftx_passes<T, false>(pl.fx, ns, buf, out, d.twx);
     // Z = FFT(a + i b): A_m = (Z_m + conj Z_{N-m}) / 2, B_m = (Z_m - conj Z_{N-m}) / 2i;
     // a warp takes 32 modes of a sequence

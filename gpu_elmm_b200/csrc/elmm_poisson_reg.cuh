@@ -38,7 +38,6 @@ struct RhsRow {
   T s_uw1, s_vs, s_wc, s_wb;
   long long c0;  // box index of the row's first cell
   T rdz;         // 1 / dzPr(k)
-  int dk;        // the row's level less the level of its tile's first row
 };
 
 template <typename T>
@@ -61,33 +60,28 @@ __device__ __forceinline__ RhsRow<T> rhs_row(const Dom<T> &d, int j, int k) {
   return r;
 }
 
-// The level sums of W2 of an x tile (Dom::wpart): each thread adds the values
-// it stages, in FP64, to the first or second level of the tile's rows.
-struct LevelSums {
-  double a[2];
+// The sum of W2 over an x tile, whose rows lie in one level (Dom::wpart): each
+// thread adds the values it stages, in FP64.
+struct TileSum {
+  double a;
   template <typename T, int VE>
   __device__ __forceinline__ void add(const T (&w)[VE], const RhsRow<T> &r) {
     double x = 0;
 #pragma unroll
     for (int e = 0; e < VE; e++) x += (double)w[e];
-    x *= (double)r.s_wc;
-    a[0] += r.dk ? 0.0 : x;
-    a[1] += r.dk ? x : 0.0;
+    a += x * (double)r.s_wc;
   }
-  // a warp's sums into red[warp]; the block then calls put after a barrier
-  __device__ __forceinline__ void warp_sums(double (*red)[2]) {
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][q] = a[q];
-    }
+  // a warp's sum into red[warp]; the block then calls put after a barrier
+  __device__ __forceinline__ void warp_sum(double *red) {
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
   }
   template <int NW>
-  static __device__ __forceinline__ void put(double (*red)[2], double *part) {
-    if (threadIdx.x < 2) {
+  static __device__ __forceinline__ void put(const double *red, double *part) {
+    if (threadIdx.x == 0) {
       double s = 0;
-      for (int w = 0; w < NW; w++) s += red[w][threadIdx.x];
-      part[threadIdx.x] = s;
+      for (int w = 0; w < NW; w++) s += red[w];
+      *part = s;
     }
   }
 };
@@ -126,7 +120,7 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
   constexpr int P = Pl::P, E = Pl::E, NS = kRegThreads / P;
   constexpr int VE = RV::n, NCH = N / VE;
   __shared__ RhsRow<T> rinfo[2 * NS];
-  __shared__ double wred[kRegThreads / 32][2];
+  __shared__ double wred[kRegThreads / 32];
   const int s = threadIdx.x / P, t = threadIdx.x - s * P;
   const int ny = d.ny, nrows = ny * d.nz;
   const int r0 = 2 * lt * NS;  // first row of the tile; sequence q holds rows r0 + 2q, r0 + 2q + 1
@@ -136,11 +130,10 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
     const int q = min(r0 + (int)threadIdx.x, nrows - 1);
     const int k = q / ny + 1;
     rinfo[threadIdx.x] = rhs_row(d, q - (k - 1) * ny + 1, k);
-    rinfo[threadIdx.x].dk = k - 1 - r0 / ny;
   }
   __syncthreads();
   const bool sums = d.wrows > 0 && !rhs_from_phi;
-  LevelSums ls{{0, 0}};
+  TileSum ls{0};
   for (int task = threadIdx.x; task < NS * NCH; task += kRegThreads) {
     const int sq = task / NCH, c = task - sq * NCH;
     T rhs[2][VE];
@@ -197,9 +190,9 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
 #pragma unroll
     for (int e = 0; e < VE; e++) dst[e] = T2{rhs[0][e], rhs[1][e]};
   }
-  if (sums) ls.warp_sums(wred);
+  if (sums) ls.warp_sum(wred);
   __syncthreads();
-  if (sums) LevelSums::put<kRegThreads / 32>(wred, d.wpart + 2 * lt);
+  if (sums) TileSum::put<kRegThreads / 32>(wred, d.wpart + lt);
   T2 *sh = smem + s * Pl::SEQ;
   T2 v[E];
 #pragma unroll

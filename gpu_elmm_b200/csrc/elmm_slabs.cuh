@@ -17,9 +17,9 @@
 // depend on the grid only: k_slab_tri_pivots runs the pivot recurrence of
 // the whole column once at creation and keeps the slab's levels, with the
 // operations of tri_pivot (so the values of a single-domain solve).  The
-// (0,0) mode is singular: its right-hand side is gathered whole into every
-// slab, and each slab runs the zero-mean prefix-sum solution of k_tri_tile
-// and keeps its own levels.
+// (0,0) mode is singular: the sums of W2 over the levels are gathered whole
+// into every slab, and each runs the solution of the single domain
+// (k_slab_zero) and takes its own levels.
 #pragma once
 
 #include "elmm_common.cuh"
@@ -51,25 +51,29 @@ __global__ void k_slab_tri_pivots(double *iv, const double *__restrict__ lamx, c
   }
 }
 
-// the (0,0) mode's right-hand side at a slab's level k (before the norm): the
-// real part from the level sums, as the single domain takes it
+// The (0,0) mode: every slab solves the whole column (zero_mode_solve) from
+// the level sums of all slabs, zpart[(k - 1) * np + q] (np: tiles a level of
+// the forward x transform, or 1 for k_wsum's sums), k = 1..nzg.  bt0, bt1:
+// the whole domain's bottom and top; dzf: its spacings, index 1..nzg.
 template <typename T>
-__device__ __forceinline__ double slab_zero_rhs(const Dom<T> &d, int k, int part, double coef_alpha2, int use_dt) {
-  if (part) return 0.0;  // the mean of a real field
+__global__ void __launch_bounds__(kZeroThreads)
+    k_slab_zero(const Dom<T> *__restrict__ dom, const double *zpart, int np, double *wsum, double *zsol,
+                const double *__restrict__ dzf, int nzg, int bt0, int bt1, double coef_alpha2, int use_dt) {
+  __shared__ double red[kZeroThreads / 32];
+  const Dom<T> &d = *dom;
+  sum_tiles(zpart, np, nzg, wsum);
   auto level = [&](int g) {
-    const Fold f = fold_vel(g, d.ext[2][2], d.bt[4], d.bt[5], true);
-    return f.zero ? 0.0 : f.sign * d.wsum[f.src];
+    const Fold f = fold_vel(g, nzg - 1, bt0, bt1, true);  // walls in z
+    return f.zero ? 0.0 : f.sign * __ldcg(wsum + f.src);
   };
-  return (level(k) - level(k - 1)) * (d.vz ? d.sgs_rdz[k] : 1.0 / d.dz) / (use_dt ? coef_alpha2 * d.dt : coef_alpha2);
+  const double coef = use_dt ? coef_alpha2 * d.dt : coef_alpha2;
+  zero_mode_solve(nzg, 0, dzf, 1.0 / coef * (1.0 / ((double)d.nx * (double)d.ny)), level, zsol, red);
 }
 
 // The maps of a slab's forward sweep with entry y(k0) = 0:
 // fmap[part * ncol + col] = A (part 0 real, 1 imaginary), fmap[2 * ncol + col] = B.
-// The (0,0) mode's right-hand side goes to zcol[part * nzg + k0 + k - 1].
 template <typename T>
-__global__ void k_slab_tri_fmap(const Dom<T> *__restrict__ dom, const double *__restrict__ iv, double *fmap,
-                                double *zcol, int k0, int nzg, double coef_alpha2,
-                                int use_dt) {
+__global__ void k_slab_tri_fmap(const Dom<T> *__restrict__ dom, const double *__restrict__ iv, double *fmap) {
   const Dom<T> &d = *dom;
   const int ncol = d.ny * d.spitch, nz = d.nz;
   const long long ks = 2LL * ncol;  // T elements per level of S
@@ -77,12 +81,8 @@ __global__ void k_slab_tri_fmap(const Dom<T> *__restrict__ dom, const double *__
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * ncol; t += gridDim.x * blockDim.x) {
     const int col = t >> 1, part = t & 1;
     const int ky = col / d.spitch, kx = col - ky * d.spitch;
-    if (kx >= d.nxh) continue;
+    if (kx >= d.nxh || (kx == 0 && ky == 0)) continue;
     const T *x = reinterpret_cast<const T *>(d.S) + 2LL * col + part;  // level k at x[(k - 1) * ks]
-    if (kx == 0 && ky == 0) {
-      for (int k = 1; k <= nz; k++) zcol[(long long)part * nzg + k0 + k - 1] = slab_zero_rhs(d, k, part, coef_alpha2, use_dt);
-      continue;
-    }
     double A = 0, B = 1;
     for (int k = 1; k <= nz; k++) {
       const double ivk = iv[(long long)(k - 1) * ncol + col];
@@ -100,13 +100,10 @@ __global__ void k_slab_tri_fmap(const Dom<T> *__restrict__ dom, const double *__
 // into S, and the map of the slab's backward sweep into bmap (layout of
 // fmap): x(k0 + 1) = A' + B' x(k0 + nzl + 1), accumulated upwards as
 // A' = sum_k y(k) prod_{j<k} g(j), B' = prod g, g = -At iv.  The (0,0)
-// mode: the zero-mean solution of the whole column from zcol (every slab
-// computes the same column; dzc, dzf are the whole domain's, index 1..nzg),
-// this slab's levels written.
+// mode: this slab's levels of the solution, zsol[1..nz] (its mean is real).
 template <typename T>
 __global__ void k_slab_tri_fwd(const Dom<T> *__restrict__ dom, const double *__restrict__ iv,
-                               const double *__restrict__ fmaps, double *bmap, const double *__restrict__ zcol,
-                               const double *__restrict__ dzc, const double *__restrict__ dzf, int k0, int nzg, int s) {
+                               const double *__restrict__ fmaps, double *bmap, const double *__restrict__ zsol, int s) {
   const Dom<T> &d = *dom;
   const int ncol = d.ny * d.spitch, nz = d.nz;
   const long long ks = 2LL * ncol, ms = 3LL * ncol;
@@ -117,19 +114,7 @@ __global__ void k_slab_tri_fwd(const Dom<T> *__restrict__ dom, const double *__r
     if (kx >= d.nxh) continue;
     T *x = reinterpret_cast<T *>(d.S) + 2LL * col + part;
     if (kx == 0 && ky == 0) {
-      // F(k) = F(k-1) + dzc(k) r(k) is the flux (x(k+1) - x(k)) / dzf(k)
-      const double *r = zcol + (long long)part * nzg;
-      double sx = 0;
-      for (int pass = 0; pass < 2; pass++) {  // the mean, then the levels less the mean
-        double F = 0, xx = 0;
-        for (int k = 1; k <= nzg; k++) {
-          if (pass == 0) sx += xx;
-          else if (k > k0 && k <= k0 + nz) x[(k - k0 - 1) * ks] = (T)(xx - sx);
-          F = F + (r[k - 1] * norm) * dzc[k];
-          xx = xx + F * dzf[k];
-        }
-        if (pass == 0) sx = sx / nzg;
-      }
+      for (int k = 1; k <= nz; k++) x[(k - 1) * ks] = part ? (T)0 : (T)zsol[k];
       continue;
     }
     double y = 0;  // y(k0)
@@ -268,8 +253,7 @@ struct SlabTile {
 // tiled k_slab_tri_fmap
 template <typename T, int COLS>
 __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
-    k_slab_tri_fmap_tile(const Dom<T> *__restrict__ dom, const double *__restrict__ iv, double *fmap, double *zcol,
-                         int k0, int nzg, double coef_alpha2, int use_dt) {
+    k_slab_tri_fmap_tile(const Dom<T> *__restrict__ dom, const double *__restrict__ iv, double *fmap) {
   typedef SlabTile<T, COLS> Tl;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Dom<T> &d = *dom;
@@ -291,9 +275,6 @@ __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
       fmap[(long long)t.part * ncol + t.col] = A;
       if (t.part == 0) fmap[2LL * ncol + t.col] = B;
     }
-    if (t.seg == 0 && t.active && t.zero)
-      for (int k = 1; k <= t.nz; k++)
-        zcol[(long long)t.part * nzg + k0 + k - 1] = slab_zero_rhs(d, k, t.part, coef_alpha2, use_dt);
     __syncthreads();  // the shared memory is free for the next tile
   }
 }
@@ -302,8 +283,7 @@ __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
 template <typename T, int COLS>
 __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
     k_slab_tri_fwd_tile(const Dom<T> *__restrict__ dom, const double *__restrict__ iv, const double *__restrict__ fmaps,
-                        double *bmap, const double *__restrict__ zcol, const double *__restrict__ dzc,
-                        const double *__restrict__ dzf, int k0, int nzg, int s) {
+                        double *bmap, const double *__restrict__ zsol, int s) {
   typedef SlabTile<T, COLS> Tl;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const Dom<T> &d = *dom;
@@ -327,21 +307,8 @@ __global__ void __launch_bounds__(SlabTile<T, COLS>::THREADS)
         t.x(k) = (T)y;
       }
     }
-    if (t.seg == 0 && t.active && t.zero) {
-      // the zero-mean solution of the whole (0,0) column (k_slab_tri_fwd)
-      const double *r = zcol + (long long)t.part * nzg;
-      double sx = 0;
-      for (int pass = 0; pass < 2; pass++) {  // the mean, then the levels less the mean
-        double F = 0, xx = 0;
-        for (int k = 1; k <= nzg; k++) {
-          if (pass == 0) sx += xx;
-          else if (k > k0 && k <= k0 + t.nz) t.x(k - k0) = (T)(xx - sx);
-          F = F + (r[k - 1] * norm) * dzc[k];
-          xx = xx + F * dzf[k];
-        }
-        if (pass == 0) sx = sx / nzg;
-      }
-    }
+    if (t.active && t.zero)
+      for (int k = t.kb; k <= t.ke; k++) t.x(k) = t.part ? (T)0 : (T)zsol[k];
     __syncthreads();  // the forward maps are read, the segments replayed
     t.bwd_map(d.At, A, B);
     t.put_maps(A, B);

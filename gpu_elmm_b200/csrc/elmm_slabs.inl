@@ -14,8 +14,8 @@
 //   after the SGS kernel      nu          both ways
 //   after the momentum kernel W2          upwards (the divergence reads W2(k-1))
 //   z solve                   the maps of the forward and backward sweeps
-//                             (3 numbers per column and slab) and the (0,0)
-//                             column (elmm_slabs.cuh)
+//                             (3 numbers per column and slab) and the level
+//                             sums of W2 (elmm_slabs.cuh)
 //   after the inverse FFTs    Phi         downwards (the projection reads Phi(k+1))
 //   after the projection      U V W P     both ways, and the pressure
 //                             reference of the top slab to every slab
@@ -37,8 +37,11 @@ struct SlabsT {
   std::vector<std::unique_ptr<BatchT<T>>> sl;
   // per slab: pivots of its levels, the sweep maps of every slab, the (0,0) column
   struct Tri {
-    double *iv = nullptr, *fmaps = nullptr, *bmaps = nullptr, *zcol = nullptr;
-    const double *dzc = nullptr, *dzf = nullptr;
+    double *iv = nullptr, *fmaps = nullptr, *bmaps = nullptr;
+    // the (0,0) mode (k_slab_zero): the parts of the level sums of W2 of every
+    // level, the sums, and the solution, both with index 1..nzg
+    double *zpart = nullptr, *wsum = nullptr, *zsol = nullptr;
+    const double *dzf = nullptr;
   };
   std::vector<Tri> tri;
   // slabs of at most kTriTileMaxNz levels take the tiled sweep kernels
@@ -46,6 +49,7 @@ struct SlabsT {
   typedef SlabTile<T, kSlabCols> Tile;
   bool tiled = false;
   size_t smem_tile = 0;
+  int zparts = 1;  // parts of a level's sum of W2 (Tri::zpart)
   std::vector<cudaEvent_t> pre, post;
   cudaEvent_t t0 = nullptr, t1 = nullptr, ev_fork = nullptr;
   double time = 0;
@@ -94,14 +98,13 @@ struct SlabsT {
     make_grid(c, ggrid);
     // the whole column's coefficients of the z solve and the (0,0) mode's
     // spacings (as init_domain forms them for one domain)
-    std::vector<double> Ab(nzg + 2, 0.0), At(nzg + 2, 0.0), dzc(nzg + 2, 0.0), dzf(nzg + 2, 0.0);
+    std::vector<double> Ab(nzg + 2, 0.0), At(nzg + 2, 0.0), dzf(nzg + 2, 0.0);
     {
       auto zP = [&](int k) { return ggrid.zPr[k + 2]; };
       auto zWf = [&](int k) { return ggrid.zW[k + 2]; };
       for (int k = 1; k <= nzg; k++) {
         Ab[k] = 1 / ((zP(k) - zP(k - 1)) * (zWf(k) - zWf(k - 1)));
         At[k] = 1 / ((zP(k + 1) - zP(k)) * (zWf(k) - zWf(k - 1)));
-        dzc[k] = zWf(k) - zWf(k - 1);
         dzf[k] = zP(k + 1) - zP(k);
       }
       Ab[1] = 0;
@@ -137,14 +140,19 @@ struct SlabsT {
       const int ncol = h.ny * h.spitch;
       Tri &x = tri[s];
       const double *Abg, *Atg;
-      if ((r = B.upload_table(&Abg, Ab)) || (r = B.upload_table(&Atg, At)) || (r = B.upload_table(&x.dzc, dzc)) ||
-          (r = B.upload_table(&x.dzf, dzf)))
-        return r;
+      if ((r = B.upload_table(&Abg, Ab)) || (r = B.upload_table(&Atg, At)) || (r = B.upload_table(&x.dzf, dzf))) return r;
+      zparts = h.wrows ? h.ny / h.wrows : 1;
       if ((r = B.dalloc((void **)&x.iv, sizeof(double) * (size_t)nzl[s] * ncol)) ||
           (r = B.dalloc((void **)&x.fmaps, sizeof(double) * 3 * (size_t)ncol * n)) ||
           (r = B.dalloc((void **)&x.bmaps, sizeof(double) * 3 * (size_t)ncol * n)) ||
-          (r = B.dalloc((void **)&x.zcol, sizeof(double) * 2 * (size_t)nzg)))
+          (r = B.dalloc((void **)&x.zpart, sizeof(double) * zparts * (size_t)nzg)) ||
+          (r = B.dalloc((void **)&x.wsum, sizeof(double) * (nzg + 2))) ||
+          (r = B.dalloc((void **)&x.zsol, sizeof(double) * (nzg + 2))))
         return r;
+      // the slab's own part of it
+      if (h.wrows) B.hdom[0].wpart = x.zpart + (size_t)k0[s] * zparts;
+      else B.hdom[0].wsum = x.zpart + k0[s] - 1;  // index 1..nz
+      if ((r = B.push_dom(0))) return r;
       k_slab_tri_pivots<<<(ncol + 127) / 128, 128, 0, B.stream>>>(x.iv, h.lamx, h.lamy, Abg, Atg, h.nxh, h.spitch, h.ny,
                                                                   k0[s], nzl[s]);
       CU(cudaStreamSynchronize(B.stream));
@@ -316,18 +324,16 @@ struct SlabsT {
       const int ntile = (ncol + kSlabCols - 1) / kSlabCols;
       if (tiled)
         k_slab_tri_fmap_tile<T, kSlabCols><<<ntile, Tile::THREADS, smem_tile, B.stream>>>(
-            B.ddom, tri[s].iv, tri[s].fmaps + 3LL * ncol * s, tri[s].zcol, k0[s], nzg, coef_alpha2, use_dt);
+            B.ddom, tri[s].iv, tri[s].fmaps + 3LL * ncol * s);
       else
-        k_slab_tri_fmap<T><<<(2 * ncol + 127) / 128, 128, 0, B.stream>>>(B.ddom, tri[s].iv, tri[s].fmaps + 3LL * ncol * s,
-                                                                         tri[s].zcol, k0[s], nzg, coef_alpha2, use_dt);
+        k_slab_tri_fmap<T><<<(2 * ncol + 127) / 128, 128, 0, B.stream>>>(B.ddom, tri[s].iv, tri[s].fmaps + 3LL * ncol * s);
       B.nlaunch++;
       for (int t = 0; t < ns; t++) {
         if (t == s) continue;
         if (t > s) cps.push_back(Copy{s, t, tri[t].fmaps + 3LL * ncol * s, tri[s].fmaps + 3LL * ncol * s,
                                       sizeof(double) * 3 * ncol});
-        for (int part = 0; part < 2; part++)
-          cps.push_back(Copy{s, t, tri[t].zcol + (size_t)part * nzg + k0[s], tri[s].zcol + (size_t)part * nzg + k0[s],
-                             sizeof(double) * nzl[s]});
+        const size_t z0 = (size_t)k0[s] * zparts;
+        cps.push_back(Copy{s, t, tri[t].zpart + z0, tri[s].zpart + z0, sizeof(double) * nzl[s] * zparts});
       }
     });
     if ((r = exchange(cps))) return r;
@@ -335,15 +341,15 @@ struct SlabsT {
     each([&](int s, BatchT<T> &B) {
       const int ncol = B.hdom[0].ny * B.hdom[0].spitch;
       const int ntile = (ncol + kSlabCols - 1) / kSlabCols;
+      k_slab_zero<T><<<1, kZeroThreads, 0, B.stream>>>(B.ddom, tri[s].zpart, zparts, tri[s].wsum, tri[s].zsol, tri[s].dzf,
+                                                      nzg, gcfg.Btype[ELMM_BO], gcfg.Btype[ELMM_TO], coef_alpha2, use_dt);
       if (tiled)
         k_slab_tri_fwd_tile<T, kSlabCols><<<ntile, Tile::THREADS, smem_tile, B.stream>>>(
-            B.ddom, tri[s].iv, tri[s].fmaps, tri[s].bmaps + 3LL * ncol * s, tri[s].zcol, tri[s].dzc, tri[s].dzf, k0[s],
-            nzg, s);
+            B.ddom, tri[s].iv, tri[s].fmaps, tri[s].bmaps + 3LL * ncol * s, tri[s].zsol + k0[s], s);
       else
-        k_slab_tri_fwd<T><<<(2 * ncol + 127) / 128, 128, 0, B.stream>>>(B.ddom, tri[s].iv, tri[s].fmaps,
-                                                                        tri[s].bmaps + 3LL * ncol * s, tri[s].zcol,
-                                                                        tri[s].dzc, tri[s].dzf, k0[s], nzg, s);
-      B.nlaunch++;
+        k_slab_tri_fwd<T><<<(2 * ncol + 127) / 128, 128, 0, B.stream>>>(
+            B.ddom, tri[s].iv, tri[s].fmaps, tri[s].bmaps + 3LL * ncol * s, tri[s].zsol + k0[s], s);
+      B.nlaunch += 2;
       for (int t = 0; t < s; t++)
         cps.push_back(Copy{s, t, tri[t].bmaps + 3LL * ncol * s, tri[s].bmaps + 3LL * ncol * s, sizeof(double) * 3 * ncol});
     });
