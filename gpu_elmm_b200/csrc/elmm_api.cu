@@ -331,6 +331,16 @@ enum { LK_CELLS = 0, LK_BOX, LK_ROWS, LK_YCOLS, LK_TRI, LK_SHELL, LK_XREG, LK_YR
 // the momentum and SGS kernels
 constexpr int kChunks[3] = {8, MKC, kMaxChunk};
 
+// The stream of a step's chain, of the highest priority: it runs ahead of the
+// scalar stage beside it (BatchT::run_stage), in the serving loop as elsewhere,
+// and there no admission (a batch of its own) gets ahead of the running chunk.
+static int chain_stream(cudaStream_t *s) {
+  int least = 0, greatest = 0;
+  CU(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  CU(cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, greatest));
+  return ELMM_OK;
+}
+
 // blocks of the host-layout pack / unpack kernels (8 per SM)
 constexpr int kPackBlocks = 148 * 8;
 
@@ -662,10 +672,8 @@ struct BatchT {
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= device) return fail(ELMM_ERR_CUDA, "no CUDA device");
     CU(cudaSetDevice(device));
-    // a step's chain runs ahead of the scalar stage beside it (run_stage)
-    int least = 0, greatest = 0;
-    CU(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    CU(cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, greatest));
+    int sr = chain_stream(&stream);
+    if (sr) return sr;
     CU(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     CU(cudaEventCreateWithFlags(&ev_ready, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&ev_packed, cudaEventDisableTiming));
@@ -1207,8 +1215,9 @@ struct BatchT {
     // The forward x transform sums W2 where its tiles lie each in one level
     // and the domain is large enough to keep the chip busy: there k_wsum beside
     // it costs the bandwidth of one more read (a step of 192 x 192 x 96 mixed 0.769 ->
-    // 0.728 ms, 256 x 256 x 128 1.569 -> 1.514).  On a smaller one k_wsum runs in idle SMs, and sums that end with the transform
-    // are a longer chain (128 x 128 x 64 0.392 -> 0.42, 64 x 64 x 32 0.195 -> 0.201).
+    // 0.728 ms, 256 x 256 x 128 1.569 -> 1.514).  On a smaller one k_wsum runs in
+    // idle SMs, and sums that end with the transform are a longer chain
+    // (128 x 128 x 64 0.392 -> 0.42, 64 x 64 x 32 0.195 -> 0.201).
     {
       const int rows = 2 * (fft_reg_supported(h.nx) ? fft_reg_batch(h.nx) : fft_any_seqs<T>(h.nx));
       if (h.ny % rows == 0 && (long long)h.nx * h.ny * (zparent ? zparent->nz : h.nz) > kTileSumCells) {

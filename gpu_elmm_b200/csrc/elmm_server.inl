@@ -85,7 +85,8 @@ struct ServerT {
     }
     arena.reset(base, (size_t)sc.hbm_budget_bytes);
     tables.reset(base + Arena::round((size_t)sc.hbm_budget_bytes), kTableBytes - Arena::kAlign);
-    CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    int r = chain_stream(&stream);
+    if (r) return r;
     CU(cudaEventCreate(&c0));
     CU(cudaEventCreate(&c1));
     st.budget_bytes = sc.hbm_budget_bytes;

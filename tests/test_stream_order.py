@@ -36,3 +36,15 @@ def test_no_fill_or_upload_on_the_default_stream():
                 if commas + 1 != nargs:
                     found.append((f, a))
     assert not found, found
+
+
+def test_every_chain_runs_at_the_highest_priority():
+    """The streams that steps run on (a batch's and the serving loop's) come
+    from chain_stream, which takes the highest priority."""
+    found = {}
+    for f in sorted(os.listdir(CSRC)):
+        text = open(os.path.join(CSRC, f)).read()
+        for name in ("cudaStreamCreate", "cudaStreamCreateWithFlags", "cudaStreamCreateWithPriority", "chain_stream"):
+            for a in _calls(text, name):
+                found.setdefault(a.split(",")[0].strip(), []).append((f, name))
+    assert found["&stream"] == [("elmm_api.cu", "chain_stream"), ("elmm_server.inl", "chain_stream")], found
