@@ -1763,7 +1763,7 @@ struct BatchT {
       for (int v = 0; v < 2 && !r; v++) {
         tune_cols = v ? 32 : 16;
         if ((r = rebuild_ls(LK_TRIT))) break;
-        tune_ms[2 + v] = time10([&] { launch_tri(0, 0); });
+        tune_ms[2 + v] = time10([&] { launch_tri(0, 1); });  // the (0,0) mode given, as in a step
       }
       tune_cols = tune_ms[3] < tune_ms[2] ? 32 : 16;
       if (!r) r = rebuild_ls(LK_TRIT);

@@ -7,9 +7,13 @@ planes) and keeps the fastest.  Each shape only changes how the work is
 partitioned, so forcing any candidate (elmm_batch_set_tuning) must give the
 autotuned run's state bit for bit, on the FP64 and the mixed path, for a
 batch with a temperature, a passive scalar and uneven domain sizes."""
+import os
+import re
+
 import numpy as np
 import pytest
 
+from conftest import ROOT
 from gpu_elmm_b200.config import grid_of, make_config
 from gpu_elmm_b200.workloads import log_profile_state, puff_state, temperature_state
 
@@ -69,3 +73,12 @@ def test_out_of_set_shapes_are_refused():
             b.set_tuning(**bad)
         assert e.value.code == 6
     b.close()
+
+
+def test_the_z_solve_is_timed_as_steps_run_it():
+    """The autotuner's launches of the z solve take the (0,0) mode as given,
+    like those of a step: solved in the kernel instead, its serial sum over the
+    levels is the longest part of a small grid's time and hides the shape's."""
+    text = open(os.path.join(ROOT, "gpu_elmm_b200", "csrc", "elmm_api.cu")).read()
+    body = text[text.index("  int autotune() {"):text.index("  int set_tuning(")]
+    assert re.findall(r"launch_tri\(([^)]*)\)", body) == ["0, 1"]
