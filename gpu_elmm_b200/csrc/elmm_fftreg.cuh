@@ -136,9 +136,9 @@ struct FPlan {
   static constexpr int P = fplan_P(N);
   static constexpr int E = N / P;
   static constexpr int YS = P + 1;         // row stride of the pass-1 exchange
-  static constexpr int SEQ = N + E + 1;    // shared-memory elements per sequence (odd)
+  static constexpr int SEQ = (N + E + 1) | 1;  // shared-memory elements per sequence, odd: no bank conflicts across sequences
   static constexpr int RR = (E + P - 1) / P;
-  static_assert(P >= 2 && E >= P, "plan");
+  static_assert(P >= 2 && E >= P && SEQ % 2 == 1, "plan");
 };
 
 // Lengths with a register FFT: the multiples of 16 from 32 to 512 that factor
@@ -154,7 +154,7 @@ __host__ __device__ constexpr bool fft_reg_supported(int n) {
 #undef ELMM_FFT_CASE
 }
 
-__host__ __device__ constexpr int fft_reg_seq(int n) { return n + n / fplan_P(n) + 1; }
+__host__ __device__ constexpr int fft_reg_seq(int n) { return (n + n / fplan_P(n) + 1) | 1; }
 
 // Length-N DFT of the sequence whose lane t in [0, P) holds v[e] = x[t + P e].
 // On return the DFT X[0..N-1] is in sh[0..N-1] (natural order).  tw is the
