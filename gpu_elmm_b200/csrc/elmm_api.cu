@@ -741,7 +741,7 @@ struct BatchT {
     smem_x = smem_y = 0;
     for (size_t d = 0; d < hdom.size(); d++) {
       if (!fft_reg_supported(hdom[d].nx)) smem_x = std::max(smem_x, fft_any_smem_x<T>(hdom[d].nx, hplan[d].nsx));
-      if (!fft_reg_supported(hdom[d].ny)) smem_y = std::max(smem_y, fft_any_smem_y<T>(hdom[d].ny));
+      if (!fft_reg_y<T>(hdom[d].ny)) smem_y = std::max(smem_y, fft_any_smem_y<T>(hdom[d].ny));
     }
     smem_tri = sizeof(double) * kTriThreads * maxnz * (anyzper ? 2 : 1);
     // the opt-in maximum, so that handles of different sizes never lower the
@@ -756,11 +756,11 @@ struct BatchT {
     CU(cudaFuncSetAttribute(k_sgs<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
     for (auto &h : hdom) {
       reg_x |= fft_reg_supported(h.nx);
-      reg_y |= fft_reg_supported(h.ny);
+      reg_y |= fft_reg_y<T>(h.ny);
       tri_tile |= tri_tiled(h);
       if (fft_reg_supported(h.nx))
         smem_xr = std::max(smem_xr, sizeof(T2) * fft_reg_batch(h.nx) * fft_reg_seq(h.nx));
-      if (fft_reg_supported(h.ny))
+      if (fft_reg_y<T>(h.ny))
         smem_yr = std::max(smem_yr, sizeof(T2) * fft_reg_batch(h.ny) * fft_reg_seq(h.ny));
       if (tri_tiled(h)) {
         smem_trit = std::max(smem_trit, tri_tile_smem<T, 16>(h.nz));
@@ -823,7 +823,8 @@ struct BatchT {
       std::vector<int> lens;
       for (auto &h : hdom) {
         const int n = ydir ? h.ny : h.nx;
-        if (fft_reg_supported(n) && std::find(lens.begin(), lens.end(), n) == lens.end()) lens.push_back(n);
+        if ((ydir ? fft_reg_y<T>(n) : fft_reg_supported(n)) && std::find(lens.begin(), lens.end(), n) == lens.end())
+          lens.push_back(n);
       }
       for (int n : lens) {
         RegSet r;
@@ -902,7 +903,7 @@ struct BatchT {
         const int rows = 2 * fft_any_seqs<T>(h.nx);
         return (h.ny * h.nz + rows - 1) / rows;
       }
-      case LK_YCOLS: return fft_reg_supported(h.ny) ? 0 : ((h.nxh + TyOf<T>::v - 1) / TyOf<T>::v) * h.nz;
+      case LK_YCOLS: return fft_reg_y<T>(h.ny) ? 0 : ((h.nxh + TyOf<T>::v - 1) / TyOf<T>::v) * h.nz;
       case LK_MOMT:
       case LK_SGST: return column_tiles(kind, h, MX, MY);
       case LK_WSUM: return h.wrows ? 0 : h.nz;
@@ -916,7 +917,7 @@ struct BatchT {
         return (h.ny * h.nz + rows - 1) / rows;
       }
       case LK_YREG: {
-        if (!fft_reg_supported(h.ny)) return 0;
+        if (!fft_reg_y<T>(h.ny)) return 0;
         const int C = fft_reg_batch(h.ny);
         return ((h.nxh + C - 1) / C) * h.nz;
       }

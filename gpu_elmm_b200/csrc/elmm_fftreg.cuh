@@ -141,9 +141,13 @@ struct FPlan {
   static_assert(P >= 2 && E >= P && SEQ % 2 == 1, "plan");
 };
 
-// Lengths with a register FFT: the multiples of 16 from 32 to 512 that factor
-// into 2, 3 and 5 (rows of whole 16-byte vectors, at most 32 elements per
-// thread); the generic transform handles the others.
+// Lengths with a register FFT in x: the multiples of 16 from 32 to 512 that
+// factor into 2, 3 and 5 (rows of whole 16-byte vectors, at most 32 elements
+// per thread); the generic transform (elmm_poisson_any.cuh) handles the others.
+// Register against generic form, N x N x nz of 5 M cells, us forward / inverse:
+// FP32 33.2 / 15.4 against 45.3 / 37.9 (256), 41.4 / 18.9 against 46.1 / 35.7
+// (480, the closest); FP64 60.5 / 27.1 against 95.7 / 66.0 (256), 92.6 / 35.3 against
+// 88.5 / 61.9 (480: forward slower, the sum faster, and at 144 alike).
 #define ELMM_FFT_SIZES(X)                                                                                      \
   X(32) X(48) X(64) X(80) X(96) X(128) X(144) X(160) X(192) X(240) X(256) X(288) X(320) X(384) X(400) X(432) \
       X(480) X(512)
@@ -152,6 +156,19 @@ __host__ __device__ constexpr bool fft_reg_supported(int n) {
 #define ELMM_FFT_CASE(n_) (n) == (n_) ||
   return ELMM_FFT_SIZES(ELMM_FFT_CASE) false;
 #undef ELMM_FFT_CASE
+}
+
+// Lengths with a register FFT in y: in FP32 all of these (register against
+// generic form, forward, grids as above: 16.8 us against 19.7 at 432, 18.9
+// against 21.4 at 512; only at 512 x 512 x 128, 86 against 80), in FP64 those whose
+// two passes hold few enough values in registers, E + P up to 36.  Beyond that
+// the FP64 kernels spill 200 to 480 bytes at one block an SM, and the generic
+// form is the faster one (160 30.2 against 39.4, 192 x 192 x 96 29.0 against 31.1, 320
+// 35.3 against 37.3; past the line 240 43.4 against 36.3, 384 x 384 x 96 96.0 against
+// 78.3, 432 41.4 against 33.3, 512 x 512 x 64 124 against 82).
+template <typename T>
+__host__ __device__ constexpr bool fft_reg_y(int n) {
+  return fft_reg_supported(n) && (sizeof(T) == 4 || n / fplan_P(n) + fplan_P(n) <= 36);
 }
 
 __host__ __device__ constexpr int fft_reg_seq(int n) { return (n + n / fplan_P(n) + 1) | 1; }

@@ -1,7 +1,8 @@
 // elmm_poisson_any.cuh -- the x and y transforms of the Poisson problem
 // (src/poisson.f90:76-210, the PoisFFT replacement) for every length that
 // factors into 2, 3 and 5 and has no register FFT of its own
-// (elmm_poisson_reg.cuh), and for elmm_poisson_solve_noalloc.
+// (fft_reg_supported and fft_reg_y, elmm_fftreg.cuh), and for
+// elmm_poisson_solve_noalloc.
 //
 // A length is split into few large radices (up to 16: two passes to 256,
 // three to 4096), each pass one decimation-in-frequency butterfly per thread
@@ -13,8 +14,8 @@
 // Bound by instructions and the latency of a tile's passes, not by memory:
 // 512 x 512 x 128, FP32, against radices 2 to 5 on strided sequences with two
 // buffers (the form before): y 0.637 -> 0.080 ms, x forward 0.868 -> 0.228,
-// x inverse 0.395 -> 0.213 (512 itself now has a register transform: 0.085,
-// 0.175 and 0.078); 135 x 135 x 75: y 20 -> 16 us, x 56 -> 24 and 26 -> 19.
+// x inverse 0.395 -> 0.213 (512 itself now has a register transform: 0.086,
+// 0.148 and 0.077); 135 x 135 x 75: y 20 -> 16 us, x 56 -> 24 and 26 -> 19.
 #pragma once
 
 #include "elmm_poisson_reg.cuh"

@@ -340,7 +340,7 @@ struct FFTRegKernels {
   int n;
   void (*fwd)(const Dom<T> *, Launch, double, int, int, int);
   void (*inv)(const Dom<T> *, Launch, int);
-  void (*yf)(const Dom<T> *, Launch, int);
+  void (*yf)(const Dom<T> *, Launch, int);  // null unless fft_reg_y
   void (*yi)(const Dom<T> *, Launch, int);
 };
 

@@ -59,3 +59,11 @@ def test_step_through_the_divergence(n, precision):
             assert rel(a, b) < 1e-11
         else:
             assert float(np.abs(a - b).max()) < P_MIXED_ABS
+
+
+# The form of the y transform at the ends of the FP64 rule (192, 288 and 320 in
+# registers, 240, 384 and 400 not), with an x length of each form beside it; 1e-12
+# as above
+@pytest.mark.parametrize("n", [(32, 192, 4), (36, 288, 4), (48, 320, 4), (32, 240, 5), (36, 384, 4), (45, 400, 4)])
+def test_fp64_y_forms(n):
+    test_poisson_of_every_pass_count(n, PREC_FP64, 1e-12)
