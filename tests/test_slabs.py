@@ -258,8 +258,8 @@ def test_slabs_carry_puffs_and_slices(precision):
 
 # The mixed path keeps the single domain's state bit for bit: the (0,0) mode
 # comes from one sum per level, whichever slab holds the level (k_wsum for
-# domains up to 1.3 M cells and rows that do not fill whole x tiles, the tiles'
-# sums beyond, register and generic transforms), solved in one order; the other
+# small domains and rows that do not fill whole x tiles, the tiles' sums
+# beyond, register and generic transforms), solved in one order; the other
 # modes' FP64 sweeps differ in grouping alone, far below FP32.
 @pytest.mark.parametrize("n, nz", [((48, 32, 24), (6, 10, 8)), ((256, 64, 96), (48, 48)), ((256, 64, 96), (30, 40, 26)),
                                    ((144, 96, 110), (60, 50)), ((300, 128, 40), (13, 27))],
