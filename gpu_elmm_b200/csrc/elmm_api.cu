@@ -61,7 +61,7 @@ static bool factorize(int n, FFTFactors &f) {
   static const int radix[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
   f.n = n;
   f.nfac = 0;
-  int cur[kMaxFac], best = kMaxFac + 1;
+  int cur[kMaxFac] = {}, best = kMaxFac + 1;
   std::function<void(int, int, size_t)> search = [&](int r, int depth, size_t from) {
     if (r == 1 && depth > 0 && (depth < best || (depth == best && cur[0] < f.fac[0]))) {
       best = depth;
@@ -324,7 +324,7 @@ struct LaunchSet {
   Launch l() const { return Launch{starts, nd, total, kc}; }
 };
 
-enum { LK_CELLS = 0, LK_BOX, LK_ROWS, LK_YCOLS, LK_TRI, LK_SHELL, LK_XREG, LK_YREG, LK_TRIT, LK_TCOL, LK_DCOL,
+enum { LK_CELLS = 0, LK_ROWS, LK_YCOLS, LK_TRI, LK_SHELL, LK_XREG, LK_YREG, LK_TRIT, LK_TCOL, LK_DCOL,
        LK_AVG, LK_COMMIT, LK_TPAIR, LK_PROJ, LK_PROJ2, LK_DCOL2, LK_MOMT, LK_SGST, LK_WM, LK_WSUM, LK_N };
 
 // the z-chunk lengths (planes of a tile's column) the autotuner tries for
@@ -897,7 +897,6 @@ struct BatchT {
     int ntx = (h.nx + TX - 1) / TX, nty = (h.ny + TY - 1) / TY;
     switch (kind) {
       case LK_CELLS: return ntx * nty * h.nz;
-      case LK_BOX: return ((h.nx + 2 + TX - 1) / TX) * ((h.ny + 2 + TY - 1) / TY) * (h.nz + 2);
       case LK_ROWS: {
         if (fft_reg_supported(h.nx)) return 0;
         const int rows = 2 * fft_any_seqs<T>(h.nx);
@@ -2336,7 +2335,7 @@ struct BatchT {
     CU(cudaSetDevice(device));
     if (frame_pending) CU(cudaStreamWaitEvent(stream, ev_packed, 0));
     CU(cudaEventRecord(t0, stream));
-    // the fused divergence of k_fftx_fwd reads U2: make U2 the current field
+    // the fused divergence of the forward x transform reads U2: make U2 the current field
     for (int d = 0; d < nd; d++) {
       size_t box = (size_t)hdom[d].plane * (hdom[d].nz + 2) * sizeof(T);
       CU(cudaMemcpyAsync(hdom[d].U2, hdom[d].U, box, cudaMemcpyDeviceToDevice, stream));

@@ -9,8 +9,8 @@
 //   pass 2: P-point DFTs over n1 for each k2, in ceil(E / P) rounds.
 // The in-register DFTs are built recursively from radix 2, 3, 4 and 5 with
 // compile-time twiddles; only W_N^(n1 k2) comes from the per-length table.
-// The result is the unnormalised DFT, as the generic shared-memory FFT of
-// elmm_fft.cuh computes it.
+// The result is the unnormalised DFT, as the generic transforms of
+// elmm_poisson_any.cuh compute it.
 #pragma once
 
 #include <type_traits>

@@ -8,20 +8,23 @@
 // number of resident blocks and each block strides over the tiles.
 //
 // Per stage:
-//   k_sgs       SubgridStresses: Smagorinsky viscosity (+ ghosts),
-//               wall-model fluxes (dynamics.f90:869-908)
+//   k_sgs       SubgridStresses: Smagorinsky viscosity (dynamics.f90:869-908);
+//               beside it k_wm_points, the wall-model fluxes
 //   k_momentum  Convection + OtherTerms: CDS2 advection, diffusion with the
 //               wall-flux corrections, RK combine, old-pressure gradient,
-//               U2 += U; writes U2 with its ghosts (dynamics.f90:230-499,
-//               tsteps.f90:263-358)
-//   k_fftx_fwd  divergence RHS (pressure.f90:688-717) fused with the real
-//               FFT along x
-//   k_ffty      complex FFT along y (forward, then inverse)
-//   k_tri       tridiagonal solve in z per wavenumber pair
-//   k_fftx_inv  inverse real FFT along x -> Phi with its ghosts
+//               U2 += U (dynamics.f90:230-499, tsteps.f90:263-358)
+//   k_fftx_fwd_reg, _any   divergence RHS (pressure.f90:688-717) fused with
+//               the real FFT along x (elmm_poisson_reg.cuh for the lengths
+//               with a register FFT, elmm_poisson_any.cuh for the others)
+//   k_wsum, k_zero_mode   the (0,0) mode, beside the transforms
+//   k_ffty_reg, _any   complex FFT along y (forward, then inverse)
+//   k_tri_tile, k_tri  tridiagonal solve in z per wavenumber pair (tiled, or
+//               for tall columns and periodic z)
+//   k_fftx_inv_reg, _any   inverse real FFT along x -> Phi
 //   k_project   PostPoisson (pressure.f90:728-991): U = U2 - coef grad Phi,
 //               Pr += Phi, top-layer partial sums for FixPressureToReference
-//   k_prref     the pressure reference (pressure.f90:1160-1220)
+//   k_ghosts    ghost shells of the fields written; after the projection
+//               also the pressure reference (pressure.f90:1160-1220)
 #pragma once
 
 #include "elmm_common.cuh"
@@ -500,8 +503,8 @@ __global__ void __launch_bounds__(kWsumThreads, 2) k_wsum(const Dom<T> *__restri
 
 // Tridiagonal solve in z for each (kx, ky): the Thomas algorithm in FP64 on
 // the rows of Residue_variable_z (poisson.f90:23-60), Neumann rows at the
-// ends or a cyclic system for periodic z; the (0,0) mode is singular: k_wsum has
-// its solution (zsol), or, for a right-hand side that is not a divergence, it
+// ends or a cyclic system for periodic z; the (0,0) mode is singular: its
+// solution is given (zsol), or, for a right-hand side that is not a divergence, it
 // is solved by two prefix sums with its mean pinned to zero.
 constexpr int kTriThreads = 64;
 
@@ -524,7 +527,7 @@ __global__ void __launch_bounds__(kTriThreads) k_tri(const Dom<T> *__restrict__ 
     const double lam = d.lamx[kx] + d.lamy[ky];
     const double *Ab = d.Ab, *At = d.At;
     if (kx == 0 && ky == 0) {
-      if (zsol) {  // solved by k_wsum
+      if (zsol) {  // solved beside the transforms
 #pragma unroll 4
         for (int k = 1; k <= nz; k++) {
           T2 o; o.x = (T)d.zsol[k]; o.y = (T)0;

@@ -38,7 +38,7 @@ struct MomCtx {
   int wallmask;  // bit s: wall-model fluxes on side s
   int vz;
   int ext[3][3];
-  const double *dzPr, *dzW, *zPr, *zW;
+  const double *dzPr, *dzW;
   const T *fluxp[kFaces], *fluxm[kFaces];
   const unsigned char *bskip[3];
 };
@@ -61,7 +61,7 @@ __device__ __forceinline__ void fill_ctx(MomCtx<T> &m, const Dom<T> &d) {
     m.wallmask = wm;
     m.vz = d.vz;
   } else if (t == 13) {
-    m.dzPr = d.dzPr; m.dzW = d.dzW; m.zPr = d.zPr; m.zW = d.zW;
+    m.dzPr = d.dzPr; m.dzW = d.dzW;
   } else if (t >= 32 && t < 32 + kFaces) {
     m.fluxp[t - 32] = d.wm_fluxp[t - 32];
     m.fluxm[t - 32] = d.wm_fluxm[t - 32];

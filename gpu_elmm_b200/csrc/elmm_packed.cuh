@@ -17,7 +17,6 @@ __device__ __forceinline__ F2 operator+(F2 a, F2 b) { return F2{__fadd2_rn(a.v, 
 __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return F2{__fmul2_rn(a.v, b.v)}; }
 // a - b: the product b * (-1) is exact, so this is one rounding of a - b
 __device__ __forceinline__ F2 operator-(F2 a, F2 b) { return F2{__ffma2_rn(b.v, make_float2(-1.f, -1.f), a.v)}; }
-__device__ __forceinline__ F2 neg2(F2 a) { return F2{__fmul2_rn(a.v, make_float2(-1.f, -1.f))}; }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return F2{__ffma2_rn(a.v, b.v, c.v)}; }
 
 // Pair accessor over the momentum plane ring: the thread's two cells sit at

@@ -1,9 +1,9 @@
 // elmm_poisson_reg.cuh -- the transforms and the z solve of the Poisson
 // problem (src/poisson.f90:23-60, the PoisFFT replacement) for the common
-// case: x and y lengths with a register FFT (ELMM_FFT_SIZES) and a
-// non-periodic z axis of at most kTriTileMaxNz cells.  Other grids use the
-// generic kernels of elmm_kernels.cuh / elmm_kernels2.cuh; both compute the
-// same discrete solution.
+// case: x and y lengths with a register FFT (fft_reg_supported, fft_reg_y) and
+// a non-periodic z axis of at most kTriTileMaxNz cells.  Other lengths take
+// the transforms of elmm_poisson_any.cuh, other z axes k_tri
+// (elmm_kernels.cuh); both compute the same discrete solution.
 #pragma once
 
 #include "elmm_fftreg.cuh"
@@ -14,15 +14,16 @@ namespace elmm {
 constexpr int kRegThreads = 256;
 // resident blocks per SM the x-transform kernels are compiled for: for up to
 // 16 elements per thread three (FP32, 80 registers) or two (FP64, 128
-// registers) fit without spills; longer FP32 sequences (up to 32 elements)
-// two blocks of 128 registers, faster than one block of ~200 (the y
-// transform of those lengths spills at 128 and keeps the compiler's choice)
+// registers), with no spills or a few (12 bytes for FP32 256 and FP64 80);
+// longer FP32 sequences (up to 32 elements) two blocks of 128 registers with
+// up to 28 bytes, faster than one block of ~200 (the y transform of those
+// lengths spills more at 128 and keeps the compiler's choice)
 template <typename T, int N>
 constexpr int fft_reg_min_blocks() { return N / fplan_P(N) <= 16 ? (sizeof(T) == 4 ? 3 : 2) : (sizeof(T) == 4 ? 2 : 1); }
 // the forward x transform (with the fused divergence) of FP32 lengths up to
 // 16 elements per thread: four resident blocks (64 registers) measured
-// faster than three (0.050 -> 0.043 ms at 256 x 256 x 128); the inverse
-// keeps three
+// faster than three (0.050 -> 0.043 ms at 256 x 256 x 128) in spite of their
+// spills (16 bytes at 256 and 128, 72 at 96 and 80); the inverse keeps three
 template <typename T, int N>
 constexpr int fft_reg_min_blocks_fwd() { return N / fplan_P(N) <= 16 && sizeof(T) == 4 ? 4 : fft_reg_min_blocks<T, N>(); }
 
@@ -109,8 +110,7 @@ template <> struct Row16<double> {
 // sequence), split into the half spectra of the two rows: S[row][0..nx/2].
 // The divergence is formed from 16-byte row vectors (a thread takes one
 // chunk of both rows of a sequence) into shared memory, from where each FFT
-// thread picks its strided elements; the arithmetic per cell is that of
-// poisson_rhs.
+// thread picks its strided elements.
 template <typename T, int N>
 __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename Vec2<T>::type *smem, double coef,
                                               int rhs_from_phi) {
@@ -368,8 +368,8 @@ __host__ __device__ constexpr int fft_reg_batch(int n) { return kRegThreads / fp
 // segment of k, the segment maps are chained through shared memory, and each
 // thread then replays its segment from the exact entry value.  The tile of S
 // is copied into shared memory with cp.async (while the pivots are rebuilt)
-// and written back at the end.  The (0,0) mode is k_wsum's solution (zsol) or
-// the zero-mean prefix sums of the generic kernel, k_tri.
+// and written back at the end.  The (0,0) mode is given (zsol) or solved
+// by the zero-mean prefix sums of the generic kernel, k_tri.
 #ifndef ELMM_TRI_COLS
 #define ELMM_TRI_COLS 16
 #endif
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(tri_tile_threads<COLS>()) k_tri_tile(const Dom
         x[(k - 1) * XS] = (T)xv;
       }
     }
-    if (active && zero_mode && zsol) {  // solved by k_wsum
+    if (active && zero_mode && zsol) {  // solved beside the transforms
       for (int k = kb; k <= ke; k++) x[(k - 1) * XS] = sys & 1 ? (T)0 : (T)d.zsol[k];
     } else if (active && zero_mode && seg == 0) {
       // F(k) = F(k-1) + dzc(k) r(k) is the flux (x(k+1) - x(k)) / dzf(k)
