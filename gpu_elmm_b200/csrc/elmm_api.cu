@@ -1216,13 +1216,15 @@ struct BatchT {
     // and W2 is large: there k_wsum beside it costs the bandwidth of one more
     // read, on a smaller domain it runs in idle SMs and sums that end with
     // the transform are a longer chain.  A step with k_wsum and with the
-    // tiles' sums, ms, FP32: 64 x 64 x 32 0.1945 and 0.1968, 128 x 128 x 48 (3.1 MB) 0.2720
-    // and 0.2727, 128 x 128 x 64 (4.2 MB) 0.3025 and 0.2958, 256 x 128 x 64 0.437 and 0.422,
-    // 192 x 192 x 48 0.440 and 0.417, 256 x 256 x 64 0.717 and 0.694; FP64: 64 x 64 x 16 0.213 and
-    // 0.221, 64 x 64 x 64 (2.1 MB) 0.2377 and 0.2358, 128 x 128 x 32 (4.2 MB) 0.310 and 0.293,
-    // 128 x 128 x 64 0.431 and 0.420, 256 x 256 x 64 1.263 and 1.259.  By the domain alone,
-    // although a batch of small domains would gain too (16 of 64 x 64 x 32 0.616 ->
-    // 0.590 ms): a domain gives the same bits alone, in a batch and in slabs.
+    // tiles' sums, ms, FP32: 64 x 64 x 32 0.1945 and 0.1968, 128 x 128 x 48 (3.1 MB)
+    // 0.2720 and 0.2727, 128 x 128 x 64 (4.2 MB) 0.3025 and 0.2958, but with a scalar
+    // beside the solve 16.73 and 16.98 (a pass of 40 steps), 192 x 192 x 36 (5.3 MB)
+    // 0.384 and 0.382, 192 x 192 x 48 0.440 and 0.417, 256 x 256 x 64 0.717 and 0.694; FP64:
+    // 64 x 64 x 16 0.213 and 0.221, 64 x 64 x 64 (2.1 MB) 0.2377 and 0.2358, 128 x 128 x 48
+    // (6.3 MB) 0.378 and 0.370, 128 x 128 x 64 0.431 and 0.420, with a scalar 0.556 and
+    // 0.546, 256 x 256 x 64 1.263 and 1.259.  By the domain alone, although a batch of small
+    // domains would gain too (16 of 64 x 64 x 32 0.616 -> 0.590 ms): a domain gives
+    // the same bits alone, in a batch and in slabs.
     {
       const int rows = 2 * (fft_reg_supported(h.nx) ? fft_reg_batch(h.nx) : fft_any_seqs<T>(h.nx));
       if (h.ny % rows == 0 && (long long)h.nx * h.ny * (zparent ? zparent->nz : h.nz) * (long long)sizeof(T) > kTileSumBytes) {

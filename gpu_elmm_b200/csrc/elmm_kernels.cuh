@@ -428,7 +428,7 @@ __device__ __forceinline__ void zero_mode(const Dom<T> &d, double coef, double *
 
 // the domains whose level sums the forward x transform left per tile: a block
 // a domain
-constexpr long long kTileSumBytes = 7 << 19;  // domains whose W2 is larger leave their sums per tile
+constexpr long long kTileSumBytes = 5 << 20;  // domains whose W2 is larger leave their sums per tile
 template <typename T>
 __global__ void __launch_bounds__(kZeroThreads) k_zero_mode(const Dom<T> *__restrict__ doms, int nd, double coef_alpha2,
                                                             int use_dt) {

@@ -10,7 +10,11 @@ Per (kx, ky) column the Thomas sweeps are affine recurrences,
     y(k) = r(k) iv(k) - Ab(k) iv(k) y(k-1),   x(k) = y(k) - At(k) iv(k) x(k+1),
 so a slab maps its entry value to its exit value with two numbers per
 column (A, B), and the slabs exchange only those maps.  The (0,0) column is
-gathered whole and solved by every slab with the zero-mean prefix sums.
+gathered whole and solved by every slab with the zero-mean prefix sums.  (The
+library, whose right-hand side is a divergence, gathers the sums of W over the
+levels in its place: they are the fluxes F below, k_slab_zero.  The prefix sums
+from the fluxes on are the same, and the GPU tests compare them with the
+single domain bit for bit.)
 """
 import numpy as np
 
