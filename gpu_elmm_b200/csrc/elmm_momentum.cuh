@@ -5,7 +5,7 @@
 // includes), the RK combine (dynamics.f90:266-354, :450-478), the
 // old-pressure gradient (dynamics.f90:58-199) and U2 += U (tsteps.f90:352-354).
 //
-// A block owns an MX x MY column of cells and marches up a chunk of MKC
+// A block owns an MX x MY column of cells and marches up a chunk of L.kc
 // planes.  U, V, W, Viscosity and Pr of each plane (with a one-cell halo in
 // x and y) and the old Ustar (tile only) arrive by tensor-map TMA in a ring
 // of kRingSlots plane slots in shared memory, requested several planes ahead
