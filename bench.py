@@ -11,9 +11,9 @@ with a full pressure projection) of that domain, inputs resident in HBM.
 
 Under torchrun every rank steps its own independent domain (weak scaling,
 no collective on the data path); the value is the total over ranks divided
-by the slowest rank's time.  `--impl reference` times the CPU restatement of
-the reference (the oracle, C++ FP64 with OpenMP on all host threads), since
-the Fortran reference itself cannot be built here.
+by the slowest rank's time.  `--impl reference` says that the reference is
+unavailable: it is Fortran and cannot be built here, and no restatement of it
+stands in for its own code (the oracle's time is `cpu_baseline`, kind "port").
 """
 from __future__ import annotations
 
@@ -48,8 +48,6 @@ DATA = ("synthetic: seeded log profile u*=0.3 + U(-0.1,0.1) perturbations on u,v
 MOMENTUM_WORDS = 15
 # timed oracle steps of the main line's cpu_baseline (a bounded sample: ~10 s on 16 cores)
 CPU_STEPS = 5
-# seconds of timed oracle steps in the reference arm (--impl reference)
-REF_BUDGET_S = 120.0
 # long run of the single domain on both paths (errors after 1, 10 and this many steps)
 LONG_STEPS = 1000
 # the array of cubes: steps run on both paths (device time over steps 10..CUBES_STEPS)
@@ -208,34 +206,13 @@ def cpu_baseline(steps=CPU_STEPS):
             "seconds": dt}
 
 
-def run_reference(args, ws, rank):
-    """The CPU restatement of the reference on this host's cores (the Fortran
-    reference cannot be built here): W untimed RK3 steps of the full
-    256x256x128 domain, then K timed ones, on rank 0 only.  A full step takes
-    about 2 s on 16 cores, so the timed steps stop at REF_BUDGET_S seconds
-    (estimated from the warm-up steps); the line reports the steps it timed
-    ("steps") beside the ones asked for ("steps_requested")."""
-    if rank != 0:
-        return 0
-    o, g, threads = _native_oracle()
-    t0 = time.perf_counter()
-    o.step(max(1, args.warmup))
-    per_step = (time.perf_counter() - t0) / max(1, args.warmup)
-    steps = max(1, min(args.steps, int(REF_BUDGET_S / per_step)))
-    t0 = time.perf_counter()
-    o.step(steps)
-    dt = time.perf_counter() - t0
-    v = g.cells() * steps / dt
-    line = {"impl": "reference", "metric": METRIC, "value": v, "unit": "cell-steps/s", "n_gpus": args.gpus,
-            "steps": steps, "steps_requested": args.steps, "warmup": args.warmup, "ms_per_step": dt / steps * 1e3,
-            "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
-            "data": DATA, "config": {"workload": WORKLOAD, "cells": g.cells(), "precision": "fp64"},
-            "cpu_baseline": {"value": v, "unit": "cell-steps/s", "cores": threads, "kind": "port",
-                             "sample": f"{steps} RK3 steps of the 256x256x128 workload after {args.warmup} "
-                                       f"untimed steps (the Fortran reference cannot be built here; its C++ FP64 "
-                                       f"restatement in oracle/, built -O3 -march=native -fopenmp, is timed)"},
-            "e2e": {"value": v, "unit": "cell-steps/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
-    print(json.dumps(line), flush=True)
+REFERENCE_UNAVAILABLE = ("the reference is Fortran 2008 on the PoisFFT library, which its sources do not contain; "
+                         "there is no Fortran compiler, scons or FFTW here to build either")
+
+
+def run_reference(rank):
+    if rank == 0:
+        print(json.dumps({"impl": "reference", "unavailable": REFERENCE_UNAVAILABLE}), flush=True)
     return 0
 
 
@@ -670,7 +647,7 @@ def main():
     ws, rank, local = dist_setup()
     try:
         if args.impl == "reference":
-            rc = run_reference(args, ws, rank)
+            rc = run_reference(rank)
         else:
             rc = run_ours(args, ws, rank, local)
     finally:
