@@ -893,14 +893,17 @@ struct BatchT {
   int column_tiles(int kind, const Dom<T> &h, int bx, int by) const {
     return ((h.nx + bx - 1) / bx) * ((h.ny + by - 1) / by) * ((h.nz + ls[kind].kc - 1) / ls[kind].kc);
   }
+  // x tiles of a domain (x_rows)
+  static int x_tiles(const Dom<T> &h, int rows) {
+    return h.wrows ? h.nz * h.wtiles() : (h.ny * h.nz + rows - 1) / rows;
+  }
   int tiles(int kind, const Dom<T> &h) const {
     int ntx = (h.nx + TX - 1) / TX, nty = (h.ny + TY - 1) / TY;
     switch (kind) {
       case LK_CELLS: return ntx * nty * h.nz;
       case LK_ROWS: {
         if (fft_reg_supported(h.nx)) return 0;
-        const int rows = 2 * fft_any_seqs<T>(h.nx);
-        return (h.ny * h.nz + rows - 1) / rows;
+        return x_tiles(h, 2 * fft_any_seqs<T>(h.nx));
       }
       case LK_YCOLS: return fft_reg_y<T>(h.ny) ? 0 : ((h.nxh + TyOf<T>::v - 1) / TyOf<T>::v) * h.nz;
       case LK_MOMT:
@@ -912,8 +915,7 @@ struct BatchT {
       case LK_SHELL: return (int)((shell_cells(h.nx, h.ny, h.nz) + kShellThreads * shell_per - 1) / (kShellThreads * shell_per));
       case LK_XREG: {
         if (!fft_reg_supported(h.nx)) return 0;
-        const int rows = 2 * fft_reg_batch(h.nx);
-        return (h.ny * h.nz + rows - 1) / rows;
+        return x_tiles(h, 2 * fft_reg_batch(h.nx));
       }
       case LK_YREG: {
         if (!fft_reg_y<T>(h.ny)) return 0;
@@ -1212,8 +1214,8 @@ struct BatchT {
     if (!slab_mode && (r = dalloc((void **)&h.wsum, sizeof(double) * (h.nz + 2)))) return r;
     if (!slab_mode && (r = dalloc((void **)&h.zsol, sizeof(double) * (h.nz + 2)))) return r;
     if ((r = dalloc((void **)&h.wticket, sizeof(int)))) return r;
-    // The forward x transform sums W2 where its tiles lie each in one level
-    // and W2 is large: there k_wsum beside it costs the bandwidth of one more
+    // The forward x transform sums W2 where its tiles can start anew at each
+    // level and W2 is large: there k_wsum beside it costs the bandwidth of one more
     // read, on a smaller domain it runs in idle SMs and sums that end with
     // the transform are a longer chain.  A step with k_wsum and with the
     // tiles' sums, ms, FP32: 64 x 64 x 32 0.1945 and 0.1968, 128 x 128 x 48 (3.1 MB)
@@ -1227,9 +1229,11 @@ struct BatchT {
     // the same bits alone, in a batch and in slabs.
     {
       const int rows = 2 * (fft_reg_supported(h.nx) ? fft_reg_batch(h.nx) : fft_any_seqs<T>(h.nx));
-      if (h.ny % rows == 0 && (long long)h.nx * h.ny * (zparent ? zparent->nz : h.nz) * (long long)sizeof(T) > kTileSumBytes) {
+      const long long w2 = (long long)h.nx * h.ny * (zparent ? zparent->nz : h.nz) * (long long)sizeof(T);
+      const int padded = (h.ny + rows - 1) / rows * rows;
+      if (w2 > kTileSumBytes && (padded - h.ny) * kTileSumPad <= h.ny) {
         h.wrows = rows;
-        if (!slab_mode && (r = dalloc((void **)&h.wpart, sizeof(double) * (h.ny / rows) * (size_t)h.nz))) return r;
+        if (!slab_mode && (r = dalloc((void **)&h.wpart, sizeof(double) * h.wtiles() * (size_t)h.nz))) return r;
       }
     }
     if ((r = dalloc((void **)&h.prm, sizeof(double)))) return r;

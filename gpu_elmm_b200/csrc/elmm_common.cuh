@@ -118,11 +118,13 @@ struct Dom {
   int zper;
   // sums of W2 over each level in FP64, index k, the solution of the (0,0)
   // mode from them, index 1..nz (null in a slab: k_slab_zero), and the count
-  // of the levels done (k_wsum); with wrows > 0 the forward x transform leaves
-  // the sums of its tiles of wrows rows (ny / wrows tiles a level) in wpart
-  // for k_zero_mode instead
+  // of the levels done (k_wsum); with wrows > 0 the x transforms' tiles of wrows
+  // rows start anew at each level (x_rows), and the forward one leaves their
+  // sums in wpart for k_zero_mode instead
   double *wpart;
   int wrows;
+  // tiles of a level then
+  ELMM_HD int wtiles() const { return (ny + wrows - 1) / wrows; }
   double *wsum, *zsol;
   int *wticket;
   // grid tables (FP64), index k + 2 for k in [-2, nz + 3]

@@ -428,7 +428,13 @@ __device__ __forceinline__ void zero_mode(const Dom<T> &d, double coef, double *
 
 // the domains whose level sums the forward x transform left per tile: a block
 // a domain
-constexpr long long kTileSumBytes = 5 << 20;  // domains whose W2 is larger leave their sums per tile
+// domains whose W2 is larger leave their sums per tile (init_domain), if tiles
+// that start anew at each level hold at most ny / kTileSumPad rows past its
+// end: a step with k_wsum and with such tiles, FP32, 300 x 270 x 50 (1 in 270) 0.901 and
+// 0.875 ms, 135 x 135 x 75 with the temperature (1 in 15) 0.6395 and 0.6343, 256 x 240 x 100
+// (1 in 15) 1.037 and 1.038
+constexpr long long kTileSumBytes = 5 << 20;
+constexpr int kTileSumPad = 14;
 template <typename T>
 __global__ void __launch_bounds__(kZeroThreads) k_zero_mode(const Dom<T> *__restrict__ doms, int nd, double coef_alpha2,
                                                             int use_dt) {
@@ -436,7 +442,7 @@ __global__ void __launch_bounds__(kZeroThreads) k_zero_mode(const Dom<T> *__rest
   for (int di = blockIdx.x; di < nd; di += gridDim.x) {
     const Dom<T> &d = doms[di];
     if (!d.wrows) continue;
-    sum_tiles(d.wpart, d.ny / d.wrows, d.nz, d.wsum);
+    sum_tiles(d.wpart, d.wtiles(), d.nz, d.wsum);
     zero_mode(d, use_dt ? coef_alpha2 * d.dt : coef_alpha2, red);
   }
 }

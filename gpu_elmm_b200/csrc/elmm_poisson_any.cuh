@@ -238,10 +238,10 @@ __device__ __forceinline__ void fftx_passes(const FFTFactors &f, int ns, typenam
 // divergence of PrePoisson (pressure.f90:688-717) from vectors of VE cells of
 // a row; and the tile's sum of W2
 template <typename T, int VE>
-__device__ __forceinline__ void fftx_stage(const Dom<T> &d, typename Vec2<T>::type *buf, const RhsRow<T> *rinfo, int r0,
+__device__ __forceinline__ void fftx_stage(const Dom<T> &d, typename Vec2<T>::type *buf, const RhsRow<T> *rinfo, XRows xr,
                                            int ns, double coef, int rhs_from_phi, TileSum &ls) {
   typedef typename Vec2<T>::type T2;
-  const int pitch = fft_any_pitch(ns), nch = d.nx / VE, ny = d.ny, nrows = ny * d.nz;
+  const int pitch = fft_any_pitch(ns), nch = d.nx / VE, ny = d.ny, r0 = xr.r0, nrows = xr.end;
   const T rdt2 = (T)(1.0 / coef);
   const T rdx = (T)(1.0 / d.dx), rdy = (T)(1.0 / d.dy), rdz = (T)(1.0 / d.dz);
   auto row = [](const T *p, T (&v)[VE]) {
@@ -320,8 +320,9 @@ __global__ void __launch_bounds__(kFFTThreadsX, sizeof(T) == 4 ? 6 : 4)
     const Dom<T> &d = doms[di];
     if (gate && !*d.refine_flag) continue;
     const PoisPlan &pl = plans[di];
-    const int N = d.nx, ny = d.ny, nrows = ny * d.nz, ns = pl.nsx, pitch = fft_any_pitch(ns);
-    const int r0 = 2 * (t - __ldg(L.starts + di)) * ns;
+    const int N = d.nx, ny = d.ny, ns = pl.nsx, pitch = fft_any_pitch(ns);
+    const XRows xr = x_rows(d, t - __ldg(L.starts + di), 2 * ns);
+    const int r0 = xr.r0, nrows = xr.end;
     const double coef = use_dt ? coef_alpha2 * d.dt : coef_alpha2;
     T2 *out = buf + N * pitch;
     if (!rhs_from_phi && threadIdx.x < 2 * ns) {
@@ -332,8 +333,8 @@ __global__ void __launch_bounds__(kFFTThreadsX, sizeof(T) == 4 ? 6 : 4)
     __syncthreads();
     const bool sums = d.wrows > 0 && !rhs_from_phi;
     TileSum ls{0};
-    if (N % Row16<T>::n == 0) fftx_stage<T, Row16<T>::n>(d, buf, rinfo, r0, ns, coef, rhs_from_phi, ls);
-    else fftx_stage<T, 1>(d, buf, rinfo, r0, ns, coef, rhs_from_phi, ls);
+    if (N % Row16<T>::n == 0) fftx_stage<T, Row16<T>::n>(d, buf, rinfo, xr, ns, coef, rhs_from_phi, ls);
+    else fftx_stage<T, 1>(d, buf, rinfo, xr, ns, coef, rhs_from_phi, ls);
     if (sums) ls.warp_sum(wred);
     __syncthreads();
     if (sums) TileSum::put<kFFTThreadsX / 32>(wred, d.wpart + (t - __ldg(L.starts + di)));
@@ -371,8 +372,9 @@ __global__ void __launch_bounds__(kFFTThreadsX, sizeof(T) == 4 ? 6 : 4)
     const Dom<T> &d = doms[di];
     if (gate && !*d.refine_flag) continue;
     const PoisPlan &pl = plans[di];
-    const int N = d.nx, ny = d.ny, nrows = ny * d.nz, ns = pl.nsx, pitch = fft_any_pitch(ns);
-    const int r0 = 2 * (t - __ldg(L.starts + di)) * ns, nxh = d.nxh, lane = threadIdx.x & 31;
+    const int N = d.nx, ny = d.ny, ns = pl.nsx, pitch = fft_any_pitch(ns);
+    const XRows xr = x_rows(d, t - __ldg(L.starts + di), 2 * ns);
+    const int r0 = xr.r0, nrows = xr.end, nxh = d.nxh, lane = threadIdx.x & 31;
     T2 *out = buf + N * pitch;
     // a warp takes 32 modes of a sequence, kLoads of them at a time
     constexpr int NW = kFFTThreadsX / 32, kLoads = 4;

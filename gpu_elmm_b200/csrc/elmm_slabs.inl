@@ -141,7 +141,7 @@ struct SlabsT {
       Tri &x = tri[s];
       const double *Abg, *Atg;
       if ((r = B.upload_table(&Abg, Ab)) || (r = B.upload_table(&Atg, At)) || (r = B.upload_table(&x.dzf, dzf))) return r;
-      zparts = h.wrows ? h.ny / h.wrows : 1;
+      zparts = h.wrows ? h.wtiles() : 1;
       if ((r = B.dalloc((void **)&x.iv, sizeof(double) * (size_t)nzl[s] * ncol)) ||
           (r = B.dalloc((void **)&x.fmaps, sizeof(double) * 3 * (size_t)ncol * n)) ||
           (r = B.dalloc((void **)&x.bmaps, sizeof(double) * 3 * (size_t)ncol * n)) ||

@@ -1,8 +1,8 @@
 """The (0,0) mode of the pressure from the level sums of W: rows of whole
 16-byte vectors and not, sums from W2 itself and from the forward x
-transform's tiles (W2 of more than 5.2 MB and rows that fill whole tiles, of the
-register and the generic form; and rows that do not), levels past the tiled z
-solve, walls and periodic z, against the oracle."""
+transform's tiles (W2 of more than 5.2 MB and rows that fill a level's tiles or
+nearly so, of the register and the generic form; and rows that do not), levels
+past the tiled z solve, walls and periodic z, against the oracle."""
 import numpy as np
 import pytest
 
@@ -31,7 +31,8 @@ BOTTOM, TOP, PERIODIC = (BC_NOSLIP, BC_FREESLIP), (BC_FREESLIP, BC_NOSLIP), (P, 
 @pytest.mark.parametrize("n,z", [((8, 6, 5), BOTTOM), ((8, 6, 5), PERIODIC), ((9, 5, 4), TOP), ((64, 72, 6), BOTTOM),
                                  ((20, 75, 5), PERIODIC), ((12, 10, 220), PERIODIC), ((12, 10, 300), BOTTOM),
                                  ((4, 4, 440), TOP), ((64, 72, 300), BOTTOM), ((81, 75, 220), PERIODIC),
-                                 ((75, 64, 280), TOP), ((64, 64, 176), BOTTOM), ((64, 128, 130), PERIODIC)])
+                                 ((75, 64, 280), TOP), ((64, 64, 176), BOTTOM), ((64, 128, 130), PERIODIC), ((256, 125, 45), BOTTOM),
+                                 ((75, 250, 80), TOP)])
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
 def test_step_follows_the_oracle(n, z, precision):
     btype = (P, P, P, P) + z

@@ -258,11 +258,12 @@ def test_slabs_carry_puffs_and_slices(precision):
 
 # The mixed path keeps the single domain's state bit for bit: the (0,0) mode
 # comes from one sum per level, whichever slab holds the level (k_wsum for
-# small domains and rows that do not fill whole x tiles, the tiles' sums
+# small domains and rows that leave x tiles half empty, the tiles' sums
 # beyond, register and generic transforms), solved in one order; the other
 # modes' FP64 sweeps differ in grouping alone, far below FP32.
 @pytest.mark.parametrize("n, nz", [((48, 32, 24), (6, 10, 8)), ((256, 64, 96), (48, 48)), ((256, 64, 96), (30, 40, 26)),
-                                   ((144, 96, 110), (60, 50)), ((300, 128, 40), (13, 27))],
+                                   ((144, 96, 110), (60, 50)), ((300, 128, 40), (13, 27)), ((256, 125, 45), (20, 25)),
+                                   ((300, 135, 36), (17, 19))],
                          ids=lambda v: "x".join(map(str, v)))
 @pytest.mark.parametrize("stretched", [False, True])
 def test_mixed_slabs_equal_the_single_domain(n, nz, stretched):
