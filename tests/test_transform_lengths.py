@@ -67,3 +67,12 @@ def test_step_through_the_divergence(n, precision):
 @pytest.mark.parametrize("n", [(32, 192, 4), (36, 288, 4), (48, 320, 4), (32, 240, 5), (36, 384, 4), (45, 400, 4)])
 def test_fp64_y_forms(n):
     test_poisson_of_every_pass_count(n, PREC_FP64, 1e-12)
+
+
+# A given right-hand side on domains whose x tiles start anew at each level
+# (W2 of more than 5.2 MB), with a last tile that is not full, of the register and
+# the generic form; bounds as above
+@pytest.mark.parametrize("precision, tol", [(PREC_FP64, 1e-12), (PREC_MIXED, 1e-5)])
+@pytest.mark.parametrize("n", [(256, 125, 45), (300, 270, 18)])
+def test_poisson_with_tiles_per_level(n, precision, tol):
+    test_poisson_of_every_pass_count(n, precision, tol)
