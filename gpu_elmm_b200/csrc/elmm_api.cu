@@ -1214,8 +1214,8 @@ struct BatchT {
     if (!slab_mode && (r = dalloc((void **)&h.wsum, sizeof(double) * (h.nz + 2)))) return r;
     if (!slab_mode && (r = dalloc((void **)&h.zsol, sizeof(double) * (h.nz + 2)))) return r;
     if ((r = dalloc((void **)&h.wticket, sizeof(int)))) return r;
-    // The forward x transform sums W2 where its tiles can start anew at each
-    // level and W2 is large: there k_wsum beside it costs the bandwidth of one more
+    // The forward x transform sums W2 where its tiles lie each in one level
+    // and W2 is large: there k_wsum beside it costs the bandwidth of one more
     // read, on a smaller domain it runs in idle SMs and sums that end with
     // the transform are a longer chain.  A step with k_wsum and with the
     // tiles' sums, ms, FP32: 64 x 64 x 32 0.1945 and 0.1968, 128 x 128 x 48 (3.1 MB)
@@ -1230,8 +1230,8 @@ struct BatchT {
     {
       const int rows = 2 * (fft_reg_supported(h.nx) ? fft_reg_batch(h.nx) : fft_any_seqs<T>(h.nx));
       const long long w2 = (long long)h.nx * h.ny * (zparent ? zparent->nz : h.nz) * (long long)sizeof(T);
-      const int padded = (h.ny + rows - 1) / rows * rows;
-      if (w2 > kTileSumBytes && (padded - h.ny) * kTileSumPad <= h.ny) {
+      const int pad = (rows - h.ny % rows) % rows;  // rows of a level's last tile past its end
+      if (w2 > kTileSumBytes && pad * kTileSumPad <= (fft_reg_supported(h.nx) ? 0 : h.ny)) {
         h.wrows = rows;
         if (!slab_mode && (r = dalloc((void **)&h.wpart, sizeof(double) * h.wtiles() * (size_t)h.nz))) return r;
       }

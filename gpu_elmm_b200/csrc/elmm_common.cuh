@@ -119,8 +119,8 @@ struct Dom {
   // sums of W2 over each level in FP64, index k, the solution of the (0,0)
   // mode from them, index 1..nz (null in a slab: k_slab_zero), and the count
   // of the levels done (k_wsum); with wrows > 0 the x transforms' tiles of wrows
-  // rows start anew at each level (x_rows), and the forward one leaves their
-  // sums in wpart for k_zero_mode instead
+  // rows lie each in one level, and the forward one leaves their sums in wpart
+  // for k_zero_mode instead
   double *wpart;
   int wrows;
   // tiles of a level then

@@ -428,11 +428,13 @@ __device__ __forceinline__ void zero_mode(const Dom<T> &d, double coef, double *
 
 // the domains whose level sums the forward x transform left per tile: a block
 // a domain
-// domains whose W2 is larger leave their sums per tile (init_domain), if tiles
-// that start anew at each level hold at most ny / kTileSumPad rows past its
-// end: a step with k_wsum and with such tiles, FP32, 300 x 270 x 50 (1 in 270) 0.901 and
-// 0.875 ms, 135 x 135 x 75 with the temperature (1 in 15) 0.6395 and 0.6343, 256 x 240 x 100
-// (1 in 15) 1.037 and 1.038
+// domains whose W2 is larger leave their sums per tile (init_domain), if a
+// level's rows fill whole tiles or, in the generic transform, whose tiles of 2
+// to 64 rows then start anew at each level, leave at most ny / kTileSumPad rows
+// empty: a step with k_wsum and with such tiles, FP32, 300 x 270 x 50 (1 in 270)
+// 0.901 and 0.875 ms, 135 x 135 x 75 with the temperature (1 in 15) 0.6395 and 0.6343.  The
+// register transforms' tiles of 32 and more rows gain nothing so (256 x 240 x 100, 1 in 15,
+// 1.037 and 1.038; 400 x 300 x 60 1.256 and 1.250), and the small domains' pay 0.4 us a stage.
 constexpr long long kTileSumBytes = 5 << 20;
 constexpr int kTileSumPad = 14;
 template <typename T>

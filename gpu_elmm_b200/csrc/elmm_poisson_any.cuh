@@ -234,6 +234,18 @@ __device__ __forceinline__ void fftx_passes(const FFTFactors &f, int ns, typenam
   __syncthreads();
 }
 
+// The rows of x tile lt: rows of them from r0 on, those before end in use.
+// Across levels, or (Dom::wrows) from the start of each level.
+struct XRows {
+  int r0, end;
+};
+template <typename T>
+__device__ __forceinline__ XRows x_rows(const Dom<T> &d, int lt, int rows) {
+  if (!d.wrows) return XRows{lt * rows, d.ny * d.nz};
+  const int np = d.wtiles(), k = lt / np;
+  return XRows{k * d.ny + (lt - k * np) * rows, (k + 1) * d.ny};
+}
+
 // the right-hand sides of an x tile's rows into buf, VE cells a task: the
 // divergence of PrePoisson (pressure.f90:688-717) from vectors of VE cells of
 // a row; and the tile's sum of W2

@@ -61,18 +61,6 @@ __device__ __forceinline__ RhsRow<T> rhs_row(const Dom<T> &d, int j, int k) {
   return r;
 }
 
-// The rows of x tile lt: rows of them from r0 on, those before end in use.
-// Across levels, or (Dom::wrows) from the start of each level.
-struct XRows {
-  int r0, end;
-};
-template <typename T>
-__device__ __forceinline__ XRows x_rows(const Dom<T> &d, int lt, int rows) {
-  if (!d.wrows) return XRows{lt * rows, d.ny * d.nz};
-  const int np = d.wtiles(), k = lt / np;
-  return XRows{k * d.ny + (lt - k * np) * rows, (k + 1) * d.ny};
-}
-
 // The sum of W2 over an x tile, whose rows lie in one level (Dom::wpart): each
 // thread adds the values it stages, in FP64.
 struct TileSum {
@@ -134,9 +122,8 @@ __device__ __forceinline__ void fftx_fwd_tile(const Dom<T> &d, int lt, typename 
   __shared__ RhsRow<T> rinfo[2 * NS];
   __shared__ double wred[kRegThreads / 32];
   const int s = threadIdx.x / P, t = threadIdx.x - s * P;
-  const int ny = d.ny;
-  const XRows xr = x_rows(d, lt, 2 * NS);
-  const int r0 = xr.r0, nrows = xr.end;  // sequence q holds rows r0 + 2q, r0 + 2q + 1
+  const int ny = d.ny, nrows = ny * d.nz;
+  const int r0 = 2 * lt * NS;  // first row of the tile; sequence q holds rows r0 + 2q, r0 + 2q + 1
   const T rdt2 = (T)(1.0 / coef);
   const T rdx = (T)(1.0 / d.dx), rdy = (T)(1.0 / d.dy), rdz = (T)(1.0 / d.dz);
   if (threadIdx.x < 2 * NS) {
@@ -301,9 +288,8 @@ __device__ __forceinline__ void fftx_inv_tile(const Dom<T> &d, int lt, typename 
   constexpr int P = Pl::P, E = Pl::E, NS = kRegThreads / P;
   constexpr int nxh = N / 2 + 1;
   const int s = threadIdx.x / P, t = threadIdx.x - s * P;
-  const int ny = d.ny;
-  const XRows xr = x_rows(d, lt, 2 * NS);
-  const int ra = xr.r0 + 2 * s, rb = ra + 1, nrows = xr.end;
+  const int ny = d.ny, nrows = ny * d.nz;
+  const int ra = 2 * (lt * NS + s), rb = ra + 1;
   const bool va = ra < nrows, vb = rb < nrows;
   const int qa = va ? ra : 0, qb = vb ? rb : 0;  // rows past the end are not read
   const T2 *Sa = d.S + (long long)qa * d.spitch, *Sb = d.S + (long long)qb * d.spitch;

@@ -1,8 +1,8 @@
 """The (0,0) mode of the pressure from the level sums of W: rows of whole
 16-byte vectors and not, sums from W2 itself and from the forward x
-transform's tiles (W2 of more than 5.2 MB and rows that fill a level's tiles or
-nearly so, of the register and the generic form; and rows that do not), levels
-past the tiled z solve, walls and periodic z, against the oracle."""
+transform's tiles (W2 of more than 5.2 MB and rows that fill a level's tiles, or
+in the generic form nearly so; and rows that do not), levels past the tiled z
+solve, walls and periodic z, against the oracle."""
 import numpy as np
 import pytest
 

@@ -258,7 +258,7 @@ def test_slabs_carry_puffs_and_slices(precision):
 
 # The mixed path keeps the single domain's state bit for bit: the (0,0) mode
 # comes from one sum per level, whichever slab holds the level (k_wsum for
-# small domains and rows that leave x tiles half empty, the tiles' sums
+# small domains and rows that do not fill x tiles, the tiles' sums
 # beyond, register and generic transforms), solved in one order; the other
 # modes' FP64 sweeps differ in grouping alone, far below FP32.
 @pytest.mark.parametrize("n, nz", [((48, 32, 24), (6, 10, 8)), ((256, 64, 96), (48, 48)), ((256, 64, 96), (30, 40, 26)),

@@ -69,9 +69,9 @@ def test_fp64_y_forms(n):
     test_poisson_of_every_pass_count(n, PREC_FP64, 1e-12)
 
 
-# A given right-hand side on domains whose x tiles start anew at each level
-# (W2 of more than 5.2 MB), with a last tile that is not full, of the register and
-# the generic form; bounds as above
+# A given right-hand side on large domains (W2 of more than 5.2 MB): register x
+# tiles across levels, and generic ones that start anew at each level with a
+# last tile that is not full; bounds as above
 @pytest.mark.parametrize("precision, tol", [(PREC_FP64, 1e-12), (PREC_MIXED, 1e-5)])
 @pytest.mark.parametrize("n", [(256, 125, 45), (300, 270, 18)])
 def test_poisson_with_tiles_per_level(n, precision, tol):
